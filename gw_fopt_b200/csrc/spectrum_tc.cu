@@ -327,6 +327,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_gemm_i8(TcArgs A) {
             constexpr int c_lo = decltype(half_c)::value * (kTcCols / 2);
             constexpr int b_lo = c_lo / CPB, b_hi = (c_lo + kTcCols / 2 - 1) / CPB;
             constexpr int nb = b_hi - b_lo + 1;
+            // A bubble whose columns straddle the two halves (3, 5, 6 or 7 sets) has an entry per
+            // half: a half may fill its entries for the next row while the other still reads this
+            // row's.  The second half's entries are moved up by one slot then.
+            constexpr int b_off = decltype(half_c)::value * ((kTcCols / 2) % CPB != 0 ? 1 : 0);
             int row = 0;
             for (int i = i0; active && i < i1 && !failed; ++i, ++row) {
                 // s_a 256^6 / F^2 e^{i w (t_a c_i - z_a)} per (w, bubble) of this row; zero for
@@ -344,7 +348,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_gemm_i8(TcArgs A) {
                         sincos(A.w[w0 + l] * (bt[b] * ci - bz[b]), &sn, &cs);
                         e = make_double2(sc * cs, sc * sn);
                     }
-                    etab[eslot(l, b)] = e;
+                    etab[eslot(l, b + b_off)] = e;
                 }
                 __syncwarp();
                 if (!tc::warp_wait_bounded(accf, row & 1, abort_flag)) {
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_gemm_i8(TcArgs A) {
                                                    (float)(int)d1[c]),
                                               kInv256, 0.0f);
                         const double y = (double)(int)d0[c] + (double)lo;
-                        const double2 e = etab[eslot(wl, b)];
+                        const double2 e = etab[eslot(wl, b + b_off)];
                         accC[sc] = fma(e.x, y, accC[sc]);
                         accS[sc] = fma(e.y, y, accS[sc]);
                     }
