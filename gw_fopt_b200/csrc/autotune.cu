@@ -110,7 +110,7 @@ LaunchShape autotune_launch_shape(Device* dev, const SpectrumJob& job) {
         auto it = g_cache.find(key);
         if (it != g_cache.end()) return it->second;
     }
-    const size_t kc_max = std::min(job.n_k, spectrum_max_frames_per_launch(job));
+    const size_t kc_max = std::min(job.n_k, spectrum_max_frames_per_launch(dev, job));
     // the sample: one launch of the largest frame count (all frames if fewer)
     const size_t n_s = kc_max;
     std::vector<size_t> frames;

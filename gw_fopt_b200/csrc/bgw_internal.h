@@ -128,7 +128,7 @@ void run_spectrum(Device* dev, const SpectrumJob& job, double* out, bool out_is_
 LaunchShape last_launch_shape(const Device* dev);
 
 // Frames per launch that the memory budget allows for this job.
-size_t spectrum_max_frames_per_launch(const SpectrumJob& job);
+size_t spectrum_max_frames_per_launch(const Device* dev, const SpectrumJob& job);
 
 // Row parts the wave-fill model picks for kn frames per launch (1 unless the
 // job runs the tensor-core GEMM).

@@ -4,9 +4,8 @@
 //   k_rotate       bubbles (t, x, y, z) rotated by R(k)            [optional]
 //   k_neighbors, k_masks_list (masks.cu)
 //                  exact first-collider search per (k, bubble, patch)
-//   k_spec_direct  plain FP64 spectrum: one complex phase per
-//                  (bubble, cos-theta row, t, w), the reference's loop nest
-//   k_reduce       deterministic sum of per-bubble partial spectra
+//   spectrum_direct.cu    plain FP64 spectrum, tensor and integrand
+//   spectrum_factored.cu  FP64 and mixed factored spectrum (spectrum_tc.cu: its tensor-core GEMM)
 //
 // Reference: rust/bubble-gw/src/many_bubbles/generalized_bulk_flow.rs (GBF).
 
@@ -22,6 +21,7 @@
 #include "bgw_internal.h"
 #include "device_common.cuh"
 #include "masks.cuh"
+#include "spectrum_direct.cuh"
 #include "spectrum_factored.cuh"
 #include "adjoint.cuh"
 
@@ -98,429 +98,6 @@ __global__ void k_rotate(const D4* __restrict__ bub, const double* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// Plain FP64 spectrum (GBF:481-586, 588-664, 775-873), one block per
-// (k-hat, radiating bubble).  Per t: the B stage evaluates every patch of
-// every cos-theta row into shared memory; the A stage gives each thread one w
-// and a stride of rows (rows split across thread groups when n_w < 256) and
-// forms sum_i B_i e^{-i w dt c_i} dc v_i; the C stage multiplies by
-// e^{i w (t - z_a)} u_t cut(t) dt.  The block writes its bubble's
-// (2, S, W) contribution times 1/(6 pi).
-// ---------------------------------------------------------------------------
-constexpr int kSpecThreads = 256;
-constexpr int kSetChunk = 4;
-
-struct SpecArgs {
-    const D4* bub;
-    size_t n_tot;
-    const uint32_t* sel;
-    size_t n_sel;
-    const double* tau;
-    int n_cos, n_phi;
-    const double* cos_thetax;
-    const double* sin2phi;
-    const double* cos2phi;
-    const double* coeffs;
-    const double* powers;
-    int n_sets, n_terms;
-    int has_damping;
-    double damping;
-    const double* t_arr;
-    const double* cutw;
-    int n_t;
-    double dt;
-    const double* w;
-    int n_w;
-    double2* partial;  // (K, n_sel, 2, S, W); with PER_T: (n_sel, 2, S, W, n_t); tensor: (K, n_sel, 6, S, W)
-    int tau_in_smem;
-    const double* cosphi;  // tensor form
-    const double* sinphi;
-};
-
-// Combination step of ndarray's unrolled_fold:
-// acc = (((0 + (p0+p4)) + (p1+p5)) + (p2+p6)) + (p3+p7), then + tail.
-__device__ __forceinline__ double unrolled_sum8(const double* p8, double tail) {
-    double acc = 0.0;
-    acc = __dadd_rn(acc, __dadd_rn(p8[0], p8[4]));
-    acc = __dadd_rn(acc, __dadd_rn(p8[1], p8[5]));
-    acc = __dadd_rn(acc, __dadd_rn(p8[2], p8[6]));
-    acc = __dadd_rn(acc, __dadd_rn(p8[3], p8[7]));
-    return __dadd_rn(acc, tail);
-}
-
-// PER_T: the time-resolved integrand of compute_c_integrand_fixed_bubble
-// (generalized_bulk_flow.rs:776-866): each step's A e^{i w (t - z_a)} times the
-// trapezoid dt weight and 1/(6 pi), one output per step (no time cutoff),
-// instead of the sum over steps.
-template <bool PER_T>
-__global__ void __launch_bounds__(kSpecThreads) k_spec_direct(SpecArgs A) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int k = blockIdx.y;
-    const size_t slot = blockIdx.x;
-    const int nd = A.n_cos * A.n_phi;
-    const double* tau_g = A.tau + ((size_t)k * A.n_sel + slot) * nd;
-    double* tau_s = reinterpret_cast<double*>(smem_raw);
-    // even number of doubles before Bsm keeps the double2 array below 16-byte aligned
-    double* Bsm = tau_s + (A.tau_in_smem ? ((nd + 1) & ~1) : 0);  // [n_cos][kSetChunk][2]
-    double2* red = reinterpret_cast<double2*>(Bsm + (size_t)A.n_cos * kSetChunk * 2);  // [256][kSetChunk][2]
-    const double* tau = A.tau_in_smem ? tau_s : tau_g;
-    if (A.tau_in_smem)
-        for (int q = threadIdx.x; q < nd; q += kSpecThreads) tau_s[q] = tau_g[q];
-    __syncthreads();
-
-    const uint32_t a = A.sel[slot];
-    const D4 xa = A.bub[(size_t)k * A.n_tot + a];
-    const double ta = xa.t, za = xa.z;
-    const int W_eff = min(A.n_w, kSpecThreads);
-    const int n_ig = kSpecThreads / W_eff;
-    const int wl = threadIdx.x % W_eff;
-    const int ig = threadIdx.x / W_eff;
-    const bool wthread = ig < n_ig;
-    const double dphi = 2.0 * CUDART_PI / (double)A.n_phi;
-    const double dcos = 2.0 / (double)(A.n_cos - 1);
-    const double inv6pi = 1.0 / (6.0 * CUDART_PI);
-
-    for (int s0 = 0; s0 < A.n_sets; s0 += kSetChunk) {
-        const int sc = min(kSetChunk, A.n_sets - s0);
-        for (int wb = 0; wb < A.n_w; wb += W_eff) {
-            const int wi = wb + wl;
-            const bool wvalid = wthread && wi < A.n_w;
-            const double wv = wvalid ? A.w[wi] : 0.0;
-            double2 cacc[kSetChunk][2];
-#pragma unroll
-            for (int s = 0; s < kSetChunk; ++s) cacc[s][0] = cacc[s][1] = make_double2(0.0, 0.0);
-
-            for (int kt = 0; kt < A.n_t; ++kt) {
-                const double t = A.t_arr[kt];
-                if (!(ta <= t)) continue;  // GBF:821
-                const double dta = t - ta;
-                // ---- B stage (GBF:481-586) ----
-                for (int i = threadIdx.x; i < A.n_cos; i += kSpecThreads) {
-                    const double c = A.cos_thetax[i];
-                    const double sin_sq = 1.0 - c * c;
-                    const double cubed = dta * (dta * dta);
-                    for (int s = 0; s < sc; ++s) {
-                        double bp = 0.0, bm = 0.0;
-                        if (dta > 0.0) {
-                            const double* trow = tau + (size_t)i * A.n_phi;
-                            const int sidx = (s0 + s) * A.n_terms;
-                            // f(t, t_n, t_nc) for patch j (GBF:549-567)
-                            auto factor = [&](int j) {
-                                const double tj = trow[j];
-                                double f = 1.0;
-                                if (tj > 0.0 && dta >= tj) {
-                                    const double ratio = tj / dta;
-                                    f = 0.0;
-                                    for (int m = 0; m < A.n_terms; ++m)
-                                        f += A.coeffs[sidx + m] * pow(ratio, A.powers[sidx + m]);
-                                    if (A.has_damping) f *= exp(-dta * (1.0 - ratio) / A.damping);
-                                }
-                                return f;
-                            };
-                            // ndarray's eight-way unrolled sum over phi (GBF:578-579)
-                            double pc[8], ps[8];
-#pragma unroll
-                            for (int u = 0; u < 8; ++u) pc[u] = ps[u] = 0.0;
-                            const int nfull = A.n_phi & ~7;
-                            for (int j0 = 0; j0 < nfull; j0 += 8) {
-#pragma unroll
-                                for (int u = 0; u < 8; ++u) {
-                                    const int j = j0 + u;
-                                    const double f = factor(j);
-                                    const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
-                                    pc[u] = __dadd_rn(pc[u], __dmul_rn(__dmul_rn(A.cos2phi[j], f), wj));
-                                    ps[u] = __dadd_rn(ps[u], __dmul_rn(__dmul_rn(A.sin2phi[j], f), wj));
-                                }
-                            }
-                            double sum_c = unrolled_sum8(pc, 0.0);
-                            double sum_s = unrolled_sum8(ps, 0.0);
-                            for (int j = nfull; j < A.n_phi; ++j) {
-                                const double f = factor(j);
-                                const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
-                                sum_c = __dadd_rn(sum_c, __dmul_rn(__dmul_rn(A.cos2phi[j], f), wj));
-                                sum_s = __dadd_rn(sum_s, __dmul_rn(__dmul_rn(A.sin2phi[j], f), wj));
-                            }
-                            bp = 0.5 * sin_sq * (sum_c * dphi * cubed);
-                            bm = 0.5 * sin_sq * (sum_s * dphi * cubed);
-                        }
-                        Bsm[((size_t)i * kSetChunk + s) * 2 + 0] = bp;
-                        Bsm[((size_t)i * kSetChunk + s) * 2 + 1] = bm;
-                    }
-                }
-                __syncthreads();
-                // ---- A stage (GBF:635-661) ----
-                double2 aacc[kSetChunk][2];
-#pragma unroll
-                for (int s = 0; s < kSetChunk; ++s) aacc[s][0] = aacc[s][1] = make_double2(0.0, 0.0);
-                if (wvalid) {
-                    for (int i = ig; i < A.n_cos; i += n_ig) {
-                        const double base_im = -dta * A.cos_thetax[i];
-                        double sn, cs;
-                        sincos(wv * base_im, &sn, &cs);
-                        const double vi = (i == 0 || i == A.n_cos - 1) ? 0.5 : 1.0;
-                        const double pr = (cs * dcos) * vi, pim = (sn * dcos) * vi;
-#pragma unroll
-                        for (int s = 0; s < kSetChunk; ++s) {
-                            if (s < sc) {
-                                const double bp = Bsm[((size_t)i * kSetChunk + s) * 2 + 0];
-                                const double bm = Bsm[((size_t)i * kSetChunk + s) * 2 + 1];
-                                aacc[s][0].x += bp * pr;
-                                aacc[s][0].y += bp * pim;
-                                aacc[s][1].x += bm * pr;
-                                aacc[s][1].y += bm * pim;
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (int s = 0; s < kSetChunk; ++s) {
-                    red[((size_t)threadIdx.x * kSetChunk + s) * 2 + 0] = aacc[s][0];
-                    red[((size_t)threadIdx.x * kSetChunk + s) * 2 + 1] = aacc[s][1];
-                }
-                __syncthreads();
-                // ---- C stage (GBF:832-851) ----
-                if (PER_T && wvalid && ig == 0) {
-                    double sn, cs;
-                    sincos(wv * (t - za), &sn, &cs);
-                    const double dtw = A.dt * ((kt == 0 || kt == A.n_t - 1) ? 0.5 : 1.0);
-                    for (int s = 0; s < sc; ++s) {
-                        for (int g = 0; g < 2; ++g) {
-                            double2 at = make_double2(0.0, 0.0);
-                            for (int q = 0; q < n_ig; ++q) {
-                                const double2 v = red[((size_t)(q * W_eff + wl) * kSetChunk + s) * 2 + g];
-                                at.x += v.x;
-                                at.y += v.y;
-                            }
-                            // (A e^{i w (t - z_a)}) (dt w_t) / (6 pi), GBF:832-840 and 862-863
-                            const double re = (at.x * cs - at.y * sn) * dtw * inv6pi;
-                            const double im = (at.x * sn + at.y * cs) * dtw * inv6pi;
-                            const size_t o = ((((size_t)slot * 2 + g) * A.n_sets + (s0 + s)) * A.n_w + wi) * A.n_t + kt;
-                            A.partial[o] = make_double2(re, im);
-                        }
-                    }
-                }
-                if (!PER_T && wvalid && ig == 0) {
-                    double sn, cs;
-                    sincos(wv * (t - za), &sn, &cs);
-                    const double uw = (kt == 0 || kt == A.n_t - 1) ? 0.5 : 1.0;
-                    const double cw = A.cutw[kt];
-                    for (int s = 0; s < sc; ++s) {
-                        for (int g = 0; g < 2; ++g) {
-                            double2 at = make_double2(0.0, 0.0);
-                            for (int q = 0; q < n_ig; ++q) {
-                                const double2 v = red[((size_t)(q * W_eff + wl) * kSetChunk + s) * 2 + g];
-                                at.x += v.x;
-                                at.y += v.y;
-                            }
-                            double re = (at.x * cs - at.y * sn) * uw * cw;
-                            double im = (at.x * sn + at.y * cs) * uw * cw;
-                            cacc[s][g].x += re * A.dt;
-                            cacc[s][g].y += im * A.dt;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-            if (!PER_T && wvalid && ig == 0) {
-                for (int s = 0; s < sc; ++s)
-                    for (int g = 0; g < 2; ++g) {
-                        size_t o = ((((size_t)k * A.n_sel + slot) * 2 + g) * A.n_sets + (s0 + s)) * A.n_w + wi;
-                        A.partial[o] = make_double2(cacc[s][g].x * inv6pi, cacc[s][g].y * inv6pi);
-                    }
-            }
-        }
-    }
-}
-
-// The tensor form of new_generalized_bulk_flow.rs (NGBF:592-1203): the phi
-// integral of x_i x_j (t - t_n)^3 f in six components (xx, xy, xz, yy, yz, zz,
-// NGBF:634-727), the same A and C stages with NGBF's factor placement
-// (NGBF:782-826, 1145-1168), no time cutoff; one coefficient set at a time.
-// PER_T: the time-resolved integrand (NGBF:832-991), each step's
-// A e^{i w (t - z_a)} (dt w_t) / (6 pi), partial (n_sel, 6, S, W, n_t).
-template <bool PER_T>
-__global__ void __launch_bounds__(kSpecThreads) k_tensor_direct(SpecArgs A) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int NG = 6;
-    const int k = blockIdx.y;
-    const size_t slot = blockIdx.x;
-    const int nd = A.n_cos * A.n_phi;
-    const double* tau_g = A.tau + ((size_t)k * A.n_sel + slot) * nd;
-    double* tau_s = reinterpret_cast<double*>(smem_raw);
-    double* Bsm = tau_s + (A.tau_in_smem ? ((nd + 1) & ~1) : 0);                      // [n_cos][6]
-    double2* red = reinterpret_cast<double2*>(Bsm + (size_t)A.n_cos * NG);            // [256][6]
-    const double* tau = A.tau_in_smem ? tau_s : tau_g;
-    if (A.tau_in_smem)
-        for (int q = threadIdx.x; q < nd; q += kSpecThreads) tau_s[q] = tau_g[q];
-    __syncthreads();
-
-    const uint32_t a = A.sel[slot];
-    const D4 xa = A.bub[(size_t)k * A.n_tot + a];
-    const double ta = xa.t, za = xa.z;
-    const int W_eff = min(A.n_w, kSpecThreads);
-    const int n_ig = kSpecThreads / W_eff;
-    const int wl = threadIdx.x % W_eff;
-    const int ig = threadIdx.x / W_eff;
-    const bool wthread = ig < n_ig;
-    const double dphi = 2.0 * CUDART_PI / (double)A.n_phi;
-    const double dcos = A.n_cos > 1 ? 2.0 / (double)(A.n_cos - 1) : 1.0;
-    const double inv6pi = 1.0 / (6.0 * CUDART_PI);
-
-    for (int s = 0; s < A.n_sets; ++s) {
-        for (int wb = 0; wb < A.n_w; wb += W_eff) {
-            const int wi = wb + wl;
-            const bool wvalid = wthread && wi < A.n_w;
-            const double wv = wvalid ? A.w[wi] : 0.0;
-            double2 cacc[NG];
-#pragma unroll
-            for (int g = 0; g < NG; ++g) cacc[g] = make_double2(0.0, 0.0);
-            for (int kt = 0; kt < A.n_t; ++kt) {
-                const double t = A.t_arr[kt];
-                if (t <= ta) continue;  // NGBF:1130
-                const double dta = t - ta;
-                // ---- B stage (NGBF:592-727) ----
-                for (int i = threadIdx.x; i < A.n_cos; i += kSpecThreads) {
-                    const double c = A.cos_thetax[i];
-                    const double st = sqrt(fmax(__dsub_rn(1.0, __dmul_rn(c, c)), 0.0));
-                    const double s2 = __dmul_rn(st, st), c2 = __dmul_rn(c, c), scz = __dmul_rn(st, c);
-                    const double cubed = __dmul_rn(__dmul_rn(dta, dta), dta);
-                    const double* trow = tau + (size_t)i * A.n_phi;
-                    const int sidx = s * A.n_terms;
-                    auto factor = [&](int j) {
-                        const double tj = trow[j];
-                        double f = 1.0;
-                        if (tj > 0.0 && dta >= tj) {
-                            const double ratio = tj / dta;
-                            f = 0.0;
-                            for (int m = 0; m < A.n_terms; ++m) f += A.coeffs[sidx + m] * pow(ratio, A.powers[sidx + m]);
-                            if (A.has_damping) f *= exp(-dta * (1.0 - ratio) / A.damping);
-                        }
-                        return f;
-                    };
-                    auto basis = [&](int j, int g) {
-                        const double cp = A.cosphi[j], sp = A.sinphi[j];
-                        switch (g) {
-                            case 0: return __dmul_rn(__dmul_rn(cp, cp), s2);
-                            case 1: return __dmul_rn(__dmul_rn(cp, sp), s2);
-                            case 2: return __dmul_rn(cp, scz);
-                            case 3: return __dmul_rn(__dmul_rn(sp, sp), s2);
-                            case 4: return __dmul_rn(sp, scz);
-                            default: return c2;
-                        }
-                    };
-                    // ndarray's eight-way unrolled sum over phi, per component
-                    double p8[NG][8];
-#pragma unroll
-                    for (int g = 0; g < NG; ++g)
-#pragma unroll
-                        for (int u = 0; u < 8; ++u) p8[g][u] = 0.0;
-                    const int nfull = A.n_phi & ~7;
-                    for (int j0 = 0; j0 < nfull; j0 += 8) {
-#pragma unroll
-                        for (int u = 0; u < 8; ++u) {
-                            const int j = j0 + u;
-                            const double f = factor(j);
-                            const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
-#pragma unroll
-                            for (int g = 0; g < NG; ++g) p8[g][u] = __dadd_rn(p8[g][u], __dmul_rn(__dmul_rn(basis(j, g), f), wj));
-                        }
-                    }
-                    double sums[NG];
-#pragma unroll
-                    for (int g = 0; g < NG; ++g) sums[g] = unrolled_sum8(p8[g], 0.0);
-                    for (int j = nfull; j < A.n_phi; ++j) {
-                        const double f = factor(j);
-                        const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
-#pragma unroll
-                        for (int g = 0; g < NG; ++g) sums[g] = __dadd_rn(sums[g], __dmul_rn(__dmul_rn(basis(j, g), f), wj));
-                    }
-#pragma unroll
-                    for (int g = 0; g < NG; ++g) Bsm[(size_t)i * NG + g] = __dmul_rn(__dmul_rn(sums[g], dphi), cubed);
-                }
-                __syncthreads();
-                // ---- A stage (NGBF:782-826): phase e^{-i w dt c_i} (dcos w_theta) ----
-                double2 aacc[NG];
-#pragma unroll
-                for (int g = 0; g < NG; ++g) aacc[g] = make_double2(0.0, 0.0);
-                if (wvalid) {
-                    for (int i = ig; i < A.n_cos; i += n_ig) {
-                        double sn, cs;
-                        sincos(wv * (-dta * A.cos_thetax[i]), &sn, &cs);
-                        const double vi = A.n_cos == 1 ? 1.0 : ((i == 0 || i == A.n_cos - 1) ? 0.5 : 1.0);
-                        const double pfs = dcos * vi;
-                        const double pr = cs * pfs, pim = sn * pfs;
-#pragma unroll
-                        for (int g = 0; g < NG; ++g) {
-                            const double b = Bsm[(size_t)i * NG + g];
-                            aacc[g].x += b * pr;
-                            aacc[g].y += b * pim;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int g = 0; g < NG; ++g) red[(size_t)threadIdx.x * NG + g] = aacc[g];
-                __syncthreads();
-                // ---- C stage (NGBF:1145-1168): A e^{i w (t - z_a)} (dt w_t) ----
-                if (PER_T && wvalid && ig == 0) {
-                    double sn, cs;
-                    sincos(wv * (t - za), &sn, &cs);
-                    const double dtw = A.dt * ((kt == 0 || kt == A.n_t - 1) ? 0.5 : 1.0);
-                    const double fr = cs * dtw, fi = sn * dtw;
-                    for (int g = 0; g < NG; ++g) {
-                        double2 at = make_double2(0.0, 0.0);
-                        for (int q = 0; q < n_ig; ++q) {
-                            const double2 v = red[(size_t)(q * W_eff + wl) * NG + g];
-                            at.x += v.x;
-                            at.y += v.y;
-                        }
-                        const size_t o = ((((size_t)slot * NG + g) * A.n_sets + s) * A.n_w + wi) * A.n_t + kt;
-                        A.partial[o] = make_double2((at.x * fr - at.y * fi) * inv6pi, (at.x * fi + at.y * fr) * inv6pi);
-                    }
-                }
-                if (!PER_T && wvalid && ig == 0) {
-                    double sn, cs;
-                    sincos(wv * (t - za), &sn, &cs);
-                    const double dtw = A.dt * ((kt == 0 || kt == A.n_t - 1) ? 0.5 : 1.0);
-                    const double fr = cs * dtw, fi = sn * dtw;
-                    for (int g = 0; g < NG; ++g) {
-                        double2 at = make_double2(0.0, 0.0);
-                        for (int q = 0; q < n_ig; ++q) {
-                            const double2 v = red[(size_t)(q * W_eff + wl) * NG + g];
-                            at.x += v.x;
-                            at.y += v.y;
-                        }
-                        cacc[g].x += at.x * fr - at.y * fi;
-                        cacc[g].y += at.x * fi + at.y * fr;
-                    }
-                }
-                __syncthreads();
-            }
-            if (!PER_T && wvalid && ig == 0) {
-                for (int g = 0; g < NG; ++g) {
-                    const size_t o = ((((size_t)k * A.n_sel + slot) * NG + g) * A.n_sets + s) * A.n_w + wi;
-                    A.partial[o] = make_double2(cacc[g].x * inv6pi, cacc[g].y * inv6pi);
-                }
-            }
-        }
-    }
-}
-
-// Sum over radiating bubbles in index order (GBF:971-981).
-__global__ void k_reduce(const double2* __restrict__ partial, size_t n_sel, size_t per, size_t kc,
-                         double2* __restrict__ out) {
-    size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t k = blockIdx.y;
-    if (q >= per || k >= kc) return;
-    double2 acc = make_double2(0.0, 0.0);
-    const double2* p = partial + k * n_sel * per + q;
-    for (size_t s = 0; s < n_sel; ++s) {
-        double2 v = p[s * per];
-        acc.x += v.x;
-        acc.y += v.y;
-    }
-    out[k * per + q] = acc;
-}
-
-// ---------------------------------------------------------------------------
 // Host orchestration.
 // ---------------------------------------------------------------------------
 namespace {
@@ -553,11 +130,10 @@ size_t mask_budget_bytes() {
 
 }  // namespace
 
-size_t spectrum_max_frames_per_launch(const SpectrumJob& job) {
+size_t spectrum_max_frames_per_launch(const Device* dev, const SpectrumJob& job) {
     const size_t nd = job.n_cos * job.n_phi;
-    const size_t per = (job.tensor ? 6 : 2) * job.n_sets * job.n_w;
     const size_t per_k = job.n_sel * nd * sizeof(double) +
-                         (job.kernel == BGWX_KERNEL_FP64_DIRECT ? job.n_sel * per * sizeof(double2)
+                         (job.kernel == BGWX_KERNEL_FP64_DIRECT ? direct_bytes_per_frame(dev, job)
                                                                 : factored_bytes_per_frame(job));
     const size_t kc = std::max<size_t>(1, mask_budget_bytes() / std::max<size_t>(per_k, 1));
     return std::min<size_t>(kc, 65535);
@@ -694,7 +270,7 @@ void run_spectrum(Device* dev, const SpectrumJob& job, double* out, bool out_is_
     if (uploads_only) return;  // the inputs are resident; a captured launch sequence follows
 
     // frames per chunk: bounded by the mask buffer budget (and by the job's launch shape)
-    size_t kc = std::min(K, spectrum_max_frames_per_launch(job));
+    size_t kc = std::min(K, spectrum_max_frames_per_launch(dev, job));
     if (job.frames_per_launch) kc = std::min(kc, job.frames_per_launch);
     dev->last_frames_per_launch = kc;
     dev->last_row_parts = job.kernel == BGWX_KERNEL_FP64_DIRECT ? 1 : 0;  // the factored launch records its own
@@ -710,7 +286,6 @@ void run_spectrum(Device* dev, const SpectrumJob& job, double* out, bool out_is_
     } else {
         dev->tau.ensure(kc * job.n_sel * nd * sizeof(double));
     }
-    if (job.kernel == BGWX_KERNEL_FP64_DIRECT) dev->partial.ensure(kc * job.n_sel * per * sizeof(double2));
     double2* final_out = out_is_device ? reinterpret_cast<double2*>(out) : nullptr;
     if (!final_out) {
         dev->out.ensure(out_blocks * per * sizeof(double2));
@@ -734,20 +309,6 @@ void run_spectrum(Device* dev, const SpectrumJob& job, double* out, bool out_is_
         CUDA_OK(cudaMemsetAsync(dev->counters.p, 0, 64, dev->stream));
     }
 
-    // shared memory of the direct kernel
-    size_t smem_fixed = job.tensor ? (size_t)job.n_cos * 6 * sizeof(double) + (size_t)kSpecThreads * 6 * sizeof(double2)
-                                   : (size_t)job.n_cos * kSetChunk * 2 * sizeof(double) +
-                                         (size_t)kSpecThreads * kSetChunk * 2 * sizeof(double2);
-    size_t smem_tau = ((nd + 1) & ~(size_t)1) * sizeof(double);
-    int max_optin = 0;
-    CUDA_OK(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev->id));
-    int tau_in_smem = smem_fixed + smem_tau <= (size_t)max_optin ? 1 : 0;
-    size_t smem = smem_fixed + (tau_in_smem ? smem_tau : 0);
-    if (smem > (size_t)max_optin) throw Error{"n_cos_thetax too large for the shared-memory layout"};
-    CUDA_OK(cudaFuncSetAttribute(k_spec_direct<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (job.tensor)
-        CUDA_OK(cudaFuncSetAttribute(k_tensor_direct<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-
     uint64_t launches = 0;
     record_event(dev, dev->ev[4]);
     for (size_t k0 = 0, ci = 0; k0 < K; k0 += kc, ++ci) {
@@ -769,46 +330,9 @@ void run_spectrum(Device* dev, const SpectrumJob& job, double* out, bool out_is_
                              job.mask_chunking);
         record_event(dev, cev[1]);
         if (job.kernel == BGWX_KERNEL_FP64_DIRECT) {
-            SpecArgs A;
-            A.bub = fb;
-            A.n_tot = job.n_tot;
-            A.sel = sel;
-            A.n_sel = job.n_sel;
-            A.tau = tau_k;
-            A.n_cos = (int)job.n_cos;
-            A.n_phi = (int)job.n_phi;
-            A.cos_thetax = cos_t;
-            A.sin2phi = sin2;
-            A.cos2phi = cos2;
-            A.coeffs = coeffs;
-            A.powers = powers;
-            A.n_sets = (int)S;
-            A.n_terms = (int)job.n_terms;
-            A.has_damping = job.has_damping ? 1 : 0;
-            A.damping = job.damping;
-            A.t_arr = t_arr;
-            A.cutw = cutw;
-            A.n_t = (int)job.n_t;
-            A.dt = job.dt;
-            A.w = w;
-            A.n_w = (int)W;
-            A.partial = (double2*)dev->partial.p;
-            A.tau_in_smem = tau_in_smem;
-            A.cosphi = cosphi;
-            A.sinphi = sinphi;
             if (job.n_sel > 0x7fffffffULL) throw Error{"too many radiating bubbles"};
-            dim3 g((unsigned)job.n_sel, (unsigned)kn);
-            if (job.tensor)
-                k_tensor_direct<false><<<g, kSpecThreads, smem, dev->stream>>>(A);
-            else
-                k_spec_direct<false><<<g, kSpecThreads, smem, dev->stream>>>(A);
-            CUDA_OK(cudaGetLastError());
-            ++launches;
-            dim3 gr((unsigned)((per + 255) / 256), (unsigned)kn);
-            k_reduce<<<gr, 256, 0, dev->stream>>>((const double2*)dev->partial.p, job.n_sel, per, kn,
-                                                  final_out + k0 * per);
-            CUDA_OK(cudaGetLastError());
-            ++launches;
+            const DirectInputs in{fb, sel, tau_k, cos_t, sin2, cos2, sinphi, cosphi, coeffs, powers, t_arr, cutw, w};
+            launches += launch_direct(dev, job, in, kn, final_out + k0 * per);
         } else {
             launches += launch_factored(dev, job, fb, sel, tau_k, cos_t, sin2, cos2, coeffs,
                                         powers, t_arr, cutw, w, k0, kn, final_out, real_tiles, &dev->fact_ev[3 * ci]);
@@ -866,7 +390,7 @@ static std::string batched_key(const SpectrumJob& b) {
 
 static void run_batched(Device* dev, SpectrumJob b, double2* eo, BgwxTimings* local) {
     // the frames per launch are fixed here: a captured sequence must not depend on free memory
-    if (!b.frames_per_launch) b.frames_per_launch = std::min(b.n_k, spectrum_max_frames_per_launch(b));
+    if (!b.frames_per_launch) b.frames_per_launch = std::min(b.n_k, spectrum_max_frames_per_launch(dev, b));
     const std::string key = batched_key(b);
     double* out = reinterpret_cast<double*>(eo);
     run_spectrum(dev, b, out, true, local, true, true);  // uploads what changed
@@ -1108,19 +632,6 @@ void run_adjoint(Device* dev, const SpectrumJob& job, const double* gbar, double
     }
 }
 
-// out += sum over the chunk's bubbles, in slot order, of their per-step values.
-__global__ void k_reduce_integrand(const double2* __restrict__ partial, size_t n, size_t per, double2* __restrict__ out) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= per) return;
-    double2 acc = out[q];
-    for (size_t a = 0; a < n; ++a) {
-        const double2 v = partial[a * per + q];
-        acc.x += v.x;
-        acc.y += v.y;
-    }
-    out[q] = acc;
-}
-
 void run_integrand(Device* dev, const SpectrumJob& job, double* out, BgwxTimings* tm) {
     CUDA_OK(cudaSetDevice(dev->id));
     const size_t nd = job.n_cos * job.n_phi;
@@ -1140,72 +651,17 @@ void run_integrand(Device* dev, const SpectrumJob& job, double* out, BgwxTimings
     uint32_t* sel = upload(dev, dev->sel, job.sel, job.n_sel, tm);
     double* cosphi = job.tensor ? upload(dev, dev->cosphi, job.cosphi, job.n_phi, tm) : nullptr;
     double* sinphi = job.tensor ? upload(dev, dev->sinphi, job.sinphi, job.n_phi, tm) : nullptr;
-    // bubbles per chunk: bounded by the per-bubble integrand buffer
-    const size_t budget = mask_budget_bytes();
-    size_t chunk = std::max<size_t>(1, std::min(job.n_sel, budget / std::max<size_t>(per * sizeof(double2), 1)));
-    chunk = std::min<size_t>(chunk, 65535);
     dev->tau.ensure(job.n_sel * nd * sizeof(double));
-    dev->partial.ensure(chunk * per * sizeof(double2));
     dev->out.ensure(per * sizeof(double2));
     dev->counters.ensure(64);
     CUDA_OK(cudaMemsetAsync(dev->counters.p, 0, 64, dev->stream));
-    CUDA_OK(cudaMemsetAsync(dev->out.p, 0, per * sizeof(double2), dev->stream));
-    size_t smem = job.tensor ? (size_t)job.n_cos * 6 * sizeof(double) + (size_t)kSpecThreads * 6 * sizeof(double2)
-                             : (size_t)job.n_cos * kSetChunk * 2 * sizeof(double) +
-                                   (size_t)kSpecThreads * kSetChunk * 2 * sizeof(double2);
-    const size_t smem_tau = ((nd + 1) & ~(size_t)1) * sizeof(double);
-    int max_optin = 0;
-    CUDA_OK(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev->id));
-    const int tau_in_smem = smem + smem_tau <= (size_t)max_optin ? 1 : 0;
-    if (tau_in_smem) smem += smem_tau;
-    if (smem > (size_t)max_optin) throw Error{"n_cos_thetax too large for the shared-memory layout"};
-    CUDA_OK(cudaFuncSetAttribute(k_spec_direct<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (job.tensor)
-        CUDA_OK(cudaFuncSetAttribute(k_tensor_direct<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     uint64_t launches = 0;
     CUDA_OK(cudaEventRecord(dev->ev[4], dev->stream));
     launch_mask_pipeline(dev, bub, bub, job.n_int, job.n_tot, sel, nullptr, job.n_sel, dirs, nd, job.n_phi, 1, (double*)dev->tau.p,
                          nullptr, (unsigned long long*)dev->counters.p, true, &launches);
-    for (size_t s0 = 0; s0 < job.n_sel; s0 += chunk) {
-        const size_t n = std::min(chunk, job.n_sel - s0);
-        CUDA_OK(cudaMemsetAsync(dev->partial.p, 0, n * per * sizeof(double2), dev->stream));
-        SpecArgs A;
-        A.bub = bub;
-        A.n_tot = job.n_tot;
-        A.sel = sel + s0;
-        A.n_sel = n;
-        A.tau = (const double*)dev->tau.p + s0 * nd;
-        A.n_cos = (int)job.n_cos;
-        A.n_phi = (int)job.n_phi;
-        A.cos_thetax = cos_t;
-        A.sin2phi = sin2;
-        A.cos2phi = cos2;
-        A.coeffs = coeffs;
-        A.powers = powers;
-        A.n_sets = (int)S;
-        A.n_terms = (int)job.n_terms;
-        A.has_damping = job.has_damping ? 1 : 0;
-        A.damping = job.damping;
-        A.t_arr = t_arr;
-        A.cutw = cutw;
-        A.n_t = (int)T;
-        A.dt = job.dt;
-        A.w = w;
-        A.n_w = (int)W;
-        A.partial = (double2*)dev->partial.p;
-        A.tau_in_smem = tau_in_smem;
-        A.cosphi = cosphi;
-        A.sinphi = sinphi;
-        if (job.tensor)
-            k_tensor_direct<true><<<dim3((unsigned)n, 1), kSpecThreads, smem, dev->stream>>>(A);
-        else
-            k_spec_direct<true><<<dim3((unsigned)n, 1), kSpecThreads, smem, dev->stream>>>(A);
-        CUDA_OK(cudaGetLastError());
-        k_reduce_integrand<<<(unsigned)((per + 255) / 256), 256, 0, dev->stream>>>((const double2*)dev->partial.p, n,
-                                                                                   per, (double2*)dev->out.p);
-        CUDA_OK(cudaGetLastError());
-        launches += 2;
-    }
+    const DirectInputs in{bub,    sel,    (const double*)dev->tau.p, cos_t,  sin2, cos2, sinphi, cosphi,
+                          coeffs, powers, t_arr,                     cutw,   w};
+    launches += launch_direct_integrand(dev, job, in, (double2*)dev->out.p);
     CUDA_OK(cudaEventRecord(dev->ev[5], dev->stream));
     CUDA_OK(cudaMemcpyAsync(out, dev->out.p, per * sizeof(double2), cudaMemcpyDeviceToHost, dev->stream));
     CUDA_OK(cudaStreamSynchronize(dev->stream));

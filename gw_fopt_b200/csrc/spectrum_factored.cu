@@ -43,6 +43,7 @@
 
 #include "bgw_internal.h"
 #include "device_common.cuh"
+#include "powers.cuh"
 #include "spectrum_factored.cuh"
 #include "spectrum_tc.cuh"
 #include "tc_ptx.cuh"
@@ -140,22 +141,6 @@ struct BetaArgs {
     double* scale;         // int8 digit layout: (kn, n_sel, n_cos) row scales, max |beta| of the row
     const double* Dmax;    // int8 digit layout: (n_sel, nblk, 1+S*M, 2) least and largest D over each block's steps
 };
-
-// x^p: binary powering for integral |p| <= 32 (a few ulp), pow() otherwise.
-__device__ __forceinline__ double tpow(double x, double p) {
-    const double r = rint(p);
-    if (r == p && fabs(r) <= 32.0) {
-        unsigned n = (unsigned)fabs(r);
-        double acc = 1.0, b = x;
-        while (n) {
-            if (n & 1u) acc *= b;
-            b *= b;
-            n >>= 1;
-        }
-        return r < 0.0 ? 1.0 / acc : acc;
-    }
-    return pow(x, p);
-}
 
 template <class Real, int SMC>
 __global__ void __launch_bounds__(256, std::is_same<Real, int8_t>::value ? 3 : 1) k_beta(BetaArgs A, Real* __restrict__ beta) {
