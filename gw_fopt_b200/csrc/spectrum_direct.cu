@@ -55,7 +55,32 @@ struct DirArgs {
     int k0, k1;       // steps [k0, k1) of this launch, k0 a multiple of 32
     int tp;           // row length of B (multiple of 32)
     double* B;        // (n_fs, n_cos, S G, tp): column s G + g
+    double* steps;    // (n_sel, 1 + S M, tf) step factors, see k_direct_steps
+    int tf;           // row length of the step factors (multiple of kStepBlock)
 };
+
+constexpr int kStepsPerLane = 4;
+constexpr int kStepBlock = 32 * kStepsPerLane;  // steps of a k_direct_b warp
+
+// Step factors of the separable scaling, frame and row independent, for blocks of kStepBlock steps with
+// dt_ref = dt at the block's last step: row 0 is dt^3 times the step weight (cutoff, dt, trapezoid
+// end), row 1 + q the factor a_q (dt_ref / dt)^{p_q} e^{(dt_ref - dt) / width}.  Zero where dt <= 0.
+__global__ void k_direct_steps(DirArgs A) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, slot = blockIdx.y + blockIdx.z * 65535;
+    if (k >= A.tf || slot >= A.n_sel) return;
+    const double ta = A.in.bub[A.in.sel[slot]].t;
+    const int klast = min(k | (kStepBlock - 1), A.n_t - 1);
+    const double dt_ref = A.in.t_arr[klast] - ta;
+    const double dt = k < A.n_t ? A.in.t_arr[k] - ta : 0.0;
+    const bool on = dt > 0.0;
+    const int SM = A.S * A.M;
+    double* o = A.steps + (size_t)slot * (1 + SM) * A.tf + k;
+    const double u = (k == 0 || k == A.n_t - 1) ? 0.5 : 1.0;
+    o[0] = on ? dt * (dt * dt) * A.in.cutw[k] * A.dt * u : 0.0;
+    const double e = on && A.has_damp ? exp((dt_ref - dt) / A.damp) : 1.0;
+    for (int q = 0; q < SM; ++q)
+        o[(size_t)(1 + q) * A.tf] = on ? A.in.coeffs[q] * tpow(dt_ref / dt, A.in.powers[q]) * e : 0.0;
+}
 
 // phi weight g of patch j without its trapezoid end weight
 template <int G>
@@ -123,13 +148,18 @@ __device__ __forceinline__ double first_collision(const double* __restrict__ tro
     return least;
 }
 
-// NS: steps per lane.  EXACT: every patch and step by pow and exp as the reference forms them, for
-// exponents and damping widths whose separated factors could leave the FP64 range (see direct_exact).
-template <int G, int NS, bool EXACT>
+// The phi sums of one (pair, row) over a block of kStepBlock steps; lane l holds steps 4 l .. 4 l + 3 of it.
+// EXACT: every patch and step by pow and exp as the reference forms them, for exponents and damping
+// widths whose separated factors could leave the FP64 range (see direct_exact).
+template <int G, bool EXACT>
 __global__ void __launch_bounds__(32 * kDirWarps) k_direct_b(DirArgs A) {
     constexpr unsigned full = 0xffffffffu;
+    constexpr int NS = kStepsPerLane;
+    // per warp: the block's collisions added up by step, one row per weight
+    __shared__ __align__(16) double s_acc[kDirWarps][G][kStepBlock];
     const int lane = threadIdx.x & 31;
-    const int nkb = (A.k1 - A.k0 + 32 * NS - 1) / (32 * NS);
+    double(*acc)[kStepBlock] = s_acc[threadIdx.x >> 5];
+    const int nkb = (A.k1 - A.k0 + kStepBlock - 1) / kStepBlock;
     const size_t wid = (size_t)blockIdx.x * kDirWarps + (threadIdx.x >> 5);
     if (wid >= A.n_fs * A.n_cos * nkb) return;
     const int kb = (int)(wid % nkb);
@@ -137,38 +167,67 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_direct_b(DirArgs A) {
     const int i = (int)(row % A.n_cos);
     const size_t fs = A.fs0 + row / A.n_cos;
     const int slot = (int)(fs % A.n_sel);
-    const size_t frame = fs / A.n_sel;
-    const double ta = A.in.bub[frame * A.n_tot + A.in.sel[slot]].t;
+    const double ta = A.in.bub[(fs / A.n_sel) * A.n_tot + A.in.sel[slot]].t;
     const double* trow = A.in.tau + (fs * A.n_cos + i) * A.n_phi;
-    const int kbase = A.k0 + kb * 32 * NS;
-    const int klast = min(kbase + 32 * NS, A.k1) - 1;
+    const int kbase = A.k0 + kb * kStepBlock;
+    const int klast = min(kbase + kStepBlock, A.k1) - 1;
     const double dt_first = A.in.t_arr[kbase] - ta, dt_last = A.in.t_arr[klast] - ta;
-    const int cols = A.S * G;
-    double* out = A.B + row * cols * A.tp + (kbase - A.k0);
-    double dta[NS];
-#pragma unroll
-    for (int m = 0; m < NS; ++m) dta[m] = A.in.t_arr[min(kbase + 32 * m + lane, klast)] - ta;
-    const double c = A.in.cos_t[i];
-    // row weight, dphi, dcos with its end weight, 1 / (6 pi)
-    const double rowf = A.dphi * A.dcos * ((i == 0 || i == A.n_cos - 1) ? 0.5 : 1.0) * (1.0 / (6.0 * CUDART_PI));
+    const int SM = A.S * A.M;
+    const double* steps = A.steps + (size_t)slot * (1 + SM) * A.tf + kbase + NS * lane;
     const bool live = dt_last > 0.0;
+    double* out = A.B + row * (A.S * G) * A.tp + (kbase - A.k0) + NS * lane;
+    // rows of B hold whole groups of 32 steps: a lane's four steps are all in or all out
+    const bool store = kbase - A.k0 + NS * lane < A.tp;
+    if (!live) {
+        if (store)
+            for (int col = 0; col < A.S * G; ++col)
+#pragma unroll
+                for (int m = 0; m < NS; m += 2)
+                    *reinterpret_cast<double2*>(out + (size_t)col * A.tp + m) = make_double2(0.0, 0.0);
+        return;
+    }
+    const double c = A.in.cos_t[i];
+    // dphi, dcos with its end weight, 1 / (6 pi)
+    const double rowf = A.dphi * A.dcos * ((i == 0 || i == A.n_cos - 1) ? 0.5 : 1.0) * (1.0 / (6.0 * CUDART_PI));
     double rw[G], quiet[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         rw[g] = row_weight<G>(c, g);
         quiet[g] = 0.0;
     }
-    if (live && !(first_collision(trow, A.n_phi) <= dt_first)) quiet_row<G>(A, c, quiet);
-    for (int s = 0; s < A.S; ++s) {
-        double res[NS][G];
-        bool hits[NS];  // some patch has collided by this step
+    const double least = first_collision(trow, A.n_phi);
+    if (!(least <= dt_first)) quiet_row<G>(A, c, quiet);
+    double wk[NS];
+    bool hits[NS];  // some patch has collided by this step
 #pragma unroll
-        for (int m = 0; m < NS; ++m) hits[m] = false;
+    for (int m = 0; m < NS; ++m) {
+        const int k = kbase + NS * lane + m;
+        wk[m] = k < A.k1 ? rowf * steps[m] : 0.0;
+        hits[m] = least <= A.in.t_arr[min(k, klast)] - ta;
+    }
+    auto put = [&](int s, const double (&res)[NS][G]) {
 #pragma unroll
-        for (int m = 0; m < NS; ++m)
+        for (int g = 0; g < G; ++g) {
+            double v[NS];
 #pragma unroll
-            for (int g = 0; g < G; ++g) res[m][g] = 0.0;
-        if (EXACT && live) {
+            for (int m = 0; m < NS; ++m) v[m] = wk[m] != 0.0 ? (hits[m] ? res[m][g] * rw[g] : quiet[g]) * wk[m] : 0.0;
+            if (store) {
+                double* o = out + (size_t)(s * G + g) * A.tp;
+                *reinterpret_cast<double2*>(o) = make_double2(v[0], v[1]);
+                *reinterpret_cast<double2*>(o + 2) = make_double2(v[2], v[3]);
+            }
+        }
+    };
+    if constexpr (EXACT) {
+        double dta[NS];
+#pragma unroll
+        for (int m = 0; m < NS; ++m) dta[m] = A.in.t_arr[min(kbase + NS * lane + m, klast)] - ta;
+        for (int s = 0; s < A.S; ++s) {
+            double res[NS][G];
+#pragma unroll
+            for (int m = 0; m < NS; ++m)
+#pragma unroll
+                for (int g = 0; g < G; ++g) res[m][g] = 0.0;
             for (int j = 0; j < A.n_phi; ++j) {
                 const double tj = trow[j];
                 const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
@@ -176,7 +235,6 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_direct_b(DirArgs A) {
                 for (int m = 0; m < NS; ++m) {
                     double f = 1.0;
                     if (tj > 0.0 && dta[m] >= tj) {
-                        hits[m] = true;
                         const double ratio = tj / dta[m];
                         f = 0.0;
                         for (int q = 0; q < A.M; ++q)
@@ -187,94 +245,125 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_direct_b(DirArgs A) {
                     for (int g = 0; g < G; ++g) res[m][g] += phi_weight<G>(A, j, g) * f * wj;
                 }
             }
-        } else if (live) {
-            for (int q = 0; q < A.M; ++q) {
-                const double p = A.in.powers[s * A.M + q], am = A.in.coeffs[s * A.M + q];
-                double P[G], U[G], Pin[NS][G];
+            put(s, res);
+        }
+    } else {
+        const double inv_dt = 1.0 / A.dt;  // the estimate below is only a starting point
+        // Adds the block's patches up: `base` (all lanes) the sum over the patches of state `pre` at the
+        // block's first step (collided: P) or uncollided at its last (U), acc the patches colliding in
+        // between, at their own step. 
+        auto sweep = [&](bool collided, double p, double (&base)[G]) {
 #pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    P[g] = U[g] = 0.0;
+            for (int g = 0; g < G; ++g) {
+                base[g] = 0.0;
 #pragma unroll
-                    for (int m = 0; m < NS; ++m) Pin[m][g] = 0.0;
-                }
-                for (int j0 = 0; j0 < A.n_phi; j0 += 32) {
-                    const int j = j0 + lane;
-                    const bool valid = j < A.n_phi;
-                    const double tj = valid ? trow[j] : 0.0;
-                    const double wj = valid ? ((j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0) : 0.0;
-                    const bool col = tj > 0.0 && dt_last >= tj;   // collided at the block's last step
-                    const bool pre = tj > 0.0 && dt_first >= tj;  // ... and at its first
-                    if (__any_sync(full, pre)) {
-#pragma unroll
-                        for (int m = 0; m < NS; ++m) hits[m] = true;
-                    }
-                    double v = 0.0, x[G];
+                for (int m = 0; m < NS; ++m) acc[g][lane + 32 * m] = 0.0;
+            }
+            __syncwarp();
+            for (int j0 = 0; j0 < A.n_phi; j0 += 32) {
+                const int j = j0 + lane;
+                const bool valid = j < A.n_phi;
+                const double tj = valid ? trow[j] : 0.0;
+                const bool col = tj > 0.0 && dt_last >= tj;   // collided at the block's last step
+                const bool pre = tj > 0.0 && dt_first >= tj;  // ... and at its first
+                const bool in = col && !pre;
+                double v = valid ? ((j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0) : 0.0;
+                if (collided) {
                     if (col) {
-                        v = tpow(tj / dt_last, p);
+                        v *= tpow(tj / dt_last, p);
                         if (A.has_damp) v *= exp(-(dt_last - tj) / A.damp);
                     }
-#pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        x[g] = valid ? wj * phi_weight<G>(A, j, g) : 0.0;
-                        if (pre) P[g] += x[g] * v;
-                        if (!col) U[g] += x[g];
-                    }
-                    for (unsigned h = __ballot_sync(full, col && !pre); h; h &= h - 1) {
-                        const int src = __ffs(h) - 1;
-                        const double ts = __shfl_sync(full, tj, src), vs = __shfl_sync(full, v, src);
-                        bool hit[NS];
-#pragma unroll
-                        for (int m = 0; m < NS; ++m) {
-                            hit[m] = dta[m] >= ts;
-                            hits[m] |= hit[m];
-                        }
-#pragma unroll
-                        for (int g = 0; g < G; ++g) {
-                            const double xs = __shfl_sync(full, x[g], src), xv = xs * vs;
-#pragma unroll
-                            for (int m = 0; m < NS; ++m) {
-                                if (hit[m]) Pin[m][g] += xv;
-                                else if (q == 0) res[m][g] += xs;
-                            }
-                        }
-                    }
                 }
+                double x[G];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
+                for (int g = 0; g < G; ++g) {
+                    x[g] = valid ? v * phi_weight<G>(A, j, g) : 0.0;
+                    if (collided ? pre : !col) base[g] += x[g];
+                }
+                if (!__any_sync(full, in)) continue;
+                int kj = 32 * NS + lane;  // position in the block of the first collided step
+                if (in) {
+                    const double est = ceil((ta + tj - A.in.t_arr[0]) * inv_dt);
+                    int k = max(kbase, min(klast, (int)fmin(fmax(est, 0.0), 2e9)));
+                    while (k > kbase && A.in.t_arr[k - 1] - ta >= tj) --k;
+                    while (!(A.in.t_arr[k] - ta >= tj)) ++k;  // holds at klast at the latest
+                    kj = k - kbase;
+                }
+                // patches of one step are added one after another, in lane order
+                const unsigned same = __match_any_sync(full, kj);
+                int rank = in ? __popc(same & ((1u << lane) - 1u)) : 32;
+                for (int r = 0; __any_sync(full, rank >= r && rank < 32); ++r) {
+                    if (rank == r) {
 #pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        P[g] += __shfl_xor_sync(full, P[g], o);
-                        if (q == 0) U[g] += __shfl_xor_sync(full, U[g], o);
+                        for (int g = 0; g < G; ++g) acc[g][kj] += x[g];
                     }
-#pragma unroll
-                for (int m = 0; m < NS; ++m) {
-                    double cm = 0.0;
-                    if (dta[m] > 0.0) {
-                        cm = am * tpow(dt_last / dta[m], p);
-                        if (A.has_damp) cm *= exp((dt_last - dta[m]) / A.damp);
-                    }
-#pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        const double sum = P[g] + Pin[m][g];
-                        if (q == 0) res[m][g] += U[g];
-                        // before the first collision there is nothing to scale (cm may be huge there)
-                        if (sum != 0.0) res[m][g] += cm * sum;
-                    }
+                    __syncwarp();
                 }
             }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int g = 0; g < G; ++g) base[g] += __shfl_xor_sync(full, base[g], o);
+        };
+        // uncollided sums: base plus the patches whose step comes later (a sum of what remains)
+        double U[NS][G], base[G];
+        sweep(false, 0.0, base);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            double v[NS], tot = 0.0;
+#pragma unroll
+            for (int m = 0; m < NS; ++m) v[m] = acc[g][NS * lane + m];
+#pragma unroll
+            for (int m = NS - 1; m >= 0; --m) {
+                U[m][g] = tot;  // later steps of this lane
+                tot += v[m];
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double t = __shfl_down_sync(full, tot, o);
+                if (lane + o < 32) tot += t;
+            }
+            double later = __shfl_down_sync(full, tot, 1);
+            if (lane == 31) later = 0.0;
+#pragma unroll
+            for (int m = 0; m < NS; ++m) U[m][g] = base[g] + (later + U[m][g]);
         }
+        __syncwarp();
+        for (int s = 0; s < A.S; ++s) {
+            double res[NS][G];
 #pragma unroll
-        for (int m = 0; m < NS; ++m) {
-            const int k = kbase + 32 * m + lane;
-            if (k - A.k0 >= A.tp) continue;
-            const bool on = k < A.k1 && dta[m] > 0.0;
-            const double wk = on ? rowf * (dta[m] * (dta[m] * dta[m])) * A.in.cutw[k] * A.dt *
-                                       ((k == 0 || k == A.n_t - 1) ? 0.5 : 1.0)
-                                 : 0.0;
+            for (int m = 0; m < NS; ++m)
 #pragma unroll
-            for (int g = 0; g < G; ++g)
-                out[(size_t)(s * G + g) * A.tp + 32 * m + lane] =
-                    on ? (hits[m] ? res[m][g] * rw[g] : quiet[g]) * wk : 0.0;
+                for (int g = 0; g < G; ++g) res[m][g] = U[m][g];
+            for (int q = 0; q < A.M; ++q) {
+                sweep(true, A.in.powers[s * A.M + q], base);
+                double cm[NS];
+#pragma unroll
+                for (int m = 0; m < NS; ++m) cm[m] = steps[(size_t)(1 + s * A.M + q) * A.tf + m];
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    double v[NS], tot = 0.0;
+#pragma unroll
+                    for (int m = 0; m < NS; ++m) {
+                        tot += acc[g][NS * lane + m];
+                        v[m] = tot;
+                    }
+                    double run = tot;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const double t = __shfl_up_sync(full, run, o);
+                        if (lane >= o) run += t;
+                    }
+                    double before = __shfl_up_sync(full, run, 1);
+                    if (lane == 0) before = 0.0;
+                    // with nothing collided there is nothing to scale (cm may be huge there)
+#pragma unroll
+                    for (int m = 0; m < NS; ++m)
+                        if (hits[m]) res[m][g] += cm[m] * (base[g] + (before + v[m]));
+                }
+                __syncwarp();
+            }
+            put(s, res);
         }
     }
 }
@@ -296,143 +385,224 @@ struct RowSumArgs {
     double2* partial; // spectrum: (pairs of the job, n_parts, G, S, W); integrand: (bubble parts, G, S, W, n_t)
 };
 
-// NC columns from column c0 = blockIdx.z NC on.
+__device__ __forceinline__ void copy16_async(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+
+// Sums of N values over the 32 lanes, one result per lane: at each of the five exchanges a lane keeps
+// half of its values and adds the other lane's (24 exchanges for 24 values instead of 120).
+template <int N>
+__device__ __forceinline__ double lane_sums(double (&v)[N]) {
+    const int lane = threadIdx.x & 31;
+    int n = N;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n == 1) {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            continue;
+        }
+        const int half = (n + 1) / 2;
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            if (q >= half) break;
+            const double up = q + half < n ? v[q + half] : 0.0;
+            const bool upper = lane & o;
+            const double got = __shfl_xor_sync(0xffffffffu, upper ? v[q] : up, o);
+            v[q] = (upper ? up : v[q]) + got;
+        }
+        n = half;
+    }
+    return v[0];
+}
+// The index of the value that lane_sums leaves in this lane; -1: a copy or nothing.
+template <int N>
+__device__ __forceinline__ int lane_value(int lane) {
+    int n = N, own = N, e = 0;  // values per lane (padded), this lane's own, the first of them
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool upper = lane & o;
+        if (n == 1) {
+            if (upper) return -1;
+            continue;
+        }
+        const int half = (n + 1) / 2;
+        e += upper ? half : 0;
+        own = upper ? own - half : min(own, half);
+        if (own <= 0) return -1;
+        n = half;
+    }
+    return e;
+}
+
+// Row pairs of one shared-memory stage: 8 KB with two columns, 12 KB with six.
+template <int NC>
+__host__ __device__ constexpr int stage_pairs() {
+    return NC <= 2 ? 8 : 4;
+}
+constexpr int kRowStages = 3;
+
+// NC columns from column c0 on, NW frequencies per warp, lane = step.  The block's warps share B: row
+// pairs (i, n_cos - 1 - i) of the NC columns and 32 steps arrive in shared memory by asynchronous
+// copies, three stages deep (from L1 and L2 directly the loads' latency was 70 % of the time: 2.09 ms
+// against 0.34 ms of FP64 work for 4 frames of 64 bubbles, 64 rows, 256 steps, 64 w, 6 columns).
 template <int NC, int NW, bool BIG, bool PER_T>
-__global__ void __launch_bounds__(32 * kDirWarps) k_direct_a(RowSumArgs R, int G) {
-    extern __shared__ double s_c[];  // cos theta of the rows
+__global__ void __launch_bounds__(32 * kDirWarps) k_direct_a(RowSumArgs R, int G, int w_tiles) {
+    constexpr int RP = stage_pairs<NC>();
+    constexpr int kStageDoubles = RP * 2 * NC * 32;
+    extern __shared__ __align__(16) double s_dyn[];
+    double* s_b = s_dyn;                                 // [kRowStages][pair][2][NC][32]
+    double* s_c = s_dyn + kRowStages * kStageDoubles;    // cos theta of the rows
     __shared__ double2 tab[kPhaseTable];
     const DirArgs& A = R.d;
     if constexpr (!BIG) phase_table_fill(tab);
     for (int q = threadIdx.x; q < A.n_cos; q += blockDim.x) s_c[q] = A.in.cos_t[q];
-    __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int w0 = (blockIdx.y * kDirWarps + (threadIdx.x >> 5)) * NW;
-    if (w0 >= A.n_w) return;
-    const int cols = A.S * G, c0 = blockIdx.z * NC;
+    // blocks of the same bubble and steps follow one another: they read the same B
+    const int w_tile = blockIdx.x % w_tiles;
+    const int unit_block = blockIdx.x / w_tiles;
+    const int w0 = (w_tile * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * NW;
+    const int cols = A.S * G, c0 = blockIdx.y * NC;
     const int nkc = (A.k1 - A.k0 + 31) >> 5;
     double wv[NW];
 #pragma unroll
     for (int u = 0; u < NW; ++u) wv[u] = A.in.w[min(w0 + u, A.n_w - 1)];
-    double cr[NW][NC], cim[NW][NC];
+    // the integrand sums over bubbles per lane; the spectrum adds each unit up over the warp's lanes
+    // (steps) at once and keeps one value per lane, the register budget of two blocks per SM
+    constexpr int NV = 2 * NW * NC;
+    double c_sum[PER_T ? NV : 1];
 #pragma unroll
-    for (int u = 0; u < NW; ++u)
-#pragma unroll
-        for (int n = 0; n < NC; ++n) cr[u][n] = cim[u][n] = 0.0;
-    // spectrum: blockIdx.x = (pair, group of step blocks); integrand: (bubble group, step block)
+    for (int v = 0; v < (PER_T ? NV : 1); ++v) c_sum[v] = 0.0;
+    // units taken in turn.  Spectrum: step blocks [lo, hi) of one pair; integrand: pairs [lo, hi) at one step block
     const int n_grp = (nkc + R.per_warp - 1) / R.per_warp;
-    size_t f_lo, f_hi;
-    int b_lo, b_hi;
-    if constexpr (PER_T) {
-        f_lo = (size_t)(blockIdx.x / nkc) * R.per_warp;
-        f_hi = min(f_lo + R.per_warp, A.n_fs);
-        b_lo = blockIdx.x % nkc;
-        b_hi = b_lo + 1;
-    } else {
-        f_lo = blockIdx.x / n_grp;
-        f_hi = f_lo + 1;
-        b_lo = (int)(blockIdx.x % n_grp) * R.per_warp;
-        b_hi = min(b_lo + R.per_warp, nkc);
-    }
-    for (size_t f = f_lo; f < f_hi; ++f) {
+    size_t lo, hi, fixed;
+    auto bubble = [&](size_t f) {
         const size_t fs = A.fs0 + f;
-        const D4 xa = A.in.bub[(fs / A.n_sel) * A.n_tot + A.in.sel[fs % A.n_sel]];
-        for (int b = b_lo; b < b_hi; ++b) {
-            const int k = A.k0 + 32 * b + lane;
-            if (!(A.in.t_arr[min(A.k0 + 32 * b + 31, A.k1 - 1)] - xa.t > 0.0)) continue;  // not nucleated yet
-            const double t = A.in.t_arr[min(k, A.k1 - 1)];
-            const double dta = t - xa.t;
-            double ar[NW][NC], ai[NW][NC];
+        return A.in.bub[(fs / A.n_sel) * A.n_tot + A.in.sel[fs % A.n_sel]];
+    };
+    D4 xa = D4{0.0, 0.0, 0.0, 0.0};
+    double t = 0.0, dta = 0.0;
+    if constexpr (PER_T) {
+        fixed = unit_block % nkc;
+        lo = (size_t)(unit_block / nkc) * R.per_warp;
+        hi = min(lo + R.per_warp, A.n_fs);
+    } else {
+        fixed = unit_block / n_grp;
+        lo = (size_t)(unit_block % n_grp) * R.per_warp;
+        hi = min(lo + R.per_warp, (size_t)nkc);
+        // step blocks before the bubble nucleates hold nothing
+        xa = bubble(fixed);
+        while (lo < hi && !(A.in.t_arr[min(A.k0 + 32 * (int)lo + 31, A.k1 - 1)] - xa.t > 0.0)) ++lo;
+    }
+    const size_t rstep = (size_t)cols * A.tp;
+    const int n_pairs = (A.n_cos + 1) >> 1;
+    const int per_unit = (n_pairs + RP - 1) / RP;
+    const size_t n_stages = (hi - lo) * per_unit;
+    auto load = [&](size_t q) {
+        if (q < n_stages) {
+            const size_t unit = lo + q / per_unit;
+            const int p0 = (int)(q % per_unit) * RP;
+            const size_t f = PER_T ? unit : fixed, b = PER_T ? fixed : unit;
+            const double* src = A.B + f * A.n_cos * rstep + (size_t)c0 * A.tp + 32 * b;
+            double* dst = s_b + (q % kRowStages) * kStageDoubles;
+            for (int e = threadIdx.x; e < RP * 2 * NC * 16; e += blockDim.x) {
+                const int line = e >> 4, at = (e & 15) * 2;  // line: (pair, side, column) of 32 steps
+                const int n = line % NC, side = (line / NC) & 1, p = p0 + line / (2 * NC);
+                if (p >= n_pairs) break;
+                const int i = side ? A.n_cos - 1 - p : p;
+                copy16_async(dst + line * 32 + at, src + i * rstep + (size_t)n * A.tp + at);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int q = 0; q < kRowStages - 1; ++q) load(q);
+    double ar[NW][NC], ai[NW][NC];
+    size_t unit = lo;
+    int st = 0;  // stage within the unit
+    for (size_t q = 0; q < n_stages; ++q) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRowStages - 2) : "memory");
+        __syncthreads();  // stage q has landed for every thread, stage q - 1 is free
+        load(q + kRowStages - 1);
+        if (st == 0) {
+            if constexpr (PER_T) xa = bubble(unit);
+            t = A.in.t_arr[min(A.k0 + 32 * (int)(PER_T ? fixed : unit) + lane, A.k1 - 1)];
+            dta = t - xa.t;
 #pragma unroll
             for (int u = 0; u < NW; ++u)
 #pragma unroll
                 for (int n = 0; n < NC; ++n) ar[u][n] = ai[u][n] = 0.0;
-            const size_t rstep = (size_t)cols * A.tp;
-            const double* b0 = A.B + f * A.n_cos * rstep + (size_t)c0 * A.tp + (32 * b + lane);
-            const double* b1 = b0 + (A.n_cos - 1) * rstep;
-            const int half = A.n_cos >> 1;
-            for (int i = 0; i < half; ++i, b0 += rstep, b1 -= rstep) {
-                double v0[NC], v1[NC];
+        }
+        const double* tile = s_b + (q % kRowStages) * kStageDoubles + lane;
+        const int p1 = min(n_pairs, (st + 1) * RP);
+        for (int p = st * RP; p < p1; ++p, tile += 2 * NC * 32) {
+            const bool twin = p != A.n_cos - 1 - p;  // the middle row of an odd number stands alone
+            double v0[NC], v1[NC];
 #pragma unroll
-                for (int n = 0; n < NC; ++n) {
-                    v0[n] = __ldg(b0 + (size_t)n * A.tp);
-                    v1[n] = __ldg(b1 + (size_t)n * A.tp);
-                }
-                const double m0 = -dta * s_c[i], m1 = -dta * s_c[A.n_cos - 1 - i];
-#pragma unroll
-                for (int u = 0; u < NW; ++u) {
-                    const double x0 = __dmul_rn(wv[u], m0), x1 = __dmul_rn(wv[u], m1);
-                    double s0, q0, s1, q1;
-                    phase_of<BIG>(tab, x0, s0, q0);
-                    if constexpr (BIG) {
-                        sincos(x1, &s1, &q1);
-                    } else {
-                        // exact: the (rounded) arguments are opposite to a few ulp
-                        const double e = __dadd_rn(x0, x1);
-                        q1 = fma(s0, e, q0);
-                        s1 = fma(q0, e, -s0);
-                    }
-#pragma unroll
-                    for (int n = 0; n < NC; ++n) {
-                        ar[u][n] = fma(v0[n], q0, fma(v1[n], q1, ar[u][n]));
-                        ai[u][n] = fma(v0[n], s0, fma(v1[n], s1, ai[u][n]));
-                    }
-                }
+            for (int n = 0; n < NC; ++n) {
+                v0[n] = tile[n * 32];
+                v1[n] = twin ? tile[(NC + n) * 32] : 0.0;
             }
-            if (A.n_cos & 1) {
-                const double m0 = -dta * s_c[half];
-#pragma unroll
-                for (int u = 0; u < NW; ++u) {
-                    double s0, q0;
-                    phase_of<BIG>(tab, __dmul_rn(wv[u], m0), s0, q0);
-#pragma unroll
-                    for (int n = 0; n < NC; ++n) {
-                        const double v = __ldg(b0 + (size_t)n * A.tp);
-                        ar[u][n] = fma(v, q0, ar[u][n]);
-                        ai[u][n] = fma(v, s0, ai[u][n]);
-                    }
-                }
-            }
-            const double tz = t - xa.z;
+            const double m0 = -dta * s_c[p], m1 = -dta * s_c[A.n_cos - 1 - p];
 #pragma unroll
             for (int u = 0; u < NW; ++u) {
-                double s0, q0;
-                phase_of<BIG>(tab, __dmul_rn(wv[u], tz), s0, q0);
+                const double x0 = __dmul_rn(wv[u], m0), x1 = __dmul_rn(wv[u], m1);
+                double s0, q0, s1, q1;
+                phase_of<BIG>(tab, x0, s0, q0);
+                if constexpr (BIG) {
+                    sincos(x1, &s1, &q1);
+                } else {
+                    // exact: the (rounded) arguments are opposite to a few ulp
+                    const double e = __dadd_rn(x0, x1);
+                    q1 = fma(s0, e, q0);
+                    s1 = fma(q0, e, -s0);
+                }
 #pragma unroll
                 for (int n = 0; n < NC; ++n) {
-                    cr[u][n] += ar[u][n] * q0 - ai[u][n] * s0;
-                    cim[u][n] += ar[u][n] * s0 + ai[u][n] * q0;
+                    ar[u][n] = fma(v0[n], q0, fma(v1[n], q1, ar[u][n]));
+                    ai[u][n] = fma(v0[n], s0, fma(v1[n], s1, ai[u][n]));
                 }
             }
         }
+        if (++st < per_unit) continue;
+        st = 0;
+        ++unit;
+        const double tz = t - xa.z;
+        double v[NV];
+#pragma unroll
+        for (int u = 0; u < NW; ++u) {
+            double s0, q0;
+            phase_of<BIG>(tab, __dmul_rn(wv[u], tz), s0, q0);
+#pragma unroll
+            for (int n = 0; n < NC; ++n) {
+                v[2 * (u * NC + n)] = ar[u][n] * q0 - ai[u][n] * s0;
+                v[2 * (u * NC + n) + 1] = ar[u][n] * s0 + ai[u][n] * q0;
+            }
+        }
+        if constexpr (PER_T) {
+#pragma unroll
+            for (int e = 0; e < NV; ++e) c_sum[e] += v[e];
+        } else {
+            c_sum[0] += lane_sums<NV>(v);
+        }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     const size_t W = A.n_w;
+    auto place = [&](int e) {  // (G, S, W) index of value e / 2
+        const int u = e / (2 * NC), col = c0 + (e / 2) % NC;
+        return ((size_t)(col % G) * A.S + col / G) * W + w0 + u;
+    };
     if constexpr (PER_T) {
-        const int k = A.k0 + 32 * b_lo + lane;
+        const int k = A.k0 + 32 * (int)fixed + lane;
         if (k >= A.k1) return;
-        double2* o = R.partial + (size_t)(blockIdx.x / nkc) * cols * W * A.n_t;
+        double2* o = R.partial + (size_t)(unit_block / nkc) * cols * W * A.n_t;
 #pragma unroll
-        for (int u = 0; u < NW; ++u)
-#pragma unroll
-            for (int n = 0; n < NC; ++n) {
-                const int col = c0 + n, g = col % G, s = col / G;
-                if (w0 + u < A.n_w)
-                    o[(((size_t)g * A.S + s) * W + w0 + u) * A.n_t + k] = make_double2(cr[u][n], cim[u][n]);
-            }
+        for (int e = 0; e < NV; e += 2)
+            if (w0 + e / (2 * NC) < A.n_w) o[place(e) * A.n_t + k] = make_double2(c_sum[e], c_sum[e + 1]);
     } else {
-        double2* o = R.partial + ((A.fs0 + f_lo) * R.n_parts + R.part0 + blockIdx.x % n_grp) * cols * W;
-#pragma unroll
-        for (int u = 0; u < NW; ++u)
-#pragma unroll
-            for (int n = 0; n < NC; ++n) {
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    cr[u][n] += __shfl_xor_sync(0xffffffffu, cr[u][n], off);
-                    cim[u][n] += __shfl_xor_sync(0xffffffffu, cim[u][n], off);
-                }
-                const int col = c0 + n, g = col % G, s = col / G;
-                if (lane == 0 && w0 + u < A.n_w)
-                    o[((size_t)g * A.S + s) * W + w0 + u] = make_double2(cr[u][n], cim[u][n]);
-            }
+        double* o = reinterpret_cast<double*>(
+            R.partial + ((A.fs0 + fixed) * R.n_parts + R.part0 + unit_block % n_grp) * cols * W);
+        const int e = lane_value<NV>(lane);
+        if (e >= 0 && w0 + e / (2 * NC) < A.n_w) o[2 * place(e) + (e & 1)] = c_sum[0];
     }
 }
 
@@ -540,29 +710,40 @@ DirArgs direct_args(const SpectrumJob& job, const DirectInputs& in) {
     return A;
 }
 
-template <int G, int NS>
+template <int G>
 void launch_b(const DirArgs& A, bool exact, cudaStream_t st) {
-    const size_t nkb = (A.k1 - A.k0 + 32 * NS - 1) / (32 * NS);
+    const size_t nkb = (A.k1 - A.k0 + kStepBlock - 1) / kStepBlock;
     const size_t blocks = (A.n_fs * A.n_cos * nkb + kDirWarps - 1) / kDirWarps;
     if (blocks > 0x7fffffffULL) throw Error{"direct kernel: too many (bubble, row, step) blocks for one launch"};
     if (exact)
-        k_direct_b<G, NS, true><<<(unsigned)blocks, 32 * kDirWarps, 0, st>>>(A);
+        k_direct_b<G, true><<<(unsigned)blocks, 32 * kDirWarps, 0, st>>>(A);
     else
-        k_direct_b<G, NS, false><<<(unsigned)blocks, 32 * kDirWarps, 0, st>>>(A);
+        k_direct_b<G, false><<<(unsigned)blocks, 32 * kDirWarps, 0, st>>>(A);
     CUDA_OK(cudaGetLastError());
 }
 
+// gx: (bubble, step block) units of the grid
 template <int NC, int NW, bool PER_T>
 void launch_a(const RowSumArgs& R, int G, size_t gx, bool big, cudaStream_t st) {
-    if (gx > 0x7fffffffULL) throw Error{"direct kernel: too many (bubble, step) blocks for one launch"};
-    const size_t gy = (R.d.n_w + NW * kDirWarps - 1) / (NW * kDirWarps);
-    if (gy > 65535) throw Error{"direct kernel: too many frequencies for one launch"};
-    const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)(R.d.S * G / NC));
-    const size_t smem = (size_t)R.d.n_cos * sizeof(double);
-    if (big)
-        k_direct_a<NC, NW, true, PER_T><<<grid, 32 * kDirWarps, smem, st>>>(R, G);
-    else
-        k_direct_a<NC, NW, false, PER_T><<<grid, 32 * kDirWarps, smem, st>>>(R, G);
+    const int groups = (R.d.n_w + NW - 1) / NW, warps = std::min(kDirWarps, groups);
+    const int w_tiles = (groups + warps - 1) / warps;
+    if (gx * w_tiles > 0x7fffffffULL) throw Error{"direct kernel: too many (bubble, step) blocks for one launch"};
+    const dim3 grid((unsigned)(gx * w_tiles), (unsigned)(R.d.S * G / NC));
+    const size_t smem = ((size_t)kRowStages * stage_pairs<NC>() * 2 * NC * 32 + R.d.n_cos) * sizeof(double);
+    auto* kernel = big ? k_direct_a<NC, NW, true, PER_T> : k_direct_a<NC, NW, false, PER_T>;
+    CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, 32 * warps, smem, st>>>(R, G, w_tiles);
+    CUDA_OK(cudaGetLastError());
+}
+
+// Step factors of the whole job (all steps, every radiating bubble).
+void launch_steps(Device* dev, DirArgs& A) {
+    A.tf = (A.n_t + kStepBlock - 1) / kStepBlock * kStepBlock;
+    dev->fact_D.ensure((size_t)A.n_sel * (1 + A.S * A.M) * A.tf * sizeof(double));
+    A.steps = (double*)dev->fact_D.p;
+    const dim3 g((unsigned)(A.tf / kStepBlock), (unsigned)std::min(A.n_sel, 65535), (unsigned)(A.n_sel / 65535 + 1));
+    if (g.z > 65535) throw Error{"too many radiating bubbles"};
+    k_direct_steps<<<g, kStepBlock, 0, dev->stream>>>(A);
     CUDA_OK(cudaGetLastError());
 }
 
@@ -593,10 +774,13 @@ uint64_t launch_direct(Device* dev, const SpectrumJob& job, const DirectInputs& 
     // B holds a range of pairs over a range of steps (whole groups of per_warp step blocks)
     const size_t group = (size_t)P.per_warp * 32;
     const size_t col_bytes = job.n_cos * cols * sizeof(double);
-    size_t steps = std::min<size_t>((size_t)P.n_parts, std::max<size_t>(1, kDirectBufferBytes / (col_bytes * group))) * group;
+    const size_t range = 4 * group;  // whole step blocks of k_direct_b too
+    const size_t steps = std::max<size_t>(1, std::min<size_t>((job.n_t + range - 1) / range,
+                                                              kDirectBufferBytes / (col_bytes * range))) * range;
     const size_t n_fs = std::min(pairs, std::max<size_t>(1, kDirectBufferBytes / (col_bytes * std::min(steps, (size_t)P.nkc * 32))));
     DirArgs A = direct_args(job, in);
-    uint64_t launches = 0;
+    launch_steps(dev, A);
+    uint64_t launches = 1;
     for (size_t k0 = 0; k0 < job.n_t; k0 += steps) {
         A.k0 = (int)k0;
         A.k1 = (int)std::min(job.n_t, k0 + steps);
@@ -607,9 +791,9 @@ uint64_t launch_direct(Device* dev, const SpectrumJob& job, const DirectInputs& 
             A.fs0 = f0;
             A.n_fs = std::min(n_fs, pairs - f0);
             if (job.tensor)
-                launch_b<6, 2>(A, exact, dev->stream);
+                launch_b<6>(A, exact, dev->stream);
             else
-                launch_b<2, 4>(A, exact, dev->stream);
+                launch_b<2>(A, exact, dev->stream);
             const RowSumArgs R{A, P.per_warp, P.n_parts, (int)(k0 / group), (double2*)dev->partial.p};
             const size_t groups = ((A.k1 - A.k0 + 31) / 32 + P.per_warp - 1) / P.per_warp;
             dispatch_a<false>(R, P, A.n_fs * groups, big, dev->stream);
@@ -630,7 +814,8 @@ uint64_t launch_direct_integrand(Device* dev, const SpectrumJob& job, const Dire
     const bool exact = direct_exact(job), big = direct_big(job);
     // B holds a range of bubbles over all steps, or one bubble over a range of steps
     const size_t step_bytes = job.n_cos * cols * 32 * sizeof(double);
-    const size_t nkc = std::min<size_t>(P.nkc, std::max<size_t>(1, kDirectBufferBytes / step_bytes));
+    // (a multiple of four 32-step blocks: whole step blocks of k_direct_b)
+    const size_t nkc = std::min<size_t>((P.nkc + 3) & ~3, std::max<size_t>(1, kDirectBufferBytes / (4 * step_bytes)) * 4);
     const size_t n_fs = std::min(pairs, std::max<size_t>(1, kDirectBufferBytes / (step_bytes * nkc)));
     // bubbles per warp: few enough for the chip to be full, as many as keep the partial outputs small
     const size_t warps = ((job.n_w + P.nw - 1) / P.nw) * (cols / P.nc) * P.nkc;
@@ -644,7 +829,8 @@ uint64_t launch_direct_integrand(Device* dev, const SpectrumJob& job, const Dire
     if (gx > 0x7fffffffULL) throw Error{"direct kernel: integrand too large for one launch"};
     DirArgs A = direct_args(job, in);
     A.B = (double*)dev->beta.p;
-    uint64_t launches = 0;
+    launch_steps(dev, A);
+    uint64_t launches = 1;
     for (size_t f0 = 0; f0 < pairs; f0 += n_fs) {
         A.fs0 = f0;
         A.n_fs = std::min(n_fs, pairs - f0);
@@ -654,9 +840,9 @@ uint64_t launch_direct_integrand(Device* dev, const SpectrumJob& job, const Dire
             A.k1 = (int)std::min(job.n_t, k0 + 32 * nkc);
             A.tp = (A.k1 - A.k0 + 31) & ~31;
             if (job.tensor)
-                launch_b<6, 2>(A, exact, dev->stream);
+                launch_b<6>(A, exact, dev->stream);
             else
-                launch_b<2, 4>(A, exact, dev->stream);
+                launch_b<2>(A, exact, dev->stream);
             const RowSumArgs R{A, P.per_warp, 0, 0, (double2*)dev->partial.p};
             dispatch_a<true>(R, P, parts * (size_t)(A.tp / 32), big, dev->stream);
             launches += 2;
