@@ -36,7 +36,7 @@ struct SpectrumJob {
     const double* dirs = nullptr;
     const double* sin2phi = nullptr;  // sin(2 phi_j)
     const double* cos2phi = nullptr;  // cos(2 phi_j)
-    const double* sinphi = nullptr;   // sin(phi_j), cos(phi_j): the tensor form
+    const double* sinphi = nullptr;   // sin(phi_j), cos(phi_j)
     const double* cosphi = nullptr;
     bool tensor = false;              // NewGeneralizedBulkFlow: (6, S, W) per k-hat, FP64 direct only
     // scaling functions
@@ -104,6 +104,8 @@ struct MaskJob {
     size_t n_int = 0, n_tot = 0;
     size_t n_cos = 0, n_phi = 0;
     const double* dirs = nullptr;
+    const double* sinphi = nullptr;  // sin(phi_j), cos(phi_j)
+    const double* cosphi = nullptr;
     const uint32_t* sel = nullptr;
     size_t n_sel = 0;
 };

@@ -911,6 +911,8 @@ BgwStatus bgwx_generalized_bulk_flow_first_colliding(bgw_generalized_bulk_flow* 
         job.n_cos = h->n_cos;
         job.n_phi = h->n_phi;
         job.dirs = h->dirs.data();
+        job.sinphi = h->sinphi.data();
+        job.cosphi = h->cosphi.data();
         job.sel = ids.data();
         job.n_sel = n;
         h->timings = BgwxTimings{};

@@ -79,6 +79,7 @@ struct Device {
     std::vector<cudaEvent_t> fact_ev;   // 3 per k-hat chunk: before beta, before GEMM, after GEMM
     DevBuf bub, bubrot, dirs, cos_t, sin2, cos2, coeffs, powers, t_arr, cutw, w, sel, rot, cosphi, sinphi;
     DevBuf tau, codes, partial, out, counters, nblists;
+    DevBuf mask_open;  // mask search: per block, whether it left directions to the second kernel
     DevBuf ranges, real_tiles;  // batched jobs: per-slot realization rows, first tile per realization
     DevBuf fact_D, fact_kfirst, beta, fact_partial;  // factored-kernel work arrays
     DevBuf ens_out;                                  // batched ensemble: all realizations' spectra
@@ -112,7 +113,7 @@ struct Device {
     unsigned long long buffers_generation() const {
         unsigned long long g = 0;
         for (const DevBuf* b : {&bub, &bubrot, &dirs, &cos_t, &sin2, &cos2, &coeffs, &powers, &t_arr, &cutw, &w, &sel,
-                                &rot, &cosphi, &sinphi, &tau, &codes, &partial, &out, &counters, &nblists, &ranges,
+                                &rot, &cosphi, &sinphi, &tau, &codes, &partial, &out, &counters, &nblists, &mask_open, &ranges,
                                 &real_tiles, &fact_D, &fact_kfirst, &beta, &fact_partial, &ens_out, &beta_scale,
                                 &fact_Dmax, &tc_atab})
             g += b->gen;

@@ -154,13 +154,15 @@ void run_masks(Device* dev, const MaskJob& job, int32_t* out_codes, double* out_
     D4* bub = reinterpret_cast<D4*>(upload(dev, dev->bub, job.bubbles, 4 * job.n_tot, tm));
     D4* dirs = reinterpret_cast<D4*>(upload(dev, dev->dirs, job.dirs, 4 * nd, tm));
     uint32_t* sel = upload(dev, dev->sel, job.sel, job.n_sel, tm);
+    double* cosphi = upload(dev, dev->cosphi, job.cosphi, job.n_phi, tm);
+    double* sinphi = upload(dev, dev->sinphi, job.sinphi, job.n_phi, tm);
     dev->tau.ensure(job.n_sel * nd * sizeof(double));
     dev->codes.ensure(job.n_sel * nd * sizeof(int32_t));
     dev->counters.ensure(64);
     CUDA_OK(cudaMemsetAsync(dev->counters.p, 0, 64, dev->stream));
     CUDA_OK(cudaEventRecord(dev->ev[0], dev->stream));
     uint64_t nl = 0;
-    launch_mask_pipeline(dev, bub, bub, job.n_int, job.n_tot, sel, nullptr, job.n_sel, dirs, nd, job.n_phi, 1, (double*)dev->tau.p,
+    launch_mask_pipeline(dev, bub, bub, job.n_int, job.n_tot, sel, nullptr, job.n_sel, dirs, cosphi, sinphi, nd, job.n_phi, 1, (double*)dev->tau.p,
                          (int32_t*)dev->codes.p, (unsigned long long*)dev->counters.p, true, &nl);
     CUDA_OK(cudaEventRecord(dev->ev[1], dev->stream));
     CUDA_OK(cudaMemcpyAsync(out_codes, dev->codes.p, job.n_sel * nd * sizeof(int32_t), cudaMemcpyDeviceToHost,
@@ -265,8 +267,8 @@ void run_spectrum(Device* dev, const SpectrumJob& job, double* out, bool out_is_
         batched ? reinterpret_cast<const uint2*>(upload(dev, dev->ranges, job.ranges, 2 * job.n_sel, tm)) : nullptr;
     const uint32_t* real_tiles = batched ? upload(dev, dev->real_tiles, job.real_tiles, job.n_real + 1, tm) : nullptr;
     const size_t out_blocks = batched ? job.n_real * K : K;  // (realization,) frame blocks of the output
-    double* cosphi = job.tensor ? upload(dev, dev->cosphi, job.cosphi, job.n_phi, tm) : nullptr;
-    double* sinphi = job.tensor ? upload(dev, dev->sinphi, job.sinphi, job.n_phi, tm) : nullptr;
+    double* cosphi = upload(dev, dev->cosphi, job.cosphi, job.n_phi, tm);
+    double* sinphi = upload(dev, dev->sinphi, job.sinphi, job.n_phi, tm);
     if (uploads_only) return;  // the inputs are resident; a captured launch sequence follows
 
     // frames per chunk: bounded by the mask buffer budget (and by the job's launch shape)
@@ -325,7 +327,7 @@ void run_spectrum(Device* dev, const SpectrumJob& job, double* out, bool out_is_
         record_event(dev, cev[0]);
         double* tau_k = keep ? (double*)dev->kept_tau.p + k0 * job.n_sel * nd : (double*)dev->tau.p;
         int32_t* codes_k = keep ? (int32_t*)dev->kept_codes.p + k0 * job.n_sel * nd : nullptr;
-        launch_mask_pipeline(dev, bub, fb, job.n_int, job.n_tot, sel, ranges, job.n_sel, dirs, nd, job.n_phi, kn,
+        launch_mask_pipeline(dev, bub, fb, job.n_int, job.n_tot, sel, ranges, job.n_sel, dirs, cosphi, sinphi, nd, job.n_phi, kn,
                              tau_k, codes_k, (unsigned long long*)dev->counters.p, k0 == 0, &launches,
                              job.mask_chunking);
         record_event(dev, cev[1]);
@@ -553,6 +555,8 @@ void run_adjoint(Device* dev, const SpectrumJob& job, const double* gbar, double
     double* w = upload(dev, dev->w, job.w, W, tm);
     uint32_t* sel = upload(dev, dev->sel, job.sel, job.n_sel, tm);
     double* rot = job.rot ? upload(dev, dev->rot, job.rot, 9 * K, tm) : nullptr;
+    double* cosphi = upload(dev, dev->cosphi, job.cosphi, job.n_phi, tm);
+    double* sinphi = upload(dev, dev->sinphi, job.sinphi, job.n_phi, tm);
     double2* gb = reinterpret_cast<double2*>(upload(dev, dev->adj_gbar, gbar, 2 * K * per, tm));
 
     const size_t per_k = adjoint_bytes_per_frame(job);
@@ -610,7 +614,7 @@ void run_adjoint(Device* dev, const SpectrumJob& job, const double* gbar, double
         const int32_t* codes_k =
             reuse ? (const int32_t*)dev->kept_codes.p + k0 * job.n_sel * nd : (const int32_t*)dev->codes.p;
         if (!reuse)
-            launch_mask_pipeline(dev, bub, fb, job.n_int, job.n_tot, sel, nullptr, job.n_sel, dirs, nd, job.n_phi, kn,
+            launch_mask_pipeline(dev, bub, fb, job.n_int, job.n_tot, sel, nullptr, job.n_sel, dirs, cosphi, sinphi, nd, job.n_phi, kn,
                                  (double*)dev->tau.p, (int32_t*)dev->codes.p, (unsigned long long*)dev->counters.p,
                                  k0 == 0, &launches);
         launches += launch_adjoint_chunk(dev, job, fb, sel, tau_k, codes_k,
@@ -649,15 +653,15 @@ void run_integrand(Device* dev, const SpectrumJob& job, double* out, BgwxTimings
     double* cutw = upload(dev, dev->cutw, job.cutoff, T, tm);
     double* w = upload(dev, dev->w, job.w, W, tm);
     uint32_t* sel = upload(dev, dev->sel, job.sel, job.n_sel, tm);
-    double* cosphi = job.tensor ? upload(dev, dev->cosphi, job.cosphi, job.n_phi, tm) : nullptr;
-    double* sinphi = job.tensor ? upload(dev, dev->sinphi, job.sinphi, job.n_phi, tm) : nullptr;
+    double* cosphi = upload(dev, dev->cosphi, job.cosphi, job.n_phi, tm);
+    double* sinphi = upload(dev, dev->sinphi, job.sinphi, job.n_phi, tm);
     dev->tau.ensure(job.n_sel * nd * sizeof(double));
     dev->out.ensure(per * sizeof(double2));
     dev->counters.ensure(64);
     CUDA_OK(cudaMemsetAsync(dev->counters.p, 0, 64, dev->stream));
     uint64_t launches = 0;
     CUDA_OK(cudaEventRecord(dev->ev[4], dev->stream));
-    launch_mask_pipeline(dev, bub, bub, job.n_int, job.n_tot, sel, nullptr, job.n_sel, dirs, nd, job.n_phi, 1, (double*)dev->tau.p,
+    launch_mask_pipeline(dev, bub, bub, job.n_int, job.n_tot, sel, nullptr, job.n_sel, dirs, cosphi, sinphi, nd, job.n_phi, 1, (double*)dev->tau.p,
                          nullptr, (unsigned long long*)dev->counters.p, true, &launches);
     const DirectInputs in{bub,    sel,    (const double*)dev->tau.p, cos_t,  sin2, cos2, sinphi, cosphi,
                           coeffs, powers, t_arr,                     cutw,   w};
