@@ -58,40 +58,43 @@ constexpr int kThreads = 256;
 constexpr int kTM = 8;           // register tile rows per thread (columns: TN = 8 FP32, 4 FP64)
 
 // ---------------------------------------------------------------------------
+// Step factors of a bubble, table row q over steps at ((slot (1 + SM) + q) tf + k): row 0 the step weight
+// (time cutoff x trapezoid end weight) times dt^3, row 1 + q the same times a_q dt^{3-p_q} e^{-dt/width};
+// zero where dt <= 0 and past n_t (tf is n_t rounded up to whole blocks of 32 steps).
 __global__ void k_time_tables(const D4* __restrict__ bub, const uint32_t* __restrict__ sel, int n_sel,
-                              const double* __restrict__ t_arr, int n_t, const double* __restrict__ powers,
+                              const double* __restrict__ t_arr, int n_t, int tf, const double* __restrict__ powers,
                               const double* __restrict__ coeffs, const double* __restrict__ cutw, int SM,
                               int has_damp, double damp, double* __restrict__ D, int* __restrict__ kfirst) {
     const int slot = blockIdx.x;
     const int k = blockIdx.y * blockDim.x + threadIdx.x;
-    if (slot >= n_sel || k >= n_t || sel[slot] == kNoSlot) return;
+    if (slot >= n_sel || k >= tf || sel[slot] == kNoSlot) return;
     const double ta = bub[sel[slot]].t;
-    const double dt = t_arr[k] - ta;
-    double* row = D + ((size_t)slot * n_t + k) * (1 + SM);
+    const double dt = k < n_t ? t_arr[k] - ta : 0.0;
+    double* row = D + (size_t)slot * (1 + SM) * tf + k;
     const bool on = dt > 0.0;
-    // step weight (time cutoff x trapezoid end weight) folded into the table
-    const double wk = cutw[k] * ((k == 0 || k == n_t - 1) ? 0.5 : 1.0);
+    const double wk = k < n_t ? cutw[k] * ((k == 0 || k == n_t - 1) ? 0.5 : 1.0) : 0.0;
     const double d3 = on ? dt * (dt * dt) : 0.0;
     row[0] = wk * d3;
     const double e = has_damp ? exp(-dt / damp) : 1.0;
-    for (int q = 0; q < SM; ++q) row[1 + q] = d3 != 0.0 ? wk * coeffs[q] * (pow(dt, 3.0 - powers[q]) * e) : 0.0;
+    for (int q = 0; q < SM; ++q)
+        row[(size_t)(1 + q) * tf] = d3 != 0.0 ? wk * coeffs[q] * (pow(dt, 3.0 - powers[q]) * e) : 0.0;
+    if (k >= n_t) return;
     // first active step (t_a <= t_k and dt > 0): monotone in k
     if (on && (k == 0 || !(t_arr[k - 1] - ta > 0.0))) kfirst[slot] = k;
     if (k == n_t - 1 && !on) kfirst[slot] = n_t;
 }
 
 // Per (bubble, block of 32 steps): the least and the largest D_q(k) of each
-// table column over the block's steps k < n_t (one warp, lane = step), stored
-// as (min, max) pairs.
-__global__ void k_time_maxima(const double* __restrict__ D, int n_sel, int n_t, int nblk, int Q,
+// table row over the block's steps (one warp, lane = step), stored as (min, max)
+// pairs.
+__global__ void k_time_maxima(const double* __restrict__ D, int n_sel, int tf, int nblk, int Q,
                               double* __restrict__ Dmax) {
     const long wid = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (wid >= (long)n_sel * nblk) return;
     const int slot = (int)(wid / nblk), b = (int)(wid % nblk);
-    const int k = (b << 5) + lane;
     for (int q = 0; q < Q; ++q) {
-        const double v = k < n_t ? D[((size_t)slot * n_t + k) * Q + q] : 0.0;
+        const double v = D[((size_t)slot * Q + q) * tf + (b << 5) + lane];
         double lo = v, hi = v;
         for (int o = 16; o > 0; o >>= 1) {
             lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
@@ -107,13 +110,23 @@ __global__ void k_time_maxima(const double* __restrict__ D, int n_sel, int n_t, 
 // ---------------------------------------------------------------------------
 // k_beta: one warp per row (frame, slot, i).  The row's collided patches
 // become events at the first step k_j with (t_k - t_a) >= tau_j (exact FP64
-// comparisons, GBF:405), counting-sorted (stable in j) into blocks of 32
-// steps.  Block b covers k = 32 b + lane: each lane gathers its step's event
-// weights, a warp inclusive scan gives the collided sums Pm(k) and a warp
-// exclusive suffix scan plus the backward block totals gives the uncollided
-// sums U(k) -- both are sums of the terms they stand for, never differences.
+// comparisons, GBF:405).  Before the row's first event and after its last the
+// collided sums Pm and the uncollided sums U are constant ("quiet" steps, two
+// sets of constants); in between the steps are formed in segments of 128, from
+// the first event's block of 32 on: every event's weights are added to its
+// step's bin in shared memory (events of one step one after another, in lane
+// order), and warp scans, lane = 4 consecutive steps, give Pm(k) as a prefix and
+// U(k) as a suffix sum -- both are sums of the terms they stand for, never
+// differences (a difference cancels catastrophically once most patches have
+// collided).  At 192 phi patches and 1024 steps a row's events span about two
+// blocks, so one segment holds them.
 // beta(k) = rf_i u_k cut_k [dt^3 U(k) + sum_m a_m dt^{3-p_m} e^{-dt/w} Pm(k)]
 // is written to beta[frame][i][col][k], col = slot*2S + 2s + g.
+//
+// What bounds it: issue.  Sorting the events into blocks and again into steps,
+// with totals and scans over every block, took two thirds of 62.8 ms for 8
+// frames of 4096 bubbles x 192 rows; the digits and stores of the quiet steps a
+// quarter.
 struct BetaArgs {
     const double* tau;     // (kn, n_sel, n_cos*n_phi)
     const D4* bub;         // bubbles (frame 0; times are frame independent)
@@ -126,7 +139,8 @@ struct BetaArgs {
     const double* sin2;
     const double* powers;  // (S*M)
     const double* coeffs;  // (S*M)
-    const double* D;       // (n_sel, n_t, 1+S*M)
+    const double* D;       // (n_sel, 1+S*M, tf) step factors
+    int tf;
     int has_damp;
     double damp;
     double dphi, dcos, dt;
@@ -136,652 +150,489 @@ struct BetaArgs {
     int tile_cols;         // columns of one GEMM tile
     int bpt;               // bubbles per tile
     int t_pad;             // row length of beta
-    int per_warp_bytes;
+    int keep;              // event segments whose bins a warp holds at once
+    int per_warp;          // doubles of shared memory per warp
     int tiles;             // column tiles per frame (int8 digit layout)
     double* scale;         // int8 digit layout: (kn, n_sel, n_cos) row scales, max |beta| of the row
     const double* Dmax;    // int8 digit layout: (n_sel, nblk, 1+S*M, 2) least and largest D over each block's steps
 };
 
+constexpr int kSegBlocks = 4;              // blocks of 32 steps in an event segment
+constexpr int kSeg = 32 * kSegBlocks;
+
+// blocks per SM: three at 80 registers with one term, two with two
 template <class Real, int SMC>
-__global__ void __launch_bounds__(256, std::is_same<Real, int8_t>::value ? 3 : 1) k_beta(BetaArgs A, Real* __restrict__ beta) {
-    extern __shared__ __align__(16) unsigned char sm_b[];
-    constexpr int NQ = 2 + 2 * SMC;
+__global__ void __launch_bounds__(256, SMC == 1 ? 3 : SMC == 2 ? 2 : 1) k_beta(BetaArgs A, Real* __restrict__ beta) {
+    extern __shared__ __align__(16) double sm_b[];
+    constexpr bool kI8 = std::is_same<Real, int8_t>::value;
+    constexpr int NQ = 2 + 2 * SMC;  // weights of an event: cos, sin; then cos and sin times each term's factor
+    constexpr unsigned full = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long row = (long)blockIdx.x * (blockDim.x >> 5) + warp;
-    if (row >= A.n_rows) return;
     const int NB = A.nblk;
-    const int EV = A.n_phi;  // event capacity: one event per patch at most
-    unsigned char* base = sm_b + (size_t)warp * A.per_warp_bytes;
-    double* evq = reinterpret_cast<double*>(base);             // [NQ][n_phi]: weight q of event e at q * n_phi + e
-    double* btot = evq + (size_t)A.n_phi * NQ;                  // [NQ][NB] block totals
-    double* uend = btot + (size_t)NQ * NB;                      // [NB][2] uncollided after block
-    double* pbeg = uend + 2 * NB;                               // [NB][2 SMC] collided before block
-    int* boff = reinterpret_cast<int*>(pbeg + (size_t)2 * SMC * NB);  // [NB+1]
-    int* brun = boff + NB + 1;                                  // [NB]
-    uint8_t* evs = reinterpret_cast<uint8_t*>(brun + NB);       // [n_phi + 4] step of each event within its block
-    // a crowded event block's per-step counts and running offsets [2][32], and its events in step order [n_phi]
-    int* scnt = reinterpret_cast<int*>(evs + ((A.n_phi + 4 + 3) & ~3));
-    uint16_t* sperm = reinterpret_cast<uint16_t*>(scnt + 64);
+    // Lane l holds the patches [c l, c l + c): neighbouring patches collide at the same or the next step,
+    // so most of a step's events are added up in registers before they reach its bin.  Their rows in shared
+    // memory have an odd pitch (no bank conflicts).
+    const int c_pat = (A.n_phi + 31) >> 5, pitch = c_pat | 1;
+    double2* s_wgt = reinterpret_cast<double2*>(sm_b);                       // [32 pitch] weights, block's own
+    double* base_w = sm_b + 64 * pitch + (size_t)warp * A.per_warp;
+    double* bins = base_w;                                                   // [keep][NQ][kSeg]
+    double* s_const = bins + (size_t)A.keep * NQ * kSeg;                     // [4 + 2 SMC] quiet constants
+    double* s_tau = s_const + 4 + 2 * SMC;                                   // [32 pitch] delays
+    int* s_kj = reinterpret_cast<int*>(s_tau + 32 * pitch);                  // [32 pitch] first collided steps
+    for (int j = threadIdx.x; j < A.n_phi; j += blockDim.x) {
+        const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
+        s_wgt[j / c_pat * pitch + j % c_pat] = make_double2(wj * A.cos2[j], wj * A.sin2[j]);
+    }
+    __syncthreads();
+    if (row >= A.n_rows) return;
     const int slot = (int)((row / A.n_cos) % A.n_sel);
     if (A.sel[slot] == kNoSlot) return;  // a padding slot of a batched job: its columns are never read
     const int i = (int)(row % A.n_cos);
     const long frame = row / ((long)A.n_cos * A.n_sel);
     const double* trow = A.tau + (size_t)row * A.n_phi;
-    // The delays of patches j = lane + 32 jj, jj < kMaxJ, are loaded first, all at once (one
-    // memory latency for the row), and kept for both passes over the patches.
-    constexpr int kMaxJ = 6;
-    double tj_c[kMaxJ];
-#pragma unroll
-    for (int jj = 0; jj < kMaxJ; ++jj) {
-        const int j = 32 * jj + lane;
-        tj_c[jj] = j < A.n_phi ? __ldcs(trow + j) : 0.0;
-    }
     const double ta = A.bub[A.sel[slot]].t;
-    const unsigned full = 0xffffffffu;
     const double inv_dt = 1.0 / A.dt;  // the estimate below is only a starting point
-    auto block_of = [&](int j, double tj, int& kj) -> int {
-        kj = A.n_t;
-        if (j >= A.n_phi) return -2;  // not a patch
-        if (!(tj > 0.0)) return -1;    // never collides
+    constexpr int kNever = 0x7fffffff;
+    auto step_of = [&](double tj) -> int {
+        if (!(tj > 0.0)) return kNever;
         // first k with (t_k - t_a) >= tau_j: arithmetic estimate, then exact
         // comparisons (the predicate is monotone in k) settle the boundary
         const double est = ceil((ta + tj - A.t_arr[0]) * inv_dt);
         int lo = est < 0.0 ? 0 : (est > (double)A.n_t ? A.n_t : (int)est);
         while (lo > 0 && A.t_arr[lo - 1] - ta >= tj) --lo;
         while (lo < A.n_t && !(A.t_arr[lo] - ta >= tj)) ++lo;
-        kj = lo;
-        return lo < A.n_t ? lo >> 5 : -1;
+        return lo < A.n_t ? lo : kNever;
     };
-    for (int b = lane; b < NB; b += 32) boff[b] = 0;
-    __syncwarp();
-    // pass 1: events per block; never-colliding weights (lane sums, fixed-order reduction).
-    // The first collided step of patches j = lane + 32 jj, jj < kMaxJ, is kept for pass 2.
-    int kj_c[kMaxJ], b_c[kMaxJ];
-    double nc = 0.0, ns = 0.0;
-    auto pass1 = [&](int j, int b) {
-        if (b == -1) {
-            const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
-            nc += wj * A.cos2[j];
-            ns += wj * A.sin2[j];
-        }
-        const unsigned m = __match_any_sync(full, b);
-        if (b >= 0 && lane == __ffs(m) - 1) boff[b] += __popc(m);
-        __syncwarp();
-    };
-#pragma unroll
-    for (int jj = 0; jj < kMaxJ; ++jj) {
-        if (32 * jj >= A.n_phi) break;
-        const int j = 32 * jj + lane;
-        kj_c[jj] = 0;
-        b_c[jj] = block_of(j, tj_c[jj], kj_c[jj]);
-        pass1(j, b_c[jj]);
-    }
-    for (int j0 = 32 * kMaxJ; j0 < A.n_phi; j0 += 32) {
-        int kj;
-        const int j = j0 + lane;
-        const int b = block_of(j, j < A.n_phi ? trow[j] : 0.0, kj);
-        pass1(j, b);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        nc += __shfl_down_sync(full, nc, o);
-        ns += __shfl_down_sync(full, ns, o);
-    }
-    // block counts -> first event of each block: an exclusive warp scan over 32 blocks at a time
-    {
-        int carry = 0;
-        for (int bc = 0; bc < NB; bc += 32) {
-            const int b = bc + lane;
-            const int c = b < NB ? boff[b] : 0;
-            int incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(full, incl, o);
-                if (lane >= o) incl += t;
-            }
-            if (b < NB) {
-                boff[b] = carry + incl - c;
-                brun[b] = carry + incl - c;
-            }
-            carry += __shfl_sync(full, incl, 31);
-        }
-        __syncwarp();
-        if (lane == 0) boff[NB] = carry;
+    int k_lo = kNever, k_hi = -1;
+#pragma unroll 2
+    for (int j = lane; j < A.n_phi; j += 32) {
+        const double tj = __ldcs(trow + j);
+        const int kj = step_of(tj), at = j / c_pat * pitch + j % c_pat;
+        s_tau[at] = tj;
+        s_kj[at] = kj;
+        k_lo = min(k_lo, kj);
+        if (kj != kNever) k_hi = max(k_hi, kj);
     }
     __syncwarp();
-    // pass 2: scatter events (stable in j within a block)
-    const unsigned lt = (1u << lane) - 1u;
-    auto pass2 = [&](int j, double tj, int kj, int b) {
-        const unsigned m = __match_any_sync(full, b);
-        int pos = 0;
-        if (b >= 0) pos = brun[b] + __popc(m & lt);
+    const int n_own = max(0, min(c_pat, A.n_phi - lane * c_pat));  // this lane's patches
+    const int own = lane * pitch;
+    k_lo = __reduce_min_sync(full, k_lo);
+    k_hi = __reduce_max_sync(full, k_hi);
+    // event segments: blocks [b_ev, b_ev + 4 n_seg); without events none, and every block is "before"
+    const int b_ev = k_hi < 0 ? NB : k_lo >> 5;
+    const int n_seg = k_hi < 0 ? 0 : ((k_hi >> 5) - b_ev) / kSegBlocks + 1;
+    const int b_aft = min(NB, b_ev + kSegBlocks * n_seg);
+    const double ci = A.cos_t[i];
+    const double vi = (i == 0 || i == A.n_cos - 1) ? 0.5 : 1.0;
+    const double rf = (0.5 * (1.0 - ci * ci) * A.dphi) * (A.dcos * vi) * A.dt * (1.0 / (6.0 * CUDART_PI));
+    const double* Dslot = A.D + (size_t)slot * (1 + SMC) * A.tf;
+    // constants of the quiet steps: uncollided sums before (0, 1) and after (2, 3) the events, collided sums
+    // after them (4 ..); held in shared memory
+    if (n_seg == 0) {
+        double u0 = 0.0, u1 = 0.0;
+        for (int m = 0; m < n_own; ++m) {
+            u0 += s_wgt[own + m].x;
+            u1 += s_wgt[own + m].y;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            u0 += __shfl_xor_sync(full, u0, o);
+            u1 += __shfl_xor_sync(full, u1, o);
+        }
+        if (lane < 4 + 2 * SMC) s_const[lane] = lane == 0 ? u0 : lane == 1 ? u1 : 0.0;
         __syncwarp();
-        if (b >= 0 && lane == __ffs(m) - 1) brun[b] += __popc(m);
+    }
+    // The running sums of segment g into bins w: rows 0, 1 the uncollided sums U after each step, the
+    // others the collided sums Pm up to it (lane: steps 4 lane .. 4 lane + 3).
+    auto form = [&](int g, double* w) {
+        const int s0 = (b_ev + g * kSegBlocks) << 5, s1 = s0 + kSeg;
+        double2* wz = reinterpret_cast<double2*>(w);
+        for (int q = lane; q < NQ * kSeg / 2; q += 32) wz[q] = make_double2(0.0, 0.0);
         __syncwarp();
-        if (b >= 0) {
-            evs[pos] = (uint8_t)(kj & 31);
-            const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
-            const double qc = wj * A.cos2[j], qs = wj * A.sin2[j];
-            double* q = evq + pos;
-            q[0] = qc;
-            q[EV] = qs;
+        double base[NQ];  // uncollided after the segment, collided before it
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) base[q] = 0.0;
+        double run[NQ];  // the lane's current run of patches with one collision step
+        int k_run = -1;
+        for (int m = 0; m <= c_pat; ++m) {
+            const int kj = m < n_own ? s_kj[own + m] : kNever;
+            const bool flush = k_run >= 0 && kj != k_run;
+            if (__any_sync(full, flush)) {
+                const unsigned same = __match_any_sync(full, flush ? k_run : -1 - lane);
+                const int rank = flush ? __popc(same & ((1u << lane) - 1u)) : -1;
+                const int rounds = __reduce_max_sync(full, rank);
+                for (int r = 0; r <= rounds; ++r) {
+                    if (rank == r) {
+                        double* e = w + (k_run - s0);
+#pragma unroll
+                        for (int q = 0; q < NQ; ++q) e[q * kSeg] += run[q];
+                    }
+                    __syncwarp();
+                }
+                if (flush) k_run = -1;
+            }
+            if (m >= n_own) continue;
+            double x[NQ];
+            const double2 wg = s_wgt[own + m];
+            x[0] = wg.x;
+            x[1] = wg.y;
+            if (kj >= s1) {
+                base[0] += x[0];
+                base[1] += x[1];
+                continue;
+            }
+            const double tj = s_tau[own + m];
             const double ed = A.has_damp ? exp(tj / A.damp) : 1.0;
 #pragma unroll
             for (int t = 0; t < SMC; ++t) {
                 const double f = tpow(tj, A.powers[t]) * ed;
-                q[(2 + 2 * t) * EV] = qc * f;
-                q[(3 + 2 * t) * EV] = qs * f;
+                x[2 + 2 * t] = x[0] * f;
+                x[3 + 2 * t] = x[1] * f;
+            }
+            if (kj < s0) {
+#pragma unroll
+                for (int q = 2; q < NQ; ++q) base[q] += x[q];
+            } else if (k_run < 0) {
+                k_run = kj;
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) run[q] = x[q];
+            } else {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) run[q] += x[q];
             }
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) base[q] += __shfl_xor_sync(full, base[q], o);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            double2* e = reinterpret_cast<double2*>(w + q * kSeg + 4 * lane);
+            const double2 lo = e[0], hi = e[1];
+            if (q < 2) {  // the sum of the later steps' events
+                const double v2 = hi.y, v1 = hi.x + v2, v0 = lo.y + v1;
+                double run = lo.x + v0;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double t = __shfl_down_sync(full, run, o);
+                    if (lane + o < 32) run += t;
+                }
+                double later = __shfl_down_sync(full, run, 1);
+                if (lane == 31) later = 0.0;
+                later += base[q];
+                e[0] = make_double2(v0 + later, v1 + later);
+                e[1] = make_double2(v2 + later, later);
+                if (g == 0 && lane == 0) s_const[q] = run + base[q];
+                if (g == n_seg - 1 && lane == 0) s_const[2 + q] = base[q];
+            } else {  // this step's and the earlier ones'
+                const double v0 = lo.x, v1 = v0 + lo.y, v2 = v1 + hi.x, v3 = v2 + hi.y;
+                double run = v3;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double t = __shfl_up_sync(full, run, o);
+                    if (lane >= o) run += t;
+                }
+                double before = __shfl_up_sync(full, run, 1);
+                if (lane == 0) before = 0.0;
+                before += base[q];
+                e[0] = make_double2(v0 + before, v1 + before);
+                e[1] = make_double2(v2 + before, v3 + before);
+                if (g == n_seg - 1 && lane == 31) s_const[2 + q] = run + base[q];
+            }
+        }
+        __syncwarp();
     };
+    // table row q at the lane's four steps of the blocks from b on
+    auto factors = [&](int q, int b, double (&v)[4]) {
+        const double2* d = reinterpret_cast<const double2*>(Dslot + (size_t)q * A.tf + (b << 5) + 4 * lane);
+        const double2 lo = __ldg(d), hi = __ldg(d + 1);
+        v[0] = lo.x;
+        v[1] = lo.y;
+        v[2] = hi.x;
+        v[3] = hi.y;
+    };
+    // beta of set s at the lane's steps of segment g from its bins
+    auto seg_values = [&](int g, const double* w, int s, double (&xc)[4], double (&xs)[4]) {
+        const int b = b_ev + g * kSegBlocks;
+        const bool on = b + (lane >> 3) < NB;
+        double d[4] = {0.0, 0.0, 0.0, 0.0};
+        if (on) factors(0, b, d);
 #pragma unroll
-    for (int jj = 0; jj < kMaxJ; ++jj) {
-        if (32 * jj >= A.n_phi) break;
-        pass2(32 * jj + lane, tj_c[jj], kj_c[jj], b_c[jj]);
-    }
-    for (int j0 = 32 * kMaxJ; j0 < A.n_phi; j0 += 32) {
-        int kj;
-        const int j = j0 + lane;
-        const double tj = j < A.n_phi ? trow[j] : 0.0;
-        const int b = block_of(j, tj, kj);
-        pass2(j, tj, kj, b);
-    }
-    __syncwarp();
-    // block totals of every weight: the lanes take a block's events in strides
-    // of 32 and a butterfly reduction adds the lane sums (a fixed order for a
-    // given event count); then the collided sums before each block (exclusive
-    // prefix over blocks) and the uncollided sums after each block (exclusive
-    // suffix plus the never-colliding weights), as warp scans over lanes = blocks
-    for (int b = lane; b < NB; b += 32)
-        if (boff[b] == boff[b + 1]) {
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) btot[(size_t)q * NB + b] = 0.0;
+        for (int m = 0; m < 4; ++m) {
+            xc[m] = d[m] * w[4 * lane + m];
+            xs[m] = d[m] * w[kSeg + 4 * lane + m];
         }
-    for (int bc = 0; bc < NB; bc += 32) {
-        const int bl = bc + lane;
-        for (unsigned h = __ballot_sync(full, bl < NB && boff[bl] != boff[bl + 1]); h; h &= h - 1) {
-            const int b = bc + __ffs(h) - 1;
-            double t[NQ];
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) t[q] = 0.0;
-            for (int e = boff[b] + lane; e < boff[b + 1]; e += 32) {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) t[q] += evq[(size_t)q * EV + e];
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) t[q] += __shfl_xor_sync(full, t[q], o);
-            }
-            if (lane == 0) {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) btot[(size_t)q * NB + b] = t[q];
-            }
-        }
-    }
-    __syncwarp();
-    {
-        double carry[2 * SMC];
-#pragma unroll
-        for (int q = 0; q < 2 * SMC; ++q) carry[q] = 0.0;
-        for (int bc = 0; bc < NB; bc += 32) {
-            const int b = bc + lane;
-            double v[2 * SMC];
-#pragma unroll
-            for (int q = 0; q < 2 * SMC; ++q) v[q] = b < NB ? btot[(size_t)(2 + q) * NB + b] : 0.0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-                for (int q = 0; q < 2 * SMC; ++q) {
-                    const double u = __shfl_up_sync(full, v[q], o);
-                    if (lane >= o) v[q] += u;
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 2 * SMC; ++q) {
-                double ex = __shfl_up_sync(full, v[q], 1);
-                if (lane == 0) ex = 0.0;
-                if (b < NB) pbeg[(size_t)b * 2 * SMC + q] = carry[q] + ex;
-                carry[q] += __shfl_sync(full, v[q], 31);
-            }
-        }
-        // the never-colliding sums were reduced into lane 0
-        double cc = __shfl_sync(full, nc, 0), cs = __shfl_sync(full, ns, 0);
-        for (int bc = ((NB - 1) >> 5) << 5; bc >= 0; bc -= 32) {
-            const int b = bc + lane;
-            double vc = b < NB ? btot[b] : 0.0, vs = b < NB ? btot[(size_t)NB + b] : 0.0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const double uc = __shfl_down_sync(full, vc, o), us = __shfl_down_sync(full, vs, o);
-                if (lane + o < 32) {
-                    vc += uc;
-                    vs += us;
-                }
-            }
-            double xc = __shfl_down_sync(full, vc, 1), xs = __shfl_down_sync(full, vs, 1);
-            if (lane == 31) xc = xs = 0.0;
-            if (b < NB) {
-                uend[2 * b] = cc + xc;
-                uend[2 * b + 1] = cs + xs;
-            }
-            cc += __shfl_sync(full, vc, 0);
-            cs += __shfl_sync(full, vs, 0);
-        }
-    }
-    __syncwarp();
-    // pass 3.  Blocks holding events ("event blocks") are formed one at a time
-    // with lane = step: each lane sums the events at its own step (their block
-    // offsets are compared four at a time as bytes), then warp scans give the
-    // collided sums up to and the uncollided sums after every step.  Blocks
-    // without events have constant sums: each lane forms 4 consecutive steps,
-    // 8 lanes a block, 4 such blocks at a time (int8 digits: 16 steps, 2 lanes
-    // a block, 16 blocks at a time).  The int8 digit layout needs the row's
-    // scale, max |beta| over its steps and columns, before any digit: a first
-    // sweep forms every value and keeps only the maximum.
-    constexpr bool kI8 = std::is_same<Real, int8_t>::value;
-    const double ci = A.cos_t[i];
-    const double vi = (i == 0 || i == A.n_cos - 1) ? 0.5 : 1.0;
-    const double rf = (0.5 * (1.0 - ci * ci) * A.dphi) * (A.dcos * vi) * A.dt * (1.0 / (6.0 * CUDART_PI));
-    const long col = (long)(slot / A.bpt) * A.tile_cols + (long)(slot % A.bpt) * 2 * A.S;
-    Real* brow = kI8 ? nullptr : beta + (((size_t)frame * A.n_cos + i) * A.cols_pad + col) * A.t_pad;
-    const double* Dslot = A.D + (size_t)slot * A.n_t * (1 + SMC);
-    const int nbase = (slot % A.bpt) * 2 * A.S;
-    int8_t* blk_row =
-        kI8 ? reinterpret_cast<int8_t*>(beta) +
-                  (((size_t)frame * A.n_cos + i) * A.tiles + slot / A.bpt) * (size_t)NB * kI8BlockSet
-            : nullptr;
-    // beta of coefficient set s at step k from the sums there: the table row
-    // holds the step weight times dt^3 and times a_m dt^{3-p_m} e^{-dt/w}
-    auto value = [&](int k, int s, const double* P, double Uc, double Us, double mul, double& xc, double& xs) {
-        const double* Dk = Dslot + (size_t)min(k, A.n_t - 1) * (1 + SMC);
-        double g[1 + SMC];
-        if constexpr ((1 + SMC) % 2 == 0) {
-#pragma unroll
-            for (int q = 0; q < 1 + SMC; q += 2) {
-                const double2 v = __ldg(reinterpret_cast<const double2*>(Dk + q));
-                g[q] = v.x;
-                g[q + 1] = v.y;
-            }
-        } else {
-#pragma unroll
-            for (int q = 0; q < 1 + SMC; ++q) g[q] = __ldg(Dk + q);
-        }
-        double vc = g[0] * Uc, vs = g[0] * Us;
-        const int t0 = s * A.M, t1 = t0 + A.M;  // the terms of set s
+        const int t0 = s * A.M, t1 = t0 + A.M;
 #pragma unroll
         for (int t = 0; t < SMC; ++t) {
-            if (t < t0 || t >= t1) continue;
-            vc += g[1 + t] * P[2 * t];
-            vs += g[1 + t] * P[2 * t + 1];
+            if (SMC > 1 && (t < t0 || t >= t1)) continue;
+            if (on) factors(1 + t, b, d);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                xc[m] = fma(d[m], w[(2 + 2 * t) * kSeg + 4 * lane + m], xc[m]);
+                xs[m] = fma(d[m], w[(3 + 2 * t) * kSeg + 4 * lane + m], xs[m]);
+            }
         }
-        const double r = k < A.n_t ? mul : 0.0;
-        xc = r * vc;
-        xs = r * vs;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            xc[m] *= rf;
+            xs[m] *= rf;
+        }
     };
-    // Collided sums through step (b << 5) + lane and uncollided sums after it, for
-    // block b, lane = step (the whole warp calls it with the same b).
-    auto step_sums = [&](int b, double (&P)[2 * SMC], double& Uc, double& Us) {
-        const int e0 = boff[b], e1 = boff[b + 1];
-        if (e0 == e1) {  // a block without events: constant sums
-#pragma unroll
-            for (int q = 0; q < 2 * SMC; ++q) P[q] = pbeg[(size_t)b * 2 * SMC + q];
-            Uc = uend[2 * b];
-            Us = uend[2 * b + 1];
-            return;
-        }
-        double dq[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) dq[q] = 0.0;
-        if (e1 - e0 > 32) {
-            // Many events: the block's events are counting-sorted by their step (stable in event
-            // order; ranks within 32 events from __match_any groups), then each lane adds the
-            // events of its own step in event order.
-            int* run = scnt + 32;
-            scnt[lane] = 0;
-            __syncwarp();
-            for (int r0 = e0; r0 < e1; r0 += 32) {
-                const int e = r0 + lane;
-                const int se = e < e1 ? (int)evs[e] : 32 + lane;
-                const unsigned m = __match_any_sync(full, se);
-                if (e < e1 && lane == __ffs(m) - 1) scnt[se] += __popc(m);
-                __syncwarp();
-            }
-            const int c = scnt[lane];
-            int incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(full, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const int ex = incl - c;  // first position of this lane's step
-            run[lane] = ex;
-            __syncwarp();
-            const unsigned lt = (1u << lane) - 1u;
-            for (int r0 = e0; r0 < e1; r0 += 32) {
-                const int e = r0 + lane;
-                const bool v = e < e1;
-                const int se = v ? (int)evs[e] : 32 + lane;
-                const unsigned m = __match_any_sync(full, se);
-                if (v) sperm[run[se] + __popc(m & lt)] = (uint16_t)e;
-                __syncwarp();
-                if (v && lane == __ffs(m) - 1) run[se] += __popc(m);
-                __syncwarp();
-            }
-            for (int r = 0; r < c; ++r) {
-                const double* qe = evq + sperm[ex + r];
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) dq[q] += qe[(size_t)q * EV];
-            }
-            __syncwarp();
-        } else {
-            const uint32_t pat = 0x01010101u * (uint32_t)lane;
-            for (int e4 = e0 & ~3; e4 < e1; e4 += 4) {
-                uint32_t eq = __vcmpeq4(*reinterpret_cast<const uint32_t*>(evs + e4), pat);
-                if (e4 < e0) eq &= 0xffffffffu << (8 * (e0 - e4));
-                if (e1 - e4 < 4) eq &= (1u << (8 * (e1 - e4))) - 1u;
-                while (eq) {
-                    const int by = (__ffs(eq) - 1) >> 3;
-                    eq &= ~(0xffu << (8 * by));
-                    const double* qe = evq + (e4 + by);
-#pragma unroll
-                    for (int q = 0; q < NQ; ++q) dq[q] += qe[(size_t)q * EV];
-                }
-            }
-        }
-        // collided sums through this step (inclusive scan), uncollided after it (suffix scan)
-        double uc = dq[0], us = dq[1];
-#pragma unroll
-        for (int q = 0; q < 2 * SMC; ++q) P[q] = dq[2 + q];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-            for (int q = 0; q < 2 * SMC; ++q) {
-                const double v = __shfl_up_sync(full, P[q], o);
-                if (lane >= o) P[q] += v;
-            }
-            const double vc = __shfl_down_sync(full, uc, o), vs = __shfl_down_sync(full, us, o);
-            if (lane + o < 32) {
-                uc += vc;
-                us += vs;
-            }
-        }
-        // uncollided after this step: the next step's inclusive suffix sum
-        Uc = __shfl_down_sync(full, uc, 1);
-        Us = __shfl_down_sync(full, us, 1);
-        if (lane == 31) Uc = Us = 0.0;
-        Uc += uend[2 * b];
-        Us += uend[2 * b + 1];
-#pragma unroll
-        for (int q = 0; q < 2 * SMC; ++q) P[q] = pbeg[(size_t)b * 2 * SMC + q] + P[q];
-    };
+    const long col = (long)(slot / A.bpt) * A.tile_cols + (long)(slot % A.bpt) * 2 * A.S;
+    const int nbase = (slot % A.bpt) * 2 * A.S;
+    double vmax = 0.0;
     if constexpr (kI8) {
-        // The row's scale is max |beta| over its steps and columns, found exactly without
-        // forming every value.
-        // (a) Every event block is formed once (lane = step) and its 2S values are kept for the
-        //     digits: a block of at least 32 events in its own weight slots (plane 2s + g, slots
-        //     boff[b] + lane; its weights are not read again), smaller blocks in the block-total
-        //     table while it has room (the rest are formed again in (c)).
-        // (b) In a block without events U and Pm are constant, so beta = rf (D0(k) U + sum_m Dm(k)
-        //     Pm) is bounded by interval arithmetic over the per-block ranges of the time table;
-        //     such blocks are formed (lane = step) in decreasing order of their bound until no
-        //     bound exceeds the largest value found (most often one block: the last one, where
-        //     dt^3 peaks).
-        // (c) Digits of every block.
-        double vmax = 0.0;
-        const double* Dmx = A.Dmax + (size_t)slot * NB * (1 + SMC) * 2;
-        int* where = brun;  // per event block: -1 not kept, -2 own slots, c >= 0 table slot c
-        const int n_tab = (NQ * NB) / (64 * A.S);
-        int used_tab = 0;
-        auto kept = [&](int b, int& stride) -> double* {
-            const int w = where[b];
-            if (w == -2) {
-                stride = EV;
-                return evq + boff[b];
+        // Digits (streaming stores: the GEMM reads them back from DRAM), lane = 4 steps of 4 blocks:
+        // the packed digits of 4 steps are transposed in registers, so that a store instruction
+        // fills whole 32-byte rows of the blocks.
+        int8_t* blk_row = reinterpret_cast<int8_t*>(beta) +
+                          (((size_t)frame * A.n_cos + i) * A.tiles + slot / A.bpt) * (size_t)NB * kI8BlockSet;
+        const int s4 = (lane & 7) * 4;
+        auto put = [&](int b, int s, uint32_t (&pc)[4], uint32_t (&ps)[4]) {
+            uint32_t wc[4], ws[4];
+            i8_transpose4(pc[0], pc[1], pc[2], pc[3], wc);
+            i8_transpose4(ps[0], ps[1], ps[2], ps[3], ws);
+            int8_t* blk = blk_row + (size_t)(b + (lane >> 3)) * kI8BlockSet;
+            const int oc = i8_swz(nbase + 2 * s, s4), os = i8_swz(nbase + 2 * s + 1, s4);
+#pragma unroll
+            for (int d = 0; d < kI8Slices; ++d) {
+                __stcs(reinterpret_cast<unsigned int*>(blk + d * kI8Block + oc), wc[d]);
+                __stcs(reinterpret_cast<unsigned int*>(blk + d * kI8Block + os), ws[d]);
             }
-            stride = 32;
-            return w >= 0 ? btot + (size_t)w * 64 * A.S : nullptr;
         };
-        for (int bc = 0; bc < NB; bc += 32) {
-            const int bl = bc + lane;
-            for (unsigned h = __ballot_sync(full, bl < NB && boff[bl] != boff[bl + 1]); h; h &= h - 1) {
-                const int b = bc + __ffs(h) - 1;
-                double P[2 * SMC], Uc, Us;
-                step_sums(b, P, Uc, Us);
-                const int k = (b << 5) + lane;
-                const int code = boff[b + 1] - boff[b] >= 32 ? -2 : (used_tab < n_tab ? used_tab++ : -1);
-                __syncwarp();
-                if (lane == 0) where[b] = code;
-                __syncwarp();
-                int stride = 0;
-                double* dst = kept(b, stride);
-                for (int s2 = 0; s2 < A.S; ++s2) {
-                    double xc, xs;
-                    value(k, s2, P, Uc, Us, rf, xc, xs);
-                    vmax = fmax(vmax, fmax(fabs(xc), fabs(xs)));
-                    if (dst) {
-                        dst[(size_t)(2 * s2) * stride + lane] = xc;
-                        dst[(size_t)(2 * s2 + 1) * stride + lane] = xs;
-                    }
-                }
-                __syncwarp();
-            }
-        }
+        // Turns 0 .. n_seg - 1 form the event segments (their values stay in the set's own bins), turn
+        // n_seg finds the scale and writes the quiet steps' digits, the others write the segments'
+        // (formed again where there are more than the warp holds).
+        double inv = 0.0;
+        for (int turn = 0; turn <= 2 * n_seg; ++turn) {
+            if (turn == n_seg) {
+                // The row's scale is max |beta| over its steps and columns, found exactly without forming
+                // every value: the event segments' are formed; a quiet block's beta = rf (D0(k) U + sum_m
+                // Dm(k) Pm) is bounded by interval arithmetic over the per-block ranges of the step
+                // factors, and such blocks are formed in decreasing order of their bound until no bound
+                // exceeds the largest value found (most often one block: the last one, where dt^3 peaks).
+                const double* Dmx = A.Dmax + (size_t)slot * NB * (1 + SMC) * 2;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(full, vmax, o));
-        for (int bc = 0; bc < NB; bc += 32) {
-            const int bl = bc + lane;
-            double bnd = -1.0;  // this lane's block's bound (-1: none or an event block)
-            if (bl < NB && boff[bl] == boff[bl + 1]) {
-                // beta of set s, column g lies in rf (D0 [U] + sum_m Dm [Pm]) with D in [min, max]
-                // over the block and U, Pm the block's constants
-                const double* mx = Dmx + (size_t)bl * (1 + SMC) * 2;
-                auto term = [&](double dlo, double dhi, double c, double& lo, double& hi, double& sa) {
-                    const double p0 = dlo * c, p1 = dhi * c;
-                    lo += fmin(p0, p1);
-                    hi += fmax(p0, p1);
-                    sa += fmax(fabs(dlo), fabs(dhi)) * fabs(c);
-                };
-                for (int s2 = 0; s2 < A.S; ++s2) {
-                    const int t0 = s2 * A.M, t1 = t0 + A.M;
+                for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(full, vmax, o));
+                for (int bc = 0; bc < NB; bc += 32) {
+                    const int bl = bc + lane;
+                    double bnd = -1.0;  // this lane's block's bound (-1: none or in a segment)
+                    if (bl < NB && (bl < b_ev || bl >= b_aft)) {
+                        const bool aft = bl >= b_aft;
+                        const double* mx = Dmx + (size_t)bl * (1 + SMC) * 2;
+                        auto term = [&](double dlo, double dhi, double c, double& lo, double& hi, double& sa) {
+                            const double p0 = dlo * c, p1 = dhi * c;
+                            lo += fmin(p0, p1);
+                            hi += fmax(p0, p1);
+                            sa += fmax(fabs(dlo), fabs(dhi)) * fabs(c);
+                        };
+                        for (int s2 = 0; s2 < A.S; ++s2) {
+                            const int t0 = s2 * A.M, t1 = t0 + A.M;
 #pragma unroll
-                    for (int g = 0; g < 2; ++g) {
-                        double lo = 0.0, hi = 0.0, sa = 0.0;
-                        term(mx[0], mx[1], uend[2 * bl + g], lo, hi, sa);
+                            for (int g = 0; g < 2; ++g) {
+                                double lo = 0.0, hi = 0.0, sa = 0.0;
+                                term(mx[0], mx[1], s_const[aft ? 2 + g : g], lo, hi, sa);
+                                if (aft) {
 #pragma unroll
-                        for (int q = 0; q < SMC; ++q)
-                            if (q >= t0 && q < t1)
-                                term(mx[2 + 2 * q], mx[3 + 2 * q], pbeg[(size_t)bl * 2 * SMC + 2 * q + g], lo, hi, sa);
-                        // relative and absolute margins cover the rounding of these sums and of
-                        // the values themselves (a few ulp of the summed magnitudes)
-                        bnd = fmax(bnd, (fmax(fabs(lo), fabs(hi)) * (1.0 + 1e-12) + 1e-13 * sa) * rf);
-                    }
-                }
-            }
-            for (;;) {
-                double bb = bnd;
-                int bi = lane;
-                for (int o = 16; o > 0; o >>= 1) {
-                    const double ob = __shfl_xor_sync(full, bb, o);
-                    const int oi = __shfl_xor_sync(full, bi, o);
-                    if (ob > bb || (ob == bb && oi < bi)) {
-                        bb = ob;
-                        bi = oi;
-                    }
-                }
-                // Every remaining bound is covered once no bound exceeds vmax (1 + 1e-10): a value up
-                // to that much above the scale still maps to |x F| <= F + 0.22, which rounds into the
-                // digit range.  (Without the slack, blocks whose values all equal the maximum, as after
-                // the last collision with powers = 3, would each be formed.)
-                if (!(bb > vmax * (1.0 + 1e-10))) break;
-                {
-                    const int b = bc + bi, k = (b << 5) + lane;
-                    const double* P = pbeg + (size_t)b * 2 * SMC;
-                    const double Uc = uend[2 * b], Us = uend[2 * b + 1];
-                    double m = 0.0;
-                    for (int s2 = 0; s2 < A.S; ++s2) {
-                        double xc, xs;
-                        value(k, s2, P, Uc, Us, rf, xc, xs);
-                        m = fmax(m, fmax(fabs(xc), fabs(xs)));
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(full, m, o));
-                    vmax = fmax(vmax, m);
-                }
-                if (lane == bi) bnd = -1.0;
-            }
-        }
-        if (lane == 0) A.scale[row] = vmax;
-        const double inv = vmax > 0.0 ? 1.0 / vmax : 0.0;
-        const double rinv = rf * inv;
-        // digits (streaming stores: the GEMM reads them back from DRAM).  Event blocks: lane = step; a
-        // quad of lanes transposes its packed digit
-        // words so that lane 4q + d holds digit d of steps 4q .. 4q + 3.  Blocks without
-        // events: 4 steps per lane (8 lanes a block, 4 blocks at a time), transposed in
-        // registers.  Either way a store instruction fills whole 32-byte rows of the blocks.
-        const bool odd = lane & 1, hi = lane & 2;
-        auto quad_transpose = [&](uint32_t p) {
-            const uint32_t t1 = __shfl_xor_sync(full, p, 1);
-            p = __byte_perm(p, t1, odd ? 0x3715 : 0x6240);
-            const uint32_t t2 = __shfl_xor_sync(full, p, 2);
-            return __byte_perm(p, t2, hi ? 0x3276 : 0x5410);
-        };
-        const int dg = lane & 3, s4 = (lane >> 2) * 4;
-        for (int bc = 0; bc < NB; bc += 32) {
-            const int bl = bc + lane;
-            const bool has = bl < NB && boff[bl] != boff[bl + 1];
-            const unsigned ev_blocks = __ballot_sync(full, has);
-            unsigned quiet = __ballot_sync(full, bl < NB && !has);
-            for (unsigned h = ev_blocks; h; h &= h - 1) {
-                const int b = bc + __ffs(h) - 1;
-                const int k = (b << 5) + lane;
-                int stride = 0;
-                const double* src = kept(b, stride);
-                double P[2 * SMC], Uc = 0.0, Us = 0.0;
-                if (!src) step_sums(b, P, Uc, Us);
-                int8_t* blk = blk_row + (size_t)b * kI8BlockSet + dg * kI8Block;
-                for (int s2 = 0; s2 < A.S; ++s2) {
-                    double xc, xs;
-                    if (src) {
-                        xc = src[(size_t)(2 * s2) * stride + lane];
-                        xs = src[(size_t)(2 * s2 + 1) * stride + lane];
-                    } else {
-                        value(k, s2, P, Uc, Us, rf, xc, xs);
-                    }
-                    const uint32_t wc = quad_transpose(i8_digits(xc * inv));
-                    const uint32_t ws = quad_transpose(i8_digits(xs * inv));
-                    __stcs(reinterpret_cast<unsigned int*>(blk + i8_swz(nbase + 2 * s2, s4)), wc);
-                    __stcs(reinterpret_cast<unsigned int*>(blk + i8_swz(nbase + 2 * s2 + 1, s4)), ws);
-                }
-            }
-            const int sub = lane >> 3, s0 = (lane & 7) * 4;
-            while (quiet) {
-                unsigned t = quiet;
-                for (int g = 0; g < sub && t; ++g) t &= t - 1;
-                const int b = t ? bc + __ffs(t) - 1 : -1;
-                for (int g = 0; g < 4 && quiet; ++g) quiet &= quiet - 1;
-                if (b < 0) continue;
-                const int k0 = (b << 5) + s0;
-                // the block's constant sums, with rf / scale folded in: 1 + SMC products per
-                // value (steps past n_t, in the last block only, go through value())
-                const bool tail = k0 + 4 > A.n_t;
-                double P[2 * SMC];
-#pragma unroll
-                for (int q = 0; q < 2 * SMC; ++q) P[q] = rinv * pbeg[(size_t)b * 2 * SMC + q];
-                const double Uc = rinv * uend[2 * b], Us = rinv * uend[2 * b + 1];
-                const double* Db = Dslot + (size_t)k0 * (1 + SMC);
-                int8_t* blk = blk_row + (size_t)b * kI8BlockSet;
-                for (int s2 = 0; s2 < A.S; ++s2) {
-                    uint32_t pc[4], ps[4];
-                    const int t0 = s2 * A.M, t1 = t0 + A.M;  // the terms of set s2
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        double xc, xs;
-                        if (tail) {
-                            value(k0 + m, s2, P, Uc, Us, 1.0, xc, xs);
-                        } else {
-                            const double* Dk = Db + (size_t)m * (1 + SMC);
-                            double g[1 + SMC];
-                            if constexpr ((1 + SMC) % 2 == 0) {
-#pragma unroll
-                                for (int q = 0; q < 1 + SMC; q += 2) {
-                                    const double2 v = __ldg(reinterpret_cast<const double2*>(Dk + q));
-                                    g[q] = v.x;
-                                    g[q + 1] = v.y;
+                                    for (int q = 0; q < SMC; ++q)
+                                        if (SMC == 1 || (q >= t0 && q < t1))
+                                            term(mx[2 + 2 * q], mx[3 + 2 * q], s_const[4 + 2 * q + g], lo, hi, sa);
                                 }
-                            } else {
-#pragma unroll
-                                for (int q = 0; q < 1 + SMC; ++q) g[q] = __ldg(Dk + q);
-                            }
-                            xc = g[0] * Uc;
-                            xs = g[0] * Us;
-#pragma unroll
-                            for (int q = 0; q < SMC; ++q) {
-                                if (SMC > 1 && (q < t0 || q >= t1)) continue;
-                                xc = fma(g[1 + q], P[2 * q], xc);
-                                xs = fma(g[1 + q], P[2 * q + 1], xs);
+                                // relative and absolute margins cover the rounding of these sums and of
+                                // the values themselves (a few ulp of the summed magnitudes)
+                                bnd = fmax(bnd, (fmax(fabs(lo), fabs(hi)) * (1.0 + 1e-12) + 1e-13 * sa) * rf);
                             }
                         }
-                        pc[m] = i8_digits(xc);
-                        ps[m] = i8_digits(xs);
                     }
-                    uint32_t wc[4], ws[4];
-                    i8_transpose4(pc[0], pc[1], pc[2], pc[3], wc);
-                    i8_transpose4(ps[0], ps[1], ps[2], ps[3], ws);
-                    const int oc = i8_swz(nbase + 2 * s2, s0), os = i8_swz(nbase + 2 * s2 + 1, s0);
+                    for (;;) {
+                        double bb = bnd;
+                        int bi = lane;
+                        for (int o = 16; o > 0; o >>= 1) {
+                            const double ob = __shfl_xor_sync(full, bb, o);
+                            const int oi = __shfl_xor_sync(full, bi, o);
+                            if (ob > bb || (ob == bb && oi < bi)) {
+                                bb = ob;
+                                bi = oi;
+                            }
+                        }
+                        // Every remaining bound is covered once no bound exceeds vmax (1 + 1e-10): a value up
+                        // to that much above the scale still maps to |x F| <= F + 0.22, which rounds into the
+                        // digit range.  (Without the slack, blocks whose values all equal the maximum, as after
+                        // the last collision with powers = 3, would each be formed.)
+                        if (!(bb > vmax * (1.0 + 1e-10))) break;
+                        {
+                            const int b = bc + bi;
+                            const bool aft = b >= b_aft;
+                            const double* d = Dslot + (b << 5) + lane;
+                            const double d0 = d[0];
+                            double m = 0.0;
+                            for (int s2 = 0; s2 < A.S; ++s2) {
+                                const int t0 = s2 * A.M, t1 = t0 + A.M;
+                                double xc = d0 * s_const[aft ? 2 : 0], xs = d0 * s_const[aft ? 3 : 1];
 #pragma unroll
-                    for (int d = 0; d < kI8Slices; ++d) {
-                        __stcs(reinterpret_cast<unsigned int*>(blk + d * kI8Block + oc), wc[d]);
-                        __stcs(reinterpret_cast<unsigned int*>(blk + d * kI8Block + os), ws[d]);
+                                for (int q = 0; q < SMC; ++q) {
+                                    if (!aft || (SMC > 1 && (q < t0 || q >= t1))) continue;
+                                    const double dq = d[(size_t)(1 + q) * A.tf];
+                                    xc = fma(dq, s_const[4 + 2 * q], xc);
+                                    xs = fma(dq, s_const[5 + 2 * q], xs);
+                                }
+                                m = fmax(m, fmax(fabs(xc), fabs(xs)));
+                            }
+                            m *= rf;
+#pragma unroll
+                            for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(full, m, o));
+                            vmax = fmax(vmax, m);
+                        }
+                        if (lane == bi) bnd = -1.0;
                     }
                 }
+                if (lane == 0) A.scale[row] = vmax;
+                inv = vmax > 0.0 ? 1.0 / vmax : 0.0;
+                // quiet steps: the constants with the scale (and F) folded in
+                const double rinv = rf * inv;
+                auto quiet = [&](int b_lo, int b_hi, bool aft) {
+                    const double* U = s_const + (aft ? 2 : 0);
+                    const double Uc = rinv * U[0], Us = rinv * U[1];
+                    const bool none = U[0] == 0.0 && U[1] == 0.0;  // every patch has collided
+                    double P[2 * SMC];
+#pragma unroll
+                    for (int q = 0; q < 2 * SMC; ++q) P[q] = rinv * s_const[4 + q];
+                    for (int b = b_lo; b < b_hi; b += kSegBlocks) {
+                        if (b + (lane >> 3) >= b_hi) continue;
+                        for (int s = 0; s < A.S; ++s) {
+                            const int t0 = s * A.M, t1 = t0 + A.M;
+                            double xc[4] = {0.0, 0.0, 0.0, 0.0}, xs[4] = {0.0, 0.0, 0.0, 0.0}, d[4];
+                            if (!none) {
+                                factors(0, b, d);
+#pragma unroll
+                                for (int m = 0; m < 4; ++m) {
+                                    xc[m] = d[m] * Uc;
+                                    xs[m] = d[m] * Us;
+                                }
+                            }
+                            if (aft) {
+#pragma unroll
+                                for (int t = 0; t < SMC; ++t) {
+                                    if (SMC > 1 && (t < t0 || t >= t1)) continue;
+                                    factors(1 + t, b, d);
+#pragma unroll
+                                    for (int m = 0; m < 4; ++m) {
+                                        xc[m] = fma(d[m], P[2 * t], xc[m]);
+                                        xs[m] = fma(d[m], P[2 * t + 1], xs[m]);
+                                    }
+                                }
+                            }
+                            uint32_t pc[4], ps[4];
+#pragma unroll
+                            for (int m = 0; m < 4; ++m) {
+                                pc[m] = i8_digits(xc[m]);
+                                ps[m] = i8_digits(xs[m]);
+                            }
+                            put(b, s, pc, ps);
+                        }
+                    }
+                };
+                quiet(0, min(b_ev, NB), false);
+                quiet(b_aft, NB, true);
+                continue;
             }
+            const int g = turn < n_seg ? turn : 2 * n_seg - turn;  // then from the last: it is still held
+            double* w = bins + (size_t)(g % A.keep) * NQ * kSeg;
+            const bool kept = turn > n_seg && g >= n_seg - A.keep;  // its values are still in its bins
+            if (!kept) form(g, w);
+            for (int s = 0; s < A.S; ++s) {
+                double xc[4], xs[4];
+                double2* e = reinterpret_cast<double2*>(w + (2 + 2 * s * A.M) * kSeg + 4 * lane);
+                double2* f = e + kSeg / 2;
+                if (kept) {
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        xc[2 * m] = e[m].x;
+                        xc[2 * m + 1] = e[m].y;
+                        xs[2 * m] = f[m].x;
+                        xs[2 * m + 1] = f[m].y;
+                    }
+                } else {
+                    seg_values(g, w, s, xc, xs);
+                }
+                if (turn < n_seg) {
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) vmax = fmax(vmax, fmax(fabs(xc[m]), fabs(xs[m])));
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        e[m] = make_double2(xc[2 * m], xc[2 * m + 1]);
+                        f[m] = make_double2(xs[2 * m], xs[2 * m + 1]);
+                    }
+                } else {
+                    uint32_t pc[4], ps[4];
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        pc[m] = i8_digits(xc[m] * inv);
+                        ps[m] = i8_digits(xs[m] * inv);
+                    }
+                    const int b = b_ev + g * kSegBlocks;
+                    if (b + (lane >> 3) < NB) put(b, s, pc, ps);
+                }
+            }
+            __syncwarp();
         }
     } else {
-        for (int bc = 0; bc < NB; bc += 32) {
-            const int bl = bc + lane;
-            const bool has = bl < NB && boff[bl] != boff[bl + 1];
-            const unsigned ev_blocks = __ballot_sync(full, has);
-            unsigned quiet = __ballot_sync(full, bl < NB && !has);
-            // ---- event blocks, lane = step
-            for (unsigned h = ev_blocks; h; h &= h - 1) {
-                const int b = bc + __ffs(h) - 1;
-                double P[2 * SMC], Uc, Us;
-                step_sums(b, P, Uc, Us);
-                const int k = (b << 5) + lane;
-                for (int s2 = 0; s2 < A.S; ++s2) {
-                    double xc, xs;
-                    value(k, s2, P, Uc, Us, rf, xc, xs);
-                    if (k < A.t_pad) {
-                        brow[(size_t)(2 * s2) * A.t_pad + k] = (Real)xc;
-                        brow[(size_t)(2 * s2 + 1) * A.t_pad + k] = (Real)xs;
-                    }
-                }
-            }
-            // ---- blocks without events, 4 steps per lane
-            const int sub = lane >> 3, s0 = (lane & 7) * 4;
-            while (quiet) {
-                unsigned t = quiet;
-                for (int g = 0; g < sub && t; ++g) t &= t - 1;
-                const int b = t ? bc + __ffs(t) - 1 : -1;
-                for (int g = 0; g < 4 && quiet; ++g) quiet &= quiet - 1;
-                if (b < 0) continue;
-                const double* P = pbeg + (size_t)b * 2 * SMC;
-                const double Uc = uend[2 * b], Us = uend[2 * b + 1];
-                const int k0 = (b << 5) + s0;
-                for (int s2 = 0; s2 < A.S; ++s2) {
-                    double xc[4], xs[4];
+        for (int g = 0; g < n_seg; ++g) {
+            form(g, bins);
+            for (int s = 0; s < A.S; ++s) {
+                double xc[4], xs[4];
+                seg_values(g, bins, s, xc, xs);
+                Real* o = beta + (((size_t)frame * A.n_cos + i) * A.cols_pad + col + 2 * s) * A.t_pad;
+                const int k = ((b_ev + g * kSegBlocks) << 5) + 4 * lane;
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) value(k0 + m, s2, P, Uc, Us, rf, xc[m], xs[m]);
+                for (int m = 0; m < 4; ++m)
+                    if (k + m < A.t_pad) {
+                        o[k + m] = (Real)xc[m];
+                        o[A.t_pad + k + m] = (Real)xs[m];
+                    }
+            }
+            __syncwarp();
+        }
+        auto quiet = [&](int b_lo, int b_hi, bool aft) {
+            const double* U = s_const + (aft ? 2 : 0);
+            for (int b = b_lo; b < b_hi; b += kSegBlocks) {
+                if (b + (lane >> 3) >= b_hi) continue;
+                for (int s = 0; s < A.S; ++s) {
+                    const int t0 = s * A.M, t1 = t0 + A.M;
+                    double xc[4], xs[4], d[4];
+                    factors(0, b, d);
 #pragma unroll
                     for (int m = 0; m < 4; ++m) {
-                        const int k = k0 + m;
-                        if (k < A.t_pad) {
-                            brow[(size_t)(2 * s2) * A.t_pad + k] = (Real)xc[m];
-                            brow[(size_t)(2 * s2 + 1) * A.t_pad + k] = (Real)xs[m];
+                        xc[m] = d[m] * U[0];
+                        xs[m] = d[m] * U[1];
+                    }
+                    if (aft) {
+#pragma unroll
+                        for (int t = 0; t < SMC; ++t) {
+                            if (SMC > 1 && (t < t0 || t >= t1)) continue;
+                            factors(1 + t, b, d);
+#pragma unroll
+                            for (int m = 0; m < 4; ++m) {
+                                xc[m] = fma(d[m], s_const[4 + 2 * t], xc[m]);
+                                xs[m] = fma(d[m], s_const[5 + 2 * t], xs[m]);
+                            }
                         }
                     }
+                    Real* o = beta + (((size_t)frame * A.n_cos + i) * A.cols_pad + col + 2 * s) * A.t_pad;
+                    const int k = (b << 5) + 4 * lane;
+#pragma unroll
+                    for (int m = 0; m < 4; ++m)
+                        if (k + m < A.t_pad) {
+                            o[k + m] = (Real)(rf * xc[m]);
+                            o[A.t_pad + k + m] = (Real)(rf * xs[m]);
+                        }
                 }
             }
-        }
+        };
+        quiet(0, min(b_ev, NB), false);
+        quiet(b_aft, NB, true);
     }
 }
 
@@ -1172,12 +1023,13 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
     const FactGeom G = fact_geom(job, sizeof(Real));
     uint64_t launches = 0;
     // per-bubble time tables (frame independent)
-    dev->fact_D.ensure((size_t)n_sel * n_t * (1 + SM) * sizeof(double));
+    const int tf = G.nblk * 32;
+    dev->fact_D.ensure((size_t)n_sel * tf * (1 + SM) * sizeof(double));
     dev->fact_kfirst.ensure((size_t)n_sel * sizeof(int));
     if ((n_t + 127) / 128 > 65535) throw Error{"too many time steps for the time-table grid"};
     {
-        dim3 g((unsigned)n_sel, (unsigned)((n_t + 127) / 128));
-        k_time_tables<<<g, 128, 0, dev->stream>>>(bub_frames, sel, n_sel, t_arr, n_t, powers, coeffs, cutw, SM,
+        dim3 g((unsigned)n_sel, (unsigned)((tf + 127) / 128));
+        k_time_tables<<<g, 128, 0, dev->stream>>>(bub_frames, sel, n_sel, t_arr, n_t, tf, powers, coeffs, cutw, SM,
                                                   job.has_damping ? 1 : 0, job.damping, (double*)dev->fact_D.p,
                                                   (int*)dev->fact_kfirst.p);
         CUDA_OK(cudaGetLastError());
@@ -1193,7 +1045,7 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
         dev->beta_scale.ensure((size_t)kn * n_sel * n_cos * sizeof(double));
         dev->fact_Dmax.ensure((size_t)n_sel * nkb * (1 + SM) * 2 * sizeof(double));
         const long warps = (long)n_sel * nkb;
-        k_time_maxima<<<(unsigned)((warps + 7) / 8), 256, 0, dev->stream>>>((const double*)dev->fact_D.p, n_sel, n_t,
+        k_time_maxima<<<(unsigned)((warps + 7) / 8), 256, 0, dev->stream>>>((const double*)dev->fact_D.p, n_sel, tf,
                                                                             nkb, 1 + SM, (double*)dev->fact_Dmax.p);
         CUDA_OK(cudaGetLastError());
         ++launches;
@@ -1222,6 +1074,7 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
         B.powers = powers;
         B.coeffs = coeffs;
         B.D = (const double*)dev->fact_D.p;
+        B.tf = tf;
         B.has_damp = job.has_damping ? 1 : 0;
         B.damp = job.damping;
         B.dphi = 2.0 * M_PI / (double)n_phi;
@@ -1233,18 +1086,20 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
         B.tile_cols = G.tile_cols;
         B.bpt = G.bpt;
         B.t_pad = G.t_pad;
-        const int NQ = 2 + 2 * SM;
-        size_t pw = (size_t)n_phi * NQ * sizeof(double) + 2 * (size_t)NQ * G.nblk * sizeof(double) +
-                    (2 * (size_t)G.nblk + 1) * sizeof(int) + (((size_t)n_phi + 4 + 3) & ~(size_t)3) +
-                    64 * sizeof(int) + (size_t)n_phi * sizeof(uint16_t);
-        pw = (pw + 15) & ~(size_t)15;
-        B.per_warp_bytes = (int)pw;
+        // shared memory of a warp: a segment's bins (a second segment's too while three blocks of 8 warps
+        // still fit an SM), the quiet constants, the row's delays and steps; of the block: the weights
+        const size_t pitch = (((size_t)n_phi + 31) / 32) | 1;
+        const size_t bins = (size_t)(2 + 2 * SM) * kSeg, others = 4 + 2 * (size_t)SM + 32 * pitch + 16 * pitch;
+        B.keep = tc && 3 * (64 * pitch + 8 * (2 * bins + others)) * sizeof(double) <= 220 * 1024 ? 2 : 1;
+        const size_t per_warp = (B.keep * bins + others + 1) & ~(size_t)1;
+        B.per_warp = (int)per_warp;
         B.tiles = G.tiles_per_frame;
         B.scale = tc ? (double*)dev->beta_scale.p : nullptr;
         B.Dmax = tc ? (const double*)dev->fact_Dmax.p : nullptr;
-        int warps = (int)std::min<size_t>(8, (200 * 1024) / pw);
-        if (warps < 1) throw Error{"n_phi too large for the beta kernel"};
-        const size_t smem = (size_t)warps * pw;
+        const size_t room = 220 * 1024 / sizeof(double);
+        if (64 * pitch + per_warp > room) throw Error{"n_phi too large for the beta kernel"};
+        const int warps = (int)std::min<size_t>(8, (room - 64 * pitch) / per_warp);
+        const size_t smem = (64 * pitch + warps * per_warp) * sizeof(double);
         const unsigned blocks = (unsigned)((B.n_rows + warps - 1) / warps);
         launch_beta<Real>(SM, B, (Real*)dev->beta.p, smem, blocks, warps * 32, dev->stream);
         CUDA_OK(cudaGetLastError());
