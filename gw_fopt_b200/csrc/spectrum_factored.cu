@@ -152,6 +152,7 @@ struct BetaArgs {
     int t_pad;             // row length of beta
     int keep;              // event segments whose bins a warp holds at once
     int per_warp;          // doubles of shared memory per warp
+    int per_warp_bytes;    // the same of k_beta_sorted, in bytes
     int tiles;             // column tiles per frame (int8 digit layout)
     double* scale;         // int8 digit layout: (kn, n_sel, n_cos) row scales, max |beta| of the row
     const double* Dmax;    // int8 digit layout: (n_sel, nblk, 1+S*M, 2) least and largest D over each block's steps
@@ -160,37 +161,45 @@ struct BetaArgs {
 constexpr int kSegBlocks = 4;              // blocks of 32 steps in an event segment
 constexpr int kSeg = 32 * kSegBlocks;
 
-// blocks per SM: three at 80 registers with one term, two with two
+__device__ __forceinline__ void copy8_async(double* smem, const double* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+
+// warps of a block, and blocks per SM: 24 warps at 80 registers with one term, 16 at 128 with two
+__host__ __device__ constexpr int beta_warps(int SMC) { return SMC == 1 ? 8 : 4; }
+__host__ __device__ constexpr int beta_blocks(int SMC) { return SMC == 1 ? 3 : SMC == 2 ? 4 : SMC <= 4 ? 3 : 2; }
+// With two terms and more a warp takes every so-manieth row and fetches the next one's delays while it
+// works (16 or 8 warps do not hide them: 564 against 760 us for 6 frames of 101 bubbles, 4 terms); with one
+// term the loop's registers spill (67 against 47 ms for 8 frames of 4096 bubbles).
+__host__ __device__ constexpr int beta_rows_held(int SMC) { return SMC == 1 ? 1 : 2; }
 template <class Real, int SMC>
-__global__ void __launch_bounds__(256, SMC == 1 ? 3 : SMC == 2 ? 2 : 1) k_beta(BetaArgs A, Real* __restrict__ beta) {
-    extern __shared__ __align__(16) double sm_b[];
-    constexpr bool kI8 = std::is_same<Real, int8_t>::value;
+__global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta(BetaArgs A, Real* __restrict__ beta) {
+    extern __shared__ __align__(16) double sm_beta[];
+    constexpr bool kI8 = std::is_same<Real, int8_t>::value, kLoop = SMC > 1;
     constexpr int NQ = 2 + 2 * SMC;  // weights of an event: cos, sin; then cos and sin times each term's factor
     constexpr unsigned full = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long row = (long)blockIdx.x * (blockDim.x >> 5) + warp;
     const int NB = A.nblk;
     // Lane l holds the patches [c l, c l + c): neighbouring patches collide at the same or the next step,
     // so most of a step's events are added up in registers before they reach its bin.  Their rows in shared
     // memory have an odd pitch (no bank conflicts).
     const int c_pat = (A.n_phi + 31) >> 5, pitch = c_pat | 1;
-    double2* s_wgt = reinterpret_cast<double2*>(sm_b);                       // [32 pitch] weights, block's own
-    double* base_w = sm_b + 64 * pitch + (size_t)warp * A.per_warp;
+    double2* s_wgt = reinterpret_cast<double2*>(sm_beta);                       // [32 pitch] weights, block's own
+    double* base_w = sm_beta + 64 * pitch + (size_t)warp * A.per_warp;
     double* bins = base_w;                                                   // [keep][NQ][kSeg]
     double* s_const = bins + (size_t)A.keep * NQ * kSeg;                     // [4 + 2 SMC] quiet constants
-    double* s_tau = s_const + 4 + 2 * SMC;                                   // [32 pitch] delays
-    int* s_kj = reinterpret_cast<int*>(s_tau + 32 * pitch);                  // [32 pitch] first collided steps
+    double* s_tau = s_const + 4 + 2 * SMC;                                   // [rows held][32 pitch] delays
+    int* s_kj = reinterpret_cast<int*>(s_tau + beta_rows_held(SMC) * 32 * pitch);  // [32 pitch] first collided steps
     for (int j = threadIdx.x; j < A.n_phi; j += blockDim.x) {
         const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
         s_wgt[j / c_pat * pitch + j % c_pat] = make_double2(wj * A.cos2[j], wj * A.sin2[j]);
     }
-    __syncthreads();
-    if (row >= A.n_rows) return;
+    auto beta_row = [&](long row, const double* s_tau) {
     const int slot = (int)((row / A.n_cos) % A.n_sel);
     if (A.sel[slot] == kNoSlot) return;  // a padding slot of a batched job: its columns are never read
     const int i = (int)(row % A.n_cos);
     const long frame = row / ((long)A.n_cos * A.n_sel);
-    const double* trow = A.tau + (size_t)row * A.n_phi;
     const double ta = A.bub[A.sel[slot]].t;
     const double inv_dt = 1.0 / A.dt;  // the estimate below is only a starting point
     constexpr int kNever = 0x7fffffff;
@@ -205,18 +214,14 @@ __global__ void __launch_bounds__(256, SMC == 1 ? 3 : SMC == 2 ? 2 : 1) k_beta(B
         return lo < A.n_t ? lo : kNever;
     };
     int k_lo = kNever, k_hi = -1;
-#pragma unroll 2
-    for (int j = lane; j < A.n_phi; j += 32) {
-        const double tj = __ldcs(trow + j);
-        const int kj = step_of(tj), at = j / c_pat * pitch + j % c_pat;
-        s_tau[at] = tj;
-        s_kj[at] = kj;
+    const int n_own = max(0, min(c_pat, A.n_phi - lane * c_pat));  // this lane's patches
+    const int own = lane * pitch;
+    for (int m = 0; m < n_own; ++m) {
+        const int kj = step_of(s_tau[own + m]);
+        s_kj[own + m] = kj;
         k_lo = min(k_lo, kj);
         if (kj != kNever) k_hi = max(k_hi, kj);
     }
-    __syncwarp();
-    const int n_own = max(0, min(c_pat, A.n_phi - lane * c_pat));  // this lane's patches
-    const int own = lane * pitch;
     k_lo = __reduce_min_sync(full, k_lo);
     k_hi = __reduce_max_sync(full, k_hi);
     // event segments: blocks [b_ev, b_ev + 4 n_seg); without events none, and every block is "before"
@@ -634,32 +639,668 @@ __global__ void __launch_bounds__(256, SMC == 1 ? 3 : SMC == 2 ? 2 : 1) k_beta(B
         quiet(0, min(b_ev, NB), false);
         quiet(b_aft, NB, true);
     }
+    };
+    auto fetch = [&](long r, double* dst) {  // a row's delays, all in flight at once
+        if (r < A.n_rows) {
+            const double* src = A.tau + (size_t)r * A.n_phi;
+            for (int j = lane; j < A.n_phi; j += 32) copy8_async(dst + j / c_pat * pitch + j % c_pat, src + j);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const long row0 = (long)blockIdx.x * (blockDim.x >> 5) + warp;
+    const long n_warps = (long)gridDim.x * (blockDim.x >> 5);
+    fetch(row0, s_tau);
+    double* s_next = s_tau + (kLoop ? 32 * pitch : 0);
+    __syncthreads();
+    for (long row = row0; row < A.n_rows; row += n_warps) {
+    if constexpr (kLoop) {
+        fetch(row + n_warps, s_next);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    __syncwarp();
+    beta_row(row, s_tau);
+    if constexpr (!kLoop) break;
+    double* t = s_tau;
+    s_tau = s_next;
+    s_next = t;
+    __syncwarp();
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 template <class Real, int SMC>
-static void launch_beta_smc(const BetaArgs& B, Real* out, size_t smem, unsigned blocks, int threads,
-                            cudaStream_t st) {
+static void launch_beta_smc(const BetaArgs& B, Real* out, size_t smem, int n_sm, int warps, cudaStream_t st) {
     CUDA_OK(cudaFuncSetAttribute(k_beta<Real, SMC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // three blocks per SM need the largest shared-memory carveout; without the preference the
     // driver may pick a smaller one (two blocks per SM) depending on the kernels run before
     CUDA_OK(cudaFuncSetAttribute(k_beta<Real, SMC>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  (int)cudaSharedmemCarveoutMaxShared));
-    k_beta<Real, SMC><<<blocks, threads, smem, st>>>(B, out);
+    const long blocks = (B.n_rows + warps - 1) / warps;
+    if (blocks > 0x7fffffffL) throw Error{"too many (bubble, row) pairs for one launch"};
+    int per_sm = 1;
+    if (SMC > 1) CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_beta<Real, SMC>, 32 * warps, smem));
+    const long grid = SMC > 1 ? std::min(blocks, (long)n_sm * std::max(1, per_sm)) : blocks;
+    k_beta<Real, SMC><<<(unsigned)grid, 32 * warps, smem, st>>>(B, out);
 }
 
 template <class Real>
-static void launch_beta(int SM, const BetaArgs& B, Real* out, size_t smem, unsigned blocks, int threads,
+static void launch_beta(int SM, const BetaArgs& B, Real* out, size_t smem, int n_sm, int warps,
                         cudaStream_t st) {
     switch (SM) {
-        case 1: launch_beta_smc<Real, 1>(B, out, smem, blocks, threads, st); break;
-        case 2: launch_beta_smc<Real, 2>(B, out, smem, blocks, threads, st); break;
-        case 3: launch_beta_smc<Real, 3>(B, out, smem, blocks, threads, st); break;
-        case 4: launch_beta_smc<Real, 4>(B, out, smem, blocks, threads, st); break;
-        case 5: launch_beta_smc<Real, 5>(B, out, smem, blocks, threads, st); break;
-        case 6: launch_beta_smc<Real, 6>(B, out, smem, blocks, threads, st); break;
-        case 7: launch_beta_smc<Real, 7>(B, out, smem, blocks, threads, st); break;
-        case 8: launch_beta_smc<Real, 8>(B, out, smem, blocks, threads, st); break;
+        case 1: launch_beta_smc<Real, 1>(B, out, smem, n_sm, warps, st); break;
+        case 2: launch_beta_smc<Real, 2>(B, out, smem, n_sm, warps, st); break;
+        case 3: launch_beta_smc<Real, 3>(B, out, smem, n_sm, warps, st); break;
+        case 4: launch_beta_smc<Real, 4>(B, out, smem, n_sm, warps, st); break;
+        case 5: launch_beta_smc<Real, 5>(B, out, smem, n_sm, warps, st); break;
+        case 6: launch_beta_smc<Real, 6>(B, out, smem, n_sm, warps, st); break;
+        case 7: launch_beta_smc<Real, 7>(B, out, smem, n_sm, warps, st); break;
+        case 8: launch_beta_smc<Real, 8>(B, out, smem, n_sm, warps, st); break;
         default: throw Error{"at most 8 (set, term) pairs in the factored kernels"};
+    }
+}
+
+// The int8 digits of a forward call whose masks are kept for the adjoint, with every sum in the order in
+// which the events are sorted: by block of 32 steps, then by step, then by patch.  The mixed adjoint's FP32
+// products turn a change of the spectrum in its last bits into one of 1e-8 in the gradients (measured with
+// k_beta's order: 1.8e-8 on 256 bubbles, 32 k-hat), so its forward keeps this order although k_beta takes
+// 3.5 ms where this kernel takes 4.4.
+template <int SMC>
+__global__ void __launch_bounds__(256, 3) k_beta_sorted(BetaArgs A, int8_t* __restrict__ beta) {
+    extern __shared__ __align__(16) unsigned char sm_b[];
+    constexpr int NQ = 2 + 2 * SMC;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long row = (long)blockIdx.x * (blockDim.x >> 5) + warp;
+    if (row >= A.n_rows) return;
+    const int NB = A.nblk;
+    const int EV = A.n_phi;  // event capacity: one event per patch at most
+    unsigned char* base = sm_b + (size_t)warp * A.per_warp_bytes;
+    double* evq = reinterpret_cast<double*>(base);             // [NQ][n_phi]: weight q of event e at q * n_phi + e
+    double* btot = evq + (size_t)A.n_phi * NQ;                  // [NQ][NB] block totals
+    double* uend = btot + (size_t)NQ * NB;                      // [NB][2] uncollided after block
+    double* pbeg = uend + 2 * NB;                               // [NB][2 SMC] collided before block
+    int* boff = reinterpret_cast<int*>(pbeg + (size_t)2 * SMC * NB);  // [NB+1]
+    int* brun = boff + NB + 1;                                  // [NB]
+    uint8_t* evs = reinterpret_cast<uint8_t*>(brun + NB);       // [n_phi + 4] step of each event within its block
+    // a crowded event block's per-step counts and running offsets [2][32], and its events in step order [n_phi]
+    int* scnt = reinterpret_cast<int*>(evs + ((A.n_phi + 4 + 3) & ~3));
+    uint16_t* sperm = reinterpret_cast<uint16_t*>(scnt + 64);
+    const int slot = (int)((row / A.n_cos) % A.n_sel);
+    if (A.sel[slot] == kNoSlot) return;  // a padding slot of a batched job: its columns are never read
+    const int i = (int)(row % A.n_cos);
+    const long frame = row / ((long)A.n_cos * A.n_sel);
+    const double* trow = A.tau + (size_t)row * A.n_phi;
+    // The delays of patches j = lane + 32 jj, jj < kMaxJ, are loaded first, all at once (one
+    // memory latency for the row), and kept for both passes over the patches.
+    constexpr int kMaxJ = 6;
+    double tj_c[kMaxJ];
+#pragma unroll
+    for (int jj = 0; jj < kMaxJ; ++jj) {
+        const int j = 32 * jj + lane;
+        tj_c[jj] = j < A.n_phi ? __ldcs(trow + j) : 0.0;
+    }
+    const double ta = A.bub[A.sel[slot]].t;
+    const unsigned full = 0xffffffffu;
+    const double inv_dt = 1.0 / A.dt;  // the estimate below is only a starting point
+    auto block_of = [&](int j, double tj, int& kj) -> int {
+        kj = A.n_t;
+        if (j >= A.n_phi) return -2;  // not a patch
+        if (!(tj > 0.0)) return -1;    // never collides
+        // first k with (t_k - t_a) >= tau_j: arithmetic estimate, then exact
+        // comparisons (the predicate is monotone in k) settle the boundary
+        const double est = ceil((ta + tj - A.t_arr[0]) * inv_dt);
+        int lo = est < 0.0 ? 0 : (est > (double)A.n_t ? A.n_t : (int)est);
+        while (lo > 0 && A.t_arr[lo - 1] - ta >= tj) --lo;
+        while (lo < A.n_t && !(A.t_arr[lo] - ta >= tj)) ++lo;
+        kj = lo;
+        return lo < A.n_t ? lo >> 5 : -1;
+    };
+    for (int b = lane; b < NB; b += 32) boff[b] = 0;
+    __syncwarp();
+    // pass 1: events per block; never-colliding weights (lane sums, fixed-order reduction).
+    // The first collided step of patches j = lane + 32 jj, jj < kMaxJ, is kept for pass 2.
+    int kj_c[kMaxJ], b_c[kMaxJ];
+    double nc = 0.0, ns = 0.0;
+    auto pass1 = [&](int j, int b) {
+        if (b == -1) {
+            const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
+            nc += wj * A.cos2[j];
+            ns += wj * A.sin2[j];
+        }
+        const unsigned m = __match_any_sync(full, b);
+        if (b >= 0 && lane == __ffs(m) - 1) boff[b] += __popc(m);
+        __syncwarp();
+    };
+#pragma unroll
+    for (int jj = 0; jj < kMaxJ; ++jj) {
+        if (32 * jj >= A.n_phi) break;
+        const int j = 32 * jj + lane;
+        kj_c[jj] = 0;
+        b_c[jj] = block_of(j, tj_c[jj], kj_c[jj]);
+        pass1(j, b_c[jj]);
+    }
+    for (int j0 = 32 * kMaxJ; j0 < A.n_phi; j0 += 32) {
+        int kj;
+        const int j = j0 + lane;
+        const int b = block_of(j, j < A.n_phi ? trow[j] : 0.0, kj);
+        pass1(j, b);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        nc += __shfl_down_sync(full, nc, o);
+        ns += __shfl_down_sync(full, ns, o);
+    }
+    // block counts -> first event of each block: an exclusive warp scan over 32 blocks at a time
+    {
+        int carry = 0;
+        for (int bc = 0; bc < NB; bc += 32) {
+            const int b = bc + lane;
+            const int c = b < NB ? boff[b] : 0;
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(full, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (b < NB) {
+                boff[b] = carry + incl - c;
+                brun[b] = carry + incl - c;
+            }
+            carry += __shfl_sync(full, incl, 31);
+        }
+        __syncwarp();
+        if (lane == 0) boff[NB] = carry;
+    }
+    __syncwarp();
+    // pass 2: scatter events (stable in j within a block)
+    const unsigned lt = (1u << lane) - 1u;
+    auto pass2 = [&](int j, double tj, int kj, int b) {
+        const unsigned m = __match_any_sync(full, b);
+        int pos = 0;
+        if (b >= 0) pos = brun[b] + __popc(m & lt);
+        __syncwarp();
+        if (b >= 0 && lane == __ffs(m) - 1) brun[b] += __popc(m);
+        __syncwarp();
+        if (b >= 0) {
+            evs[pos] = (uint8_t)(kj & 31);
+            const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
+            const double qc = wj * A.cos2[j], qs = wj * A.sin2[j];
+            double* q = evq + pos;
+            q[0] = qc;
+            q[EV] = qs;
+            const double ed = A.has_damp ? exp(tj / A.damp) : 1.0;
+#pragma unroll
+            for (int t = 0; t < SMC; ++t) {
+                const double f = tpow(tj, A.powers[t]) * ed;
+                q[(2 + 2 * t) * EV] = qc * f;
+                q[(3 + 2 * t) * EV] = qs * f;
+            }
+        }
+    };
+#pragma unroll
+    for (int jj = 0; jj < kMaxJ; ++jj) {
+        if (32 * jj >= A.n_phi) break;
+        pass2(32 * jj + lane, tj_c[jj], kj_c[jj], b_c[jj]);
+    }
+    for (int j0 = 32 * kMaxJ; j0 < A.n_phi; j0 += 32) {
+        int kj;
+        const int j = j0 + lane;
+        const double tj = j < A.n_phi ? trow[j] : 0.0;
+        const int b = block_of(j, tj, kj);
+        pass2(j, tj, kj, b);
+    }
+    __syncwarp();
+    // block totals of every weight: the lanes take a block's events in strides
+    // of 32 and a butterfly reduction adds the lane sums (a fixed order for a
+    // given event count); then the collided sums before each block (exclusive
+    // prefix over blocks) and the uncollided sums after each block (exclusive
+    // suffix plus the never-colliding weights), as warp scans over lanes = blocks
+    for (int b = lane; b < NB; b += 32)
+        if (boff[b] == boff[b + 1]) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) btot[(size_t)q * NB + b] = 0.0;
+        }
+    for (int bc = 0; bc < NB; bc += 32) {
+        const int bl = bc + lane;
+        for (unsigned h = __ballot_sync(full, bl < NB && boff[bl] != boff[bl + 1]); h; h &= h - 1) {
+            const int b = bc + __ffs(h) - 1;
+            double t[NQ];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) t[q] = 0.0;
+            for (int e = boff[b] + lane; e < boff[b + 1]; e += 32) {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) t[q] += evq[(size_t)q * EV + e];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) t[q] += __shfl_xor_sync(full, t[q], o);
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) btot[(size_t)q * NB + b] = t[q];
+            }
+        }
+    }
+    __syncwarp();
+    {
+        double carry[2 * SMC];
+#pragma unroll
+        for (int q = 0; q < 2 * SMC; ++q) carry[q] = 0.0;
+        for (int bc = 0; bc < NB; bc += 32) {
+            const int b = bc + lane;
+            double v[2 * SMC];
+#pragma unroll
+            for (int q = 0; q < 2 * SMC; ++q) v[q] = b < NB ? btot[(size_t)(2 + q) * NB + b] : 0.0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+                for (int q = 0; q < 2 * SMC; ++q) {
+                    const double u = __shfl_up_sync(full, v[q], o);
+                    if (lane >= o) v[q] += u;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 2 * SMC; ++q) {
+                double ex = __shfl_up_sync(full, v[q], 1);
+                if (lane == 0) ex = 0.0;
+                if (b < NB) pbeg[(size_t)b * 2 * SMC + q] = carry[q] + ex;
+                carry[q] += __shfl_sync(full, v[q], 31);
+            }
+        }
+        // the never-colliding sums were reduced into lane 0
+        double cc = __shfl_sync(full, nc, 0), cs = __shfl_sync(full, ns, 0);
+        for (int bc = ((NB - 1) >> 5) << 5; bc >= 0; bc -= 32) {
+            const int b = bc + lane;
+            double vc = b < NB ? btot[b] : 0.0, vs = b < NB ? btot[(size_t)NB + b] : 0.0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double uc = __shfl_down_sync(full, vc, o), us = __shfl_down_sync(full, vs, o);
+                if (lane + o < 32) {
+                    vc += uc;
+                    vs += us;
+                }
+            }
+            double xc = __shfl_down_sync(full, vc, 1), xs = __shfl_down_sync(full, vs, 1);
+            if (lane == 31) xc = xs = 0.0;
+            if (b < NB) {
+                uend[2 * b] = cc + xc;
+                uend[2 * b + 1] = cs + xs;
+            }
+            cc += __shfl_sync(full, vc, 0);
+            cs += __shfl_sync(full, vs, 0);
+        }
+    }
+    __syncwarp();
+    // pass 3.  Blocks holding events ("event blocks") are formed one at a time
+    // with lane = step: each lane sums the events at its own step (their block
+    // offsets are compared four at a time as bytes), then warp scans give the
+    // collided sums up to and the uncollided sums after every step.  Blocks
+    // without events have constant sums: each lane forms 4 consecutive steps,
+    // 8 lanes a block, 4 such blocks at a time (int8 digits: 16 steps, 2 lanes
+    // a block, 16 blocks at a time).  The int8 digit layout needs the row's
+    // scale, max |beta| over its steps and columns, before any digit: a first
+    // sweep forms every value and keeps only the maximum.
+    const double ci = A.cos_t[i];
+    const double vi = (i == 0 || i == A.n_cos - 1) ? 0.5 : 1.0;
+    const double rf = (0.5 * (1.0 - ci * ci) * A.dphi) * (A.dcos * vi) * A.dt * (1.0 / (6.0 * CUDART_PI));
+    const double* Dslot = A.D + (size_t)slot * (1 + SMC) * A.tf;
+    const int nbase = (slot % A.bpt) * 2 * A.S;
+    int8_t* blk_row = beta + (((size_t)frame * A.n_cos + i) * A.tiles + slot / A.bpt) * (size_t)NB * kI8BlockSet;
+    // beta of coefficient set s at step k from the sums there: the table row
+    // holds the step weight times dt^3 and times a_m dt^{3-p_m} e^{-dt/w}
+    auto value = [&](int k, int s, const double* P, double Uc, double Us, double mul, double& xc, double& xs) {
+        double g[1 + SMC];
+#pragma unroll
+        for (int q = 0; q < 1 + SMC; ++q) g[q] = __ldg(Dslot + (size_t)q * A.tf + min(k, A.n_t - 1));
+        double vc = g[0] * Uc, vs = g[0] * Us;
+        const int t0 = s * A.M, t1 = t0 + A.M;  // the terms of set s
+#pragma unroll
+        for (int t = 0; t < SMC; ++t) {
+            if (t < t0 || t >= t1) continue;
+            vc += g[1 + t] * P[2 * t];
+            vs += g[1 + t] * P[2 * t + 1];
+        }
+        const double r = k < A.n_t ? mul : 0.0;
+        xc = r * vc;
+        xs = r * vs;
+    };
+    // Collided sums through step (b << 5) + lane and uncollided sums after it, for
+    // block b, lane = step (the whole warp calls it with the same b).
+    auto step_sums = [&](int b, double (&P)[2 * SMC], double& Uc, double& Us) {
+        const int e0 = boff[b], e1 = boff[b + 1];
+        if (e0 == e1) {  // a block without events: constant sums
+#pragma unroll
+            for (int q = 0; q < 2 * SMC; ++q) P[q] = pbeg[(size_t)b * 2 * SMC + q];
+            Uc = uend[2 * b];
+            Us = uend[2 * b + 1];
+            return;
+        }
+        double dq[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) dq[q] = 0.0;
+        if (e1 - e0 > 32) {
+            // Many events: the block's events are counting-sorted by their step (stable in event
+            // order; ranks within 32 events from __match_any groups), then each lane adds the
+            // events of its own step in event order.
+            int* run = scnt + 32;
+            scnt[lane] = 0;
+            __syncwarp();
+            for (int r0 = e0; r0 < e1; r0 += 32) {
+                const int e = r0 + lane;
+                const int se = e < e1 ? (int)evs[e] : 32 + lane;
+                const unsigned m = __match_any_sync(full, se);
+                if (e < e1 && lane == __ffs(m) - 1) scnt[se] += __popc(m);
+                __syncwarp();
+            }
+            const int c = scnt[lane];
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(full, incl, o);
+                if (lane >= o) incl += t;
+            }
+            const int ex = incl - c;  // first position of this lane's step
+            run[lane] = ex;
+            __syncwarp();
+            const unsigned lt = (1u << lane) - 1u;
+            for (int r0 = e0; r0 < e1; r0 += 32) {
+                const int e = r0 + lane;
+                const bool v = e < e1;
+                const int se = v ? (int)evs[e] : 32 + lane;
+                const unsigned m = __match_any_sync(full, se);
+                if (v) sperm[run[se] + __popc(m & lt)] = (uint16_t)e;
+                __syncwarp();
+                if (v && lane == __ffs(m) - 1) run[se] += __popc(m);
+                __syncwarp();
+            }
+            for (int r = 0; r < c; ++r) {
+                const double* qe = evq + sperm[ex + r];
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) dq[q] += qe[(size_t)q * EV];
+            }
+            __syncwarp();
+        } else {
+            const uint32_t pat = 0x01010101u * (uint32_t)lane;
+            for (int e4 = e0 & ~3; e4 < e1; e4 += 4) {
+                uint32_t eq = __vcmpeq4(*reinterpret_cast<const uint32_t*>(evs + e4), pat);
+                if (e4 < e0) eq &= 0xffffffffu << (8 * (e0 - e4));
+                if (e1 - e4 < 4) eq &= (1u << (8 * (e1 - e4))) - 1u;
+                while (eq) {
+                    const int by = (__ffs(eq) - 1) >> 3;
+                    eq &= ~(0xffu << (8 * by));
+                    const double* qe = evq + (e4 + by);
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) dq[q] += qe[(size_t)q * EV];
+                }
+            }
+        }
+        // collided sums through this step (inclusive scan), uncollided after it (suffix scan)
+        double uc = dq[0], us = dq[1];
+#pragma unroll
+        for (int q = 0; q < 2 * SMC; ++q) P[q] = dq[2 + q];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+            for (int q = 0; q < 2 * SMC; ++q) {
+                const double v = __shfl_up_sync(full, P[q], o);
+                if (lane >= o) P[q] += v;
+            }
+            const double vc = __shfl_down_sync(full, uc, o), vs = __shfl_down_sync(full, us, o);
+            if (lane + o < 32) {
+                uc += vc;
+                us += vs;
+            }
+        }
+        // uncollided after this step: the next step's inclusive suffix sum
+        Uc = __shfl_down_sync(full, uc, 1);
+        Us = __shfl_down_sync(full, us, 1);
+        if (lane == 31) Uc = Us = 0.0;
+        Uc += uend[2 * b];
+        Us += uend[2 * b + 1];
+#pragma unroll
+        for (int q = 0; q < 2 * SMC; ++q) P[q] = pbeg[(size_t)b * 2 * SMC + q] + P[q];
+    };
+    // The row's scale is max |beta| over its steps and columns, found exactly without
+    // forming every value.
+    // (a) Every event block is formed once (lane = step) and its 2S values are kept for the
+    //     digits: a block of at least 32 events in its own weight slots (plane 2s + g, slots
+    //     boff[b] + lane; its weights are not read again), smaller blocks in the block-total
+    //     table while it has room (the rest are formed again in (c)).
+    // (b) In a block without events U and Pm are constant, so beta = rf (D0(k) U + sum_m Dm(k)
+    //     Pm) is bounded by interval arithmetic over the per-block ranges of the time table;
+    //     such blocks are formed (lane = step) in decreasing order of their bound until no
+    //     bound exceeds the largest value found (most often one block: the last one, where
+    //     dt^3 peaks).
+    // (c) Digits of every block.
+    double vmax = 0.0;
+    const double* Dmx = A.Dmax + (size_t)slot * NB * (1 + SMC) * 2;
+    int* where = brun;  // per event block: -1 not kept, -2 own slots, c >= 0 table slot c
+    const int n_tab = (NQ * NB) / (64 * A.S);
+    int used_tab = 0;
+    auto kept = [&](int b, int& stride) -> double* {
+        const int w = where[b];
+        if (w == -2) {
+            stride = EV;
+            return evq + boff[b];
+        }
+        stride = 32;
+        return w >= 0 ? btot + (size_t)w * 64 * A.S : nullptr;
+    };
+    for (int bc = 0; bc < NB; bc += 32) {
+        const int bl = bc + lane;
+        for (unsigned h = __ballot_sync(full, bl < NB && boff[bl] != boff[bl + 1]); h; h &= h - 1) {
+            const int b = bc + __ffs(h) - 1;
+            double P[2 * SMC], Uc, Us;
+            step_sums(b, P, Uc, Us);
+            const int k = (b << 5) + lane;
+            const int code = boff[b + 1] - boff[b] >= 32 ? -2 : (used_tab < n_tab ? used_tab++ : -1);
+            __syncwarp();
+            if (lane == 0) where[b] = code;
+            __syncwarp();
+            int stride = 0;
+            double* dst = kept(b, stride);
+            for (int s2 = 0; s2 < A.S; ++s2) {
+                double xc, xs;
+                value(k, s2, P, Uc, Us, rf, xc, xs);
+                vmax = fmax(vmax, fmax(fabs(xc), fabs(xs)));
+                if (dst) {
+                    dst[(size_t)(2 * s2) * stride + lane] = xc;
+                    dst[(size_t)(2 * s2 + 1) * stride + lane] = xs;
+                }
+            }
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(full, vmax, o));
+    for (int bc = 0; bc < NB; bc += 32) {
+        const int bl = bc + lane;
+        double bnd = -1.0;  // this lane's block's bound (-1: none or an event block)
+        if (bl < NB && boff[bl] == boff[bl + 1]) {
+            // beta of set s, column g lies in rf (D0 [U] + sum_m Dm [Pm]) with D in [min, max]
+            // over the block and U, Pm the block's constants
+            const double* mx = Dmx + (size_t)bl * (1 + SMC) * 2;
+            auto term = [&](double dlo, double dhi, double c, double& lo, double& hi, double& sa) {
+                const double p0 = dlo * c, p1 = dhi * c;
+                lo += fmin(p0, p1);
+                hi += fmax(p0, p1);
+                sa += fmax(fabs(dlo), fabs(dhi)) * fabs(c);
+            };
+            for (int s2 = 0; s2 < A.S; ++s2) {
+                const int t0 = s2 * A.M, t1 = t0 + A.M;
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    double lo = 0.0, hi = 0.0, sa = 0.0;
+                    term(mx[0], mx[1], uend[2 * bl + g], lo, hi, sa);
+#pragma unroll
+                    for (int q = 0; q < SMC; ++q)
+                        if (q >= t0 && q < t1)
+                            term(mx[2 + 2 * q], mx[3 + 2 * q], pbeg[(size_t)bl * 2 * SMC + 2 * q + g], lo, hi, sa);
+                    // relative and absolute margins cover the rounding of these sums and of
+                    // the values themselves (a few ulp of the summed magnitudes)
+                    bnd = fmax(bnd, (fmax(fabs(lo), fabs(hi)) * (1.0 + 1e-12) + 1e-13 * sa) * rf);
+                }
+            }
+        }
+        for (;;) {
+            double bb = bnd;
+            int bi = lane;
+            for (int o = 16; o > 0; o >>= 1) {
+                const double ob = __shfl_xor_sync(full, bb, o);
+                const int oi = __shfl_xor_sync(full, bi, o);
+                if (ob > bb || (ob == bb && oi < bi)) {
+                    bb = ob;
+                    bi = oi;
+                }
+            }
+            // Every remaining bound is covered once no bound exceeds vmax (1 + 1e-10): a value up
+            // to that much above the scale still maps to |x F| <= F + 0.22, which rounds into the
+            // digit range.  (Without the slack, blocks whose values all equal the maximum, as after
+            // the last collision with powers = 3, would each be formed.)
+            if (!(bb > vmax * (1.0 + 1e-10))) break;
+            {
+                const int b = bc + bi, k = (b << 5) + lane;
+                const double* P = pbeg + (size_t)b * 2 * SMC;
+                const double Uc = uend[2 * b], Us = uend[2 * b + 1];
+                double m = 0.0;
+                for (int s2 = 0; s2 < A.S; ++s2) {
+                    double xc, xs;
+                    value(k, s2, P, Uc, Us, rf, xc, xs);
+                    m = fmax(m, fmax(fabs(xc), fabs(xs)));
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(full, m, o));
+                vmax = fmax(vmax, m);
+            }
+            if (lane == bi) bnd = -1.0;
+        }
+    }
+    if (lane == 0) A.scale[row] = vmax;
+    const double inv = vmax > 0.0 ? 1.0 / vmax : 0.0;
+    const double rinv = rf * inv;
+    // digits (streaming stores: the GEMM reads them back from DRAM).  Event blocks: lane = step; a
+    // quad of lanes transposes its packed digit
+    // words so that lane 4q + d holds digit d of steps 4q .. 4q + 3.  Blocks without
+    // events: 4 steps per lane (8 lanes a block, 4 blocks at a time), transposed in
+    // registers.  Either way a store instruction fills whole 32-byte rows of the blocks.
+    const bool odd = lane & 1, hi = lane & 2;
+    auto quad_transpose = [&](uint32_t p) {
+        const uint32_t t1 = __shfl_xor_sync(full, p, 1);
+        p = __byte_perm(p, t1, odd ? 0x3715 : 0x6240);
+        const uint32_t t2 = __shfl_xor_sync(full, p, 2);
+        return __byte_perm(p, t2, hi ? 0x3276 : 0x5410);
+    };
+    const int dg = lane & 3, s4 = (lane >> 2) * 4;
+    for (int bc = 0; bc < NB; bc += 32) {
+        const int bl = bc + lane;
+        const bool has = bl < NB && boff[bl] != boff[bl + 1];
+        const unsigned ev_blocks = __ballot_sync(full, has);
+        unsigned quiet = __ballot_sync(full, bl < NB && !has);
+        for (unsigned h = ev_blocks; h; h &= h - 1) {
+            const int b = bc + __ffs(h) - 1;
+            const int k = (b << 5) + lane;
+            int stride = 0;
+            const double* src = kept(b, stride);
+            double P[2 * SMC], Uc = 0.0, Us = 0.0;
+            if (!src) step_sums(b, P, Uc, Us);
+            int8_t* blk = blk_row + (size_t)b * kI8BlockSet + dg * kI8Block;
+            for (int s2 = 0; s2 < A.S; ++s2) {
+                double xc, xs;
+                if (src) {
+                    xc = src[(size_t)(2 * s2) * stride + lane];
+                    xs = src[(size_t)(2 * s2 + 1) * stride + lane];
+                } else {
+                    value(k, s2, P, Uc, Us, rf, xc, xs);
+                }
+                const uint32_t wc = quad_transpose(i8_digits(xc * inv));
+                const uint32_t ws = quad_transpose(i8_digits(xs * inv));
+                __stcs(reinterpret_cast<unsigned int*>(blk + i8_swz(nbase + 2 * s2, s4)), wc);
+                __stcs(reinterpret_cast<unsigned int*>(blk + i8_swz(nbase + 2 * s2 + 1, s4)), ws);
+            }
+        }
+        const int sub = lane >> 3, s0 = (lane & 7) * 4;
+        while (quiet) {
+            unsigned t = quiet;
+            for (int g = 0; g < sub && t; ++g) t &= t - 1;
+            const int b = t ? bc + __ffs(t) - 1 : -1;
+            for (int g = 0; g < 4 && quiet; ++g) quiet &= quiet - 1;
+            if (b < 0) continue;
+            const int k0 = (b << 5) + s0;
+            // the block's constant sums, with rf / scale folded in: 1 + SMC products per
+            // value (steps past n_t, in the last block only, go through value())
+            const bool tail = k0 + 4 > A.n_t;
+            double P[2 * SMC];
+#pragma unroll
+            for (int q = 0; q < 2 * SMC; ++q) P[q] = rinv * pbeg[(size_t)b * 2 * SMC + q];
+            const double Uc = rinv * uend[2 * b], Us = rinv * uend[2 * b + 1];
+            const double* Db = Dslot + k0;
+            int8_t* blk = blk_row + (size_t)b * kI8BlockSet;
+            for (int s2 = 0; s2 < A.S; ++s2) {
+                uint32_t pc[4], ps[4];
+                const int t0 = s2 * A.M, t1 = t0 + A.M;  // the terms of set s2
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    double xc, xs;
+                    if (tail) {
+                        value(k0 + m, s2, P, Uc, Us, 1.0, xc, xs);
+                    } else {
+                        double g[1 + SMC];
+#pragma unroll
+                        for (int q = 0; q < 1 + SMC; ++q) g[q] = __ldg(Db + (size_t)q * A.tf + m);
+                        xc = g[0] * Uc;
+                        xs = g[0] * Us;
+#pragma unroll
+                        for (int q = 0; q < SMC; ++q) {
+                            if (SMC > 1 && (q < t0 || q >= t1)) continue;
+                            xc = fma(g[1 + q], P[2 * q], xc);
+                            xs = fma(g[1 + q], P[2 * q + 1], xs);
+                        }
+                    }
+                    pc[m] = i8_digits(xc);
+                    ps[m] = i8_digits(xs);
+                }
+                uint32_t wc[4], ws[4];
+                i8_transpose4(pc[0], pc[1], pc[2], pc[3], wc);
+                i8_transpose4(ps[0], ps[1], ps[2], ps[3], ws);
+                const int oc = i8_swz(nbase + 2 * s2, s0), os = i8_swz(nbase + 2 * s2 + 1, s0);
+#pragma unroll
+                for (int d = 0; d < kI8Slices; ++d) {
+                    __stcs(reinterpret_cast<unsigned int*>(blk + d * kI8Block + oc), wc[d]);
+                    __stcs(reinterpret_cast<unsigned int*>(blk + d * kI8Block + os), ws[d]);
+                }
+            }
+        }
+    }
+}
+
+template <int SMC>
+static void launch_sorted_smc(BetaArgs& B, int8_t* out, cudaStream_t st) {
+    const int NQ = 2 + 2 * SMC, n_phi = B.n_phi;
+    size_t pw = (size_t)n_phi * NQ * sizeof(double) + 2 * (size_t)NQ * B.nblk * sizeof(double) +
+                (2 * (size_t)B.nblk + 1) * sizeof(int) + (((size_t)n_phi + 4 + 3) & ~(size_t)3) + 64 * sizeof(int) +
+                (size_t)n_phi * sizeof(uint16_t);
+    pw = (pw + 15) & ~(size_t)15;
+    B.per_warp_bytes = (int)pw;
+    const int warps = (int)std::min<size_t>(8, (200 * 1024) / pw);
+    if (warps < 1) throw Error{"n_phi too large for the beta kernel"};
+    const size_t smem = (size_t)warps * pw;
+    CUDA_OK(cudaFuncSetAttribute(k_beta_sorted<SMC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CUDA_OK(cudaFuncSetAttribute(k_beta_sorted<SMC>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared));
+    k_beta_sorted<SMC><<<(unsigned)((B.n_rows + warps - 1) / warps), warps * 32, smem, st>>>(B, out);
+}
+
+static void launch_sorted(int SM, BetaArgs& B, int8_t* out, cudaStream_t st) {
+    switch (SM) {
+        case 1: return launch_sorted_smc<1>(B, out, st);
+        case 2: return launch_sorted_smc<2>(B, out, st);
+        case 3: return launch_sorted_smc<3>(B, out, st);
+        case 4: return launch_sorted_smc<4>(B, out, st);
+        case 5: return launch_sorted_smc<5>(B, out, st);
+        case 6: return launch_sorted_smc<6>(B, out, st);
+        case 7: return launch_sorted_smc<7>(B, out, st);
+        default: return launch_sorted_smc<8>(B, out, st);
     }
 }
 
@@ -1086,22 +1727,29 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
         B.tile_cols = G.tile_cols;
         B.bpt = G.bpt;
         B.t_pad = G.t_pad;
-        // shared memory of a warp: a segment's bins (a second segment's too while three blocks of 8 warps
-        // still fit an SM), the quiet constants, the row's delays and steps; of the block: the weights
+        // shared memory of a warp: a segment's bins (a second segment's too while the blocks still fit an
+        // SM), the quiet constants, the row's delays and steps; of the block: the weights
         const size_t pitch = (((size_t)n_phi + 31) / 32) | 1;
-        const size_t bins = (size_t)(2 + 2 * SM) * kSeg, others = 4 + 2 * (size_t)SM + 32 * pitch + 16 * pitch;
-        B.keep = tc && 3 * (64 * pitch + 8 * (2 * bins + others)) * sizeof(double) <= 220 * 1024 ? 2 : 1;
+        const size_t bins = (size_t)(2 + 2 * SM) * kSeg;
+        const size_t others = 4 + 2 * (size_t)SM + beta_rows_held(SM) * 32 * pitch + 16 * pitch;
+        const size_t blocks_sm = beta_blocks(SM), most = beta_warps(SM);
+        B.keep = tc && blocks_sm * (64 * pitch + most * (2 * bins + others)) * sizeof(double) <= 220 * 1024 ? 2 : 1;
         const size_t per_warp = (B.keep * bins + others + 1) & ~(size_t)1;
         B.per_warp = (int)per_warp;
         B.tiles = G.tiles_per_frame;
         B.scale = tc ? (double*)dev->beta_scale.p : nullptr;
         B.Dmax = tc ? (const double*)dev->fact_Dmax.p : nullptr;
-        const size_t room = 220 * 1024 / sizeof(double);
-        if (64 * pitch + per_warp > room) throw Error{"n_phi too large for the beta kernel"};
-        const int warps = (int)std::min<size_t>(8, (room - 64 * pitch) / per_warp);
-        const size_t smem = (64 * pitch + warps * per_warp) * sizeof(double);
-        const unsigned blocks = (unsigned)((B.n_rows + warps - 1) / warps);
-        launch_beta<Real>(SM, B, (Real*)dev->beta.p, smem, blocks, warps * 32, dev->stream);
+        bool sorted = false;
+        if constexpr (tc) sorted = job.keep_masks;
+        if (sorted) {
+            if constexpr (tc) launch_sorted(SM, B, (int8_t*)dev->beta.p, dev->stream);
+        } else {
+            const size_t room = 220 * 1024 / sizeof(double);
+            if (64 * pitch + per_warp > room) throw Error{"n_phi too large for the beta kernel"};
+            const int warps = (int)std::min<size_t>(most, (room - 64 * pitch) / per_warp);
+            const size_t smem = (64 * pitch + warps * per_warp) * sizeof(double);
+            launch_beta<Real>(SM, B, (Real*)dev->beta.p, smem, dev->n_sm, warps, dev->stream);
+        }
         CUDA_OK(cudaGetLastError());
         ++launches;
     }
