@@ -241,9 +241,13 @@ void compute_common(bgw_generalized_bulk_flow* h, const double* w_arr, size_t n_
     if (out_device && out_len != expected)
         throw Error{"out_len=" + std::to_string(out_len) + " does not match expected length " +
                     std::to_string(expected)};
-    std::vector<double> result(out_device ? 0 : 2 * expected, 0.0);
+    // the result goes straight into the caller's array (a wrong length is reported after the computation,
+    // as it always was)
+    static_assert(sizeof(BgwComplex64) == 2 * sizeof(double), "interleaved complex");
+    const bool direct = out && out_len == expected;
+    std::vector<double> result(out_device || direct ? 0 : 2 * expected, 0.0);
     h->timings = BgwxTimings{};
-    bool device_written = false;
+    bool device_written = false, written = false;
     if (!ids.empty()) {
         double tb = has_t_begin ? t_begin : 0.0;
         if (tb > t_end)
@@ -264,7 +268,9 @@ void compute_common(bgw_generalized_bulk_flow* h, const double* w_arr, size_t n_
                 bgw::run_spectrum(device(h), job, static_cast<double*>(out_device), true, &h->timings);
                 device_written = true;
             } else {
-                bgw::run_spectrum(device(h), job, result.data(), false, &h->timings);
+                bgw::run_spectrum(device(h), job, direct ? reinterpret_cast<double*>(out) : result.data(), false,
+                                  &h->timings);
+                written = direct;
             }
         }
     }
@@ -277,7 +283,8 @@ void compute_common(bgw_generalized_bulk_flow* h, const double* w_arr, size_t n_
         throw Error{"out_len=" + std::to_string(out_len) + " does not match expected length " +
                     std::to_string(expected)};
     BgwComplex64* o = const_cast<BgwComplex64*>(slice(out, out_len, "out"));
-    for (size_t q = 0; q < expected; ++q) o[q] = BgwComplex64{result[2 * q], result[2 * q + 1]};
+    if (!written)  // nothing radiates
+        for (size_t q = 0; q < expected; ++q) o[q] = BgwComplex64{0.0, 0.0};
 }
 
 }  // namespace
@@ -767,10 +774,8 @@ void integrand_common(bgw_generalized_bulk_flow* bulk_flow, const double* w_arr,
         job.sel = live.data();
         job.n_sel = live.size();
         job.tensor = tensor;
-        std::vector<double> result(2 * expected);
         h->timings = BgwxTimings{};
-        bgw::run_integrand(device(h), job, result.data(), &h->timings);
-        for (size_t q = 0; q < expected; ++q) o[q] = BgwComplex64{result[2 * q], result[2 * q + 1]};
+        bgw::run_integrand(device(h), job, reinterpret_cast<double*>(o), &h->timings);
     }
 }
 }  // namespace

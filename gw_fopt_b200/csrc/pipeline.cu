@@ -71,6 +71,7 @@ Device::~Device() {
     if (stream) cudaStreamSynchronize(stream);
     if (ens_graph) cudaGraphExecDestroy(ens_graph);
     if (own_stream) cudaStreamDestroy(own_stream);
+    if (pinned) cudaFreeHost(pinned);
     for (auto& e : ev)
         if (e) cudaEventDestroy(e);
     for (auto& e : chunk_ev)
@@ -120,13 +121,46 @@ T* upload(Device* dev, DevBuf& buf, const T* host, size_t n, BgwxTimings* tm) {
     return static_cast<T*>(buf.p);
 }
 
-size_t mask_budget_bytes() {
+// Work-array budget for a call that could use `need` bytes: a third of the free memory, at least 256 MiB
+// (a smaller need asks no further: the query takes 67 us, a quarter of a small call) and at most 64 GiB.
+size_t mask_budget_bytes(size_t need) {
+    const size_t least = (size_t)256 << 20, cap = (size_t)64 << 30;
+    if (need <= least) return least;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return (size_t)1 << 30;
-    size_t b = free_b / 3;
-    const size_t cap = (size_t)64 << 30;
-    return std::max<size_t>((size_t)256 << 20, std::min(b, cap));
+    return std::max<size_t>(least, std::min(free_b / 3, cap));
 }
+
+// Device -> host copies of a call's small results: queued into pinned memory, handed over after the one
+// synchronisation (copies to pageable memory wait for the device one by one).  A larger copy goes directly.
+struct Readback {
+    static constexpr size_t kBytes = 1 << 18;
+    Device* dev;
+    size_t used = 0;
+    struct Part {
+        void* dst;
+        size_t at, bytes;
+    };
+    std::vector<Part> parts;
+    explicit Readback(Device* d) : dev(d) {
+        if (!dev->pinned) CUDA_OK(cudaMallocHost(&dev->pinned, kBytes));
+    }
+    void add(void* dst, const void* src, size_t bytes) {
+        if (used + bytes <= kBytes) {
+            CUDA_OK(cudaMemcpyAsync(static_cast<char*>(dev->pinned) + used, src, bytes, cudaMemcpyDeviceToHost, dev->stream));
+            parts.push_back({dst, used, bytes});
+            used = (used + bytes + 15) & ~(size_t)15;
+        } else {
+            CUDA_OK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, dev->stream));
+        }
+    }
+    void wait() {
+        CUDA_OK(cudaStreamSynchronize(dev->stream));
+        for (const Part& p : parts) std::memcpy(p.dst, static_cast<char*>(dev->pinned) + p.at, p.bytes);
+        parts.clear();
+        used = 0;
+    }
+};
 
 }  // namespace
 
@@ -135,7 +169,7 @@ size_t spectrum_max_frames_per_launch(const Device* dev, const SpectrumJob& job)
     const size_t per_k = job.n_sel * nd * sizeof(double) +
                          (job.kernel == BGWX_KERNEL_FP64_DIRECT ? direct_bytes_per_frame(dev, job)
                                                                 : factored_bytes_per_frame(job));
-    const size_t kc = std::max<size_t>(1, mask_budget_bytes() / std::max<size_t>(per_k, 1));
+    const size_t kc = std::max<size_t>(1, mask_budget_bytes(per_k * job.n_k) / std::max<size_t>(per_k, 1));
     return std::min<size_t>(kc, 65535);
 }
 
@@ -165,14 +199,12 @@ void run_masks(Device* dev, const MaskJob& job, int32_t* out_codes, double* out_
     launch_mask_pipeline(dev, bub, bub, job.n_int, job.n_tot, sel, nullptr, job.n_sel, dirs, cosphi, sinphi, nd, job.n_phi, 1, (double*)dev->tau.p,
                          (int32_t*)dev->codes.p, (unsigned long long*)dev->counters.p, true, &nl);
     CUDA_OK(cudaEventRecord(dev->ev[1], dev->stream));
-    CUDA_OK(cudaMemcpyAsync(out_codes, dev->codes.p, job.n_sel * nd * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                            dev->stream));
-    if (out_tau)
-        CUDA_OK(cudaMemcpyAsync(out_tau, dev->tau.p, job.n_sel * nd * sizeof(double), cudaMemcpyDeviceToHost,
-                                dev->stream));
     unsigned long long fb = 0;
-    CUDA_OK(cudaMemcpyAsync(&fb, dev->counters.p, sizeof fb, cudaMemcpyDeviceToHost, dev->stream));
-    CUDA_OK(cudaStreamSynchronize(dev->stream));
+    Readback back(dev);
+    back.add(out_codes, dev->codes.p, job.n_sel * nd * sizeof(int32_t));
+    if (out_tau) back.add(out_tau, dev->tau.p, job.n_sel * nd * sizeof(double));
+    back.add(&fb, dev->counters.p, sizeof fb);
+    back.wait();
     float ms = 0;
     CUDA_OK(cudaEventElapsedTime(&ms, dev->ev[0], dev->ev[1]));
     if (tm) {
@@ -229,10 +261,14 @@ static void add_stage_times(Device* dev, BgwxTimings* tm) {
 
 // Error counters of a call: [0] mask fallbacks (u64), [1] non-zero when a
 // tensor-core pipeline wait gave up.
-static void check_counters(Device* dev, unsigned long long* fallbacks) {
+// Waits for the call's work; `out`, `bytes`: its result, copied along.
+static void check_counters(Device* dev, unsigned long long* fallbacks, void* out = nullptr, const void* src = nullptr,
+                           size_t bytes = 0) {
     unsigned long long cnt[2] = {0, 0};
-    CUDA_OK(cudaMemcpyAsync(cnt, dev->counters.p, sizeof cnt, cudaMemcpyDeviceToHost, dev->stream));
-    CUDA_OK(cudaStreamSynchronize(dev->stream));
+    Readback back(dev);
+    back.add(cnt, dev->counters.p, sizeof cnt);
+    if (bytes) back.add(out, src, bytes);
+    back.wait();
     if (cnt[1] != 0) throw Error{"tensor-core GEMM: a pipeline wait gave up; the result is invalid"};
     if (fallbacks) *fallbacks = cnt[0];
 }
@@ -279,8 +315,8 @@ void run_spectrum(Device* dev, const SpectrumJob& job, double* out, bool out_is_
     dev->last_gemm_stages = 0;
     dev->last_mask_chunking = job.mask_chunking > 0 ? job.mask_chunking : 1;
     // masks kept for an adjoint call: every frame's delays and codes, written in place
-    const bool keep = job.keep_masks && !batched && !job.tensor &&
-                      K * job.n_sel * nd * (sizeof(double) + sizeof(int32_t)) <= mask_budget_bytes();
+    const size_t kept_bytes = K * job.n_sel * nd * (sizeof(double) + sizeof(int32_t));
+    const bool keep = job.keep_masks && !batched && !job.tensor && kept_bytes <= mask_budget_bytes(kept_bytes);
     if (keep) {
         dev->kept_valid = false;
         dev->kept_tau.ensure(K * job.n_sel * nd * sizeof(double));
@@ -353,9 +389,8 @@ void run_spectrum(Device* dev, const SpectrumJob& job, double* out, bool out_is_
         if (!nested) check_counters(dev, nullptr);
         return;
     }
-    CUDA_OK(cudaMemcpyAsync(out, final_out, out_blocks * per * sizeof(double2), cudaMemcpyDeviceToHost, dev->stream));
     unsigned long long fbk = 0;
-    check_counters(dev, &fbk);
+    check_counters(dev, &fbk, out, final_out, out_blocks * per * sizeof(double2));
     float total = 0;
     CUDA_OK(cudaEventElapsedTime(&total, dev->ev[4], dev->ev[5]));
     if (tm) {
@@ -520,8 +555,7 @@ void run_ensemble(Device* dev, const std::vector<SpectrumJob>& jobs, double* out
         }
     }
     CUDA_OK(cudaEventRecord(dev->ev[7], dev->stream));
-    CUDA_OK(cudaMemcpyAsync(out, eo, R * per_r * sizeof(double2), cudaMemcpyDeviceToHost, dev->stream));
-    check_counters(dev, nullptr);
+    check_counters(dev, nullptr, out, eo, R * per_r * sizeof(double2));
     float total = 0;
     CUDA_OK(cudaEventElapsedTime(&total, dev->ev[6], dev->ev[7]));
     if (tm) {
@@ -560,7 +594,7 @@ void run_adjoint(Device* dev, const SpectrumJob& job, const double* gbar, double
     double2* gb = reinterpret_cast<double2*>(upload(dev, dev->adj_gbar, gbar, 2 * K * per, tm));
 
     const size_t per_k = adjoint_bytes_per_frame(job);
-    size_t kc = std::max<size_t>(1, std::min(K, mask_budget_bytes() / std::max<size_t>(per_k, 1)));
+    size_t kc = std::max<size_t>(1, std::min(K, mask_budget_bytes(per_k * K) / std::max<size_t>(per_k, 1)));
     kc = std::min<size_t>(kc, 65535);
     const size_t rows = job.n_sel * job.n_cos;
     // the masks kept by the last spectrum call on the same inputs are reused (same stream, so that
@@ -623,9 +657,10 @@ void run_adjoint(Device* dev, const SpectrumJob& job, const double* gbar, double
                                          d_gpar);
     }
     CUDA_OK(cudaEventRecord(dev->ev[5], dev->stream));
-    CUDA_OK(cudaMemcpyAsync(g_bub, d_gbub, 4 * job.n_tot * sizeof(double), cudaMemcpyDeviceToHost, dev->stream));
-    CUDA_OK(cudaMemcpyAsync(g_par, d_gpar, 2 * SM * sizeof(double), cudaMemcpyDeviceToHost, dev->stream));
-    CUDA_OK(cudaStreamSynchronize(dev->stream));
+    Readback back(dev);
+    back.add(g_bub, d_gbub, 4 * job.n_tot * sizeof(double));
+    back.add(g_par, d_gpar, 2 * SM * sizeof(double));
+    back.wait();
     float total = 0;
     CUDA_OK(cudaEventElapsedTime(&total, dev->ev[4], dev->ev[5]));
     if (tm) {
@@ -667,8 +702,9 @@ void run_integrand(Device* dev, const SpectrumJob& job, double* out, BgwxTimings
                           coeffs, powers, t_arr,                     cutw,   w};
     launches += launch_direct_integrand(dev, job, in, (double2*)dev->out.p);
     CUDA_OK(cudaEventRecord(dev->ev[5], dev->stream));
-    CUDA_OK(cudaMemcpyAsync(out, dev->out.p, per * sizeof(double2), cudaMemcpyDeviceToHost, dev->stream));
-    CUDA_OK(cudaStreamSynchronize(dev->stream));
+    Readback back(dev);
+    back.add(out, dev->out.p, per * sizeof(double2));
+    back.wait();
     float total = 0;
     CUDA_OK(cudaEventElapsedTime(&total, dev->ev[4], dev->ev[5]));
     if (tm) {
