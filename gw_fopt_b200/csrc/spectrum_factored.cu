@@ -1442,72 +1442,44 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
             }
             __syncthreads();
             if (ch + 1 < n_chunks) fetch(k0 + kKC);  // in flight during the GEMM below
-            if constexpr (sizeof(Real) == 8) {
-#pragma unroll 4
-                for (int n = 0; n < kKC; ++n) {
-                    double a[kTM], bb[TN];
-                    const double2* ap = reinterpret_cast<const double2*>(Msm + n * kRows + ty * kTM);
-                    const double2* bp0 = reinterpret_cast<const double2*>(Bsm + n * BS + tx * (TN / 2));
-                    const double2* bp1 = reinterpret_cast<const double2*>(Bsm + n * BS + COLS / 2 + tx * (TN / 2));
-#pragma unroll
-                    for (int r = 0; r < kTM / 2; ++r) {
-                        const double2 v = ap[r];
-                        a[2 * r] = v.x;
-                        a[2 * r + 1] = v.y;
-                    }
-#pragma unroll
-                    for (int u = 0; u < TN / 4; ++u) {
-                        const double2 v0 = bp0[u], v1 = bp1[u];
-                        bb[2 * u] = v0.x;
-                        bb[2 * u + 1] = v0.y;
-                        bb[TN / 2 + 2 * u] = v1.x;
-                        bb[TN / 2 + 2 * u + 1] = v1.y;
-                    }
-#pragma unroll
-                    for (int r = 0; r < kTM; ++r)
-#pragma unroll
-                        for (int u = 0; u < TN; ++u) acc[r][u] = fma(a[r], bb[u], acc[r][u]);
-                }
-            } else {
 #pragma unroll 1
-                for (int n0 = 0; n0 < kKC; n0 += kFold) {
-                    float cacc[kTM][TN];
+            for (int n0 = 0; n0 < kKC; n0 += kFold) {
+                float cacc[kTM][TN];
 #pragma unroll
-                    for (int r = 0; r < kTM; ++r)
+                for (int r = 0; r < kTM; ++r)
 #pragma unroll
-                        for (int u = 0; u < TN; ++u) cacc[r][u] = 0.0f;
+                    for (int u = 0; u < TN; ++u) cacc[r][u] = 0.0f;
 #pragma unroll
-                    for (int n = n0; n < n0 + kFold; ++n) {
-                        float a[kTM], bb[TN];
-                        const float4* ap = reinterpret_cast<const float4*>(Msm + n * kRows + ty * kTM);
-                        const float4 b0 = *reinterpret_cast<const float4*>(Bsm + n * BS + tx * (TN / 2));
-                        const float4 b1 = *reinterpret_cast<const float4*>(Bsm + n * BS + COLS / 2 + tx * (TN / 2));
+                for (int n = n0; n < n0 + kFold; ++n) {
+                    float a[kTM], bb[TN];
+                    const float4* ap = reinterpret_cast<const float4*>(Msm + n * kRows + ty * kTM);
+                    const float4 b0 = *reinterpret_cast<const float4*>(Bsm + n * BS + tx * (TN / 2));
+                    const float4 b1 = *reinterpret_cast<const float4*>(Bsm + n * BS + COLS / 2 + tx * (TN / 2));
 #pragma unroll
-                        for (int r = 0; r < kTM / 4; ++r) {
-                            const float4 v = ap[r];
-                            a[4 * r] = v.x;
-                            a[4 * r + 1] = v.y;
-                            a[4 * r + 2] = v.z;
-                            a[4 * r + 3] = v.w;
-                        }
-                        bb[0] = b0.x;
-                        bb[1] = b0.y;
-                        bb[2] = b0.z;
-                        bb[3] = b0.w;
-                        bb[4] = b1.x;
-                        bb[5] = b1.y;
-                        bb[6] = b1.z;
-                        bb[7] = b1.w;
-#pragma unroll
-                        for (int r = 0; r < kTM; ++r)
-#pragma unroll
-                            for (int u = 0; u < TN; ++u) cacc[r][u] = fmaf(a[r], bb[u], cacc[r][u]);
+                    for (int r = 0; r < kTM / 4; ++r) {
+                        const float4 v = ap[r];
+                        a[4 * r] = v.x;
+                        a[4 * r + 1] = v.y;
+                        a[4 * r + 2] = v.z;
+                        a[4 * r + 3] = v.w;
                     }
+                    bb[0] = b0.x;
+                    bb[1] = b0.y;
+                    bb[2] = b0.z;
+                    bb[3] = b0.w;
+                    bb[4] = b1.x;
+                    bb[5] = b1.y;
+                    bb[6] = b1.z;
+                    bb[7] = b1.w;
 #pragma unroll
                     for (int r = 0; r < kTM; ++r)
 #pragma unroll
-                        for (int u = 0; u < TN; ++u) acc[r][u] += (double)cacc[r][u];
+                        for (int u = 0; u < TN; ++u) cacc[r][u] = fmaf(a[r], bb[u], cacc[r][u]);
                 }
+#pragma unroll
+                for (int r = 0; r < kTM; ++r)
+#pragma unroll
+                    for (int u = 0; u < TN; ++u) acc[r][u] += (double)cacc[r][u];
             }
             __syncthreads();
         }
@@ -1552,6 +1524,223 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
         if (wi >= A.n_w) continue;
         const size_t o = ((((size_t)frame * A.tiles_per_frame + tile) * 2 + g) * A.S + s) * A.n_w + wi;
         A.partial[o] = Cacc[q];
+    }
+}
+
+// FP64: the same product folded about the middle of the time grid.  Steps hi = h0 + d and lo = l0 - d lie
+// symmetrically about t_mid, so with theta_d = w (1 - c_i) (t_hi - t_lo) / 2
+//   sum_k e^{i w (1 - c_i) t_k} beta_k = e^{i w (1 - c_i) t_mid} [ sum_d cos theta_d (beta_hi + beta_lo)
+//                                                             + i sum_d sin theta_d (beta_hi - beta_lo) ]:
+// one real product per (frequency, pair) for each of Re and Im where the plain form has one per step, and
+// the middle phase goes into the epilogue's.  What bounds it: FP64 FMAs (half of the plain form's; 9.2 ms
+// before, of which 4.1 at the FP64 peak, for 4 frames of 512 bubbles x 128 rows x 512 steps x 128 w).  The
+// rows are split over CTAs, 8 rows each at least: a small call had 16 CTAs (1.7 ms for 8 frames of 48
+// bubbles).  The split depends on the grid alone, so that a realization's sums do not depend on its batch.
+constexpr int kFoldTN = 4, kFoldCols = 16 * kFoldTN, kFoldBS = kFoldCols + 2;
+
+struct FoldSmem {  // doubles
+    static constexpr int m = 0;                                // [kKC][kRows]
+    static constexpr int e = m + kKC * kRows;                  // [kKC][kFoldBS]
+    static constexpr int o = e + kKC * kFoldBS;
+    static constexpr int p_re = o + kKC * kFoldBS;             // [kKC][kWT]
+    static constexpr int p_im = p_re + kKC * kWT;
+    static constexpr int anc = p_im + kKC * kWT;               // [2][kWT]
+    static constexpr int main = anc + 2 * kWT;
+};
+static int fold_work(int S) { return std::max(FoldSmem::main, kThreads * 4 * 2 * S * 2); }  // or the epilogue's partials
+static size_t fold_smem_bytes(int S) {
+    return ((size_t)fold_work(S) + kWT * 2 * S * 2 + 2 * 64) * sizeof(double) + 64 * sizeof(int);
+}
+static int fold_row_parts(int n_cos) { return std::max(1, std::min(16, n_cos / 8)); }
+
+// e^{i w (t_a c - z_a + (1 - c) t_mid)} with the argument's roundings made good to first order: this phase
+// multiplies a whole row, where the plain form's time phases each had a rounding of their own.
+__device__ __forceinline__ void middle_phase(double w, double ta, double za, double c, double t_mid, double& s, double& co) {
+    const double d = __dsub_rn(1.0, c), ed = __dsub_rn(__dsub_rn(1.0, d), c);
+    const double p = __dmul_rn(ta, c), ep = fma(ta, c, -p);
+    const double q = __dmul_rn(d, t_mid), eq = fma(d, t_mid, -q);
+    // two-sums of p - za and of that + q
+    const double u = __dsub_rn(p, za), bu = __dsub_rn(p, u);
+    const double eu = __dadd_rn(__dsub_rn(p, __dadd_rn(u, bu)), __dsub_rn(bu, za));
+    const double v = __dadd_rn(u, q), bv = __dsub_rn(v, u);
+    const double ev = __dadd_rn(__dsub_rn(u, __dsub_rn(v, bv)), __dsub_rn(q, bv));
+    const double x = __dmul_rn(w, v);
+    const double e = fma(w, ((ep + eq) + (eu + ev)) + ed * t_mid, fma(w, v, -x));
+    double sn, cs;
+    sincos(x, &sn, &cs);
+    s = fma(e, cs, sn);
+    co = fma(-e, sn, cs);
+}
+
+__global__ void __launch_bounds__(kThreads, 1) k_gemm_fold(FactArgs A, int work) {
+    extern __shared__ __align__(16) double fsm[];
+    double* Msm = fsm + FoldSmem::m;
+    double* Esm = fsm + FoldSmem::e;
+    double* Osm = fsm + FoldSmem::o;
+    double* Pn_re = fsm + FoldSmem::p_re;
+    double* Pn_im = fsm + FoldSmem::p_im;
+    double* anc = fsm + FoldSmem::anc;
+    double2* red = reinterpret_cast<double2*>(fsm);            // [4 cpb][kThreads], between the rows' products
+    double2* Cacc = reinterpret_cast<double2*>(fsm + work);    // [kWT][2S]
+    double* bt = fsm + work + kWT * 2 * A.S * 2;               // [64] t_a
+    double* bz = bt + 64;                                      // [64] z_a
+    int* binfo = reinterpret_cast<int*>(bz + 64);              // [64]: slot or -1
+    constexpr int TN = kFoldTN, COLS = kFoldCols, BS = kFoldBS;
+    constexpr int NPRE = COLS * kKC / kThreads;
+
+    const int tid = threadIdx.x;
+    const int ty = tid / 16, tx = tid % 16;
+    const int w0 = blockIdx.x * kWT;
+    const int frame = blockIdx.y / A.tiles_per_frame;
+    const int tile = blockIdx.y % A.tiles_per_frame;
+    const int part = blockIdx.z, parts = gridDim.z;
+    const int cpb = 2 * A.S;
+    const D4* B = A.bub + (size_t)frame * A.n_tot;
+    const double* beta = static_cast<const double*>(A.beta);
+
+    if (tid < 64) {
+        const int slot = tile * A.bpt + tid;
+        const bool ok = tid < A.bpt && slot < A.n_sel && A.sel[slot] != kNoSlot;
+        binfo[tid] = ok ? slot : -1;
+        if (ok) {
+            const D4 xa = B[A.sel[slot]];
+            bt[tid] = xa.t;
+            bz[tid] = xa.z;
+        }
+    }
+    for (int q = tid; q < kWT * cpb; q += kThreads) Cacc[q] = make_double2(0.0, 0.0);
+    __syncthreads();
+    int kstart = A.n_t;
+    for (int b = 0; b < A.bpt; ++b)
+        if (binfo[b] >= 0) kstart = min(kstart, A.kfirst[binfo[b]]);
+    // pairs d: hi = h0 + d, lo = l0 - d (an odd grid's middle step is its own pair, d = 0)
+    const int h0 = A.n_t >> 1, l0 = (A.n_t - 1) >> 1;
+    const int n_pairs = A.n_t - h0;
+    const double t_mid = 0.5 * (A.t_arr[h0] + A.t_arr[l0]);
+    const int c_start = max(0, kstart - h0) / kKC;
+    const int n_chunks = kstart < A.n_t ? (n_pairs + kKC - 1) / kKC : 0;
+    const long col0 = (long)tile * COLS;
+    const int lane = tid & 31, wp = tid >> 5;
+
+    for (int i = A.n_cos * part / parts; i < A.n_cos * (part + 1) / parts; ++i) {
+        const double ci = A.cos_t[i];
+        const double one_m_c = 1.0 - ci;
+        for (int q = tid; q < kKC * kWT; q += kThreads) {
+            const int n = q / kWT, wl = q % kWT;
+            const int wi = w0 + wl;
+            double sn = 0.0, cs = 1.0;
+            if (wi < A.n_w) phase<double>(A.w[wi] * one_m_c * (n * A.dt), sn, cs);
+            Pn_re[q] = cs;
+            Pn_im[q] = sn;
+        }
+        const double* bi = beta + (((size_t)frame * A.n_cos + i) * A.cols_pad + col0) * A.t_pad;
+        // a warp's lanes take 32 consecutive pairs of one column: both halves are read in whole lines
+        double hi[NPRE], lo[NPRE];
+        auto fetch = [&](int d0) {
+            const int d = d0 + lane;
+            const bool in = d < n_pairs;
+#pragma unroll
+            for (int v = 0; v < NPRE; ++v) {
+                const double* c = bi + (size_t)(wp + 8 * v) * A.t_pad;
+                hi[v] = in ? __ldg(c + h0 + d) : 0.0;
+                lo[v] = in && h0 + d != l0 - d ? __ldg(c + l0 - d) : 0.0;
+            }
+        };
+        double acc[kTM][TN];
+#pragma unroll
+        for (int r = 0; r < kTM; ++r)
+#pragma unroll
+            for (int u = 0; u < TN; ++u) acc[r][u] = 0.0;
+        if (c_start < n_chunks) fetch(c_start * kKC);
+        __syncthreads();
+
+        for (int ch = c_start; ch < n_chunks; ++ch) {
+            const int d0 = ch * kKC;
+            if (tid < kWT) {
+                const int wi = w0 + tid;
+                double sn = 0.0, cs = 0.0;
+                if (wi < A.n_w) phase<double>(A.w[wi] * one_m_c * (0.5 * (A.t_arr[h0 + d0] - A.t_arr[l0 - d0])), sn, cs);
+                anc[tid] = cs;
+                anc[kWT + tid] = sn;
+            }
+#pragma unroll
+            for (int v = 0; v < NPRE; ++v) {
+                Esm[lane * BS + wp + 8 * v] = hi[v] + lo[v];
+                // (the middle step of an odd grid has no sine)
+                Osm[lane * BS + wp + 8 * v] = hi[v] - lo[v];
+            }
+            __syncthreads();
+            for (int q = tid; q < kKC * kWT; q += kThreads) {
+                const int n = q / kWT, wl = q % kWT;
+                const double ar = anc[wl], ai = anc[kWT + wl];
+                const double pr = Pn_re[q], pi = Pn_im[q];
+                const bool valid = d0 + n < n_pairs;
+                *reinterpret_cast<double2*>(Msm + n * kRows + 2 * wl) =
+                    valid ? make_double2(ar * pr - ai * pi, ar * pi + ai * pr) : make_double2(0.0, 0.0);
+            }
+            __syncthreads();
+            if (ch + 1 < n_chunks) fetch(d0 + kKC);  // in flight during the products below
+#pragma unroll 4
+            for (int n = 0; n < kKC; ++n) {
+                const double2* ap = reinterpret_cast<const double2*>(Msm + n * kRows + ty * kTM);
+                const double* ep = Esm + n * BS + tx * (TN / 2);
+                const double* op = Osm + n * BS + tx * (TN / 2);
+                const double2 e0 = *reinterpret_cast<const double2*>(ep), e1 = *reinterpret_cast<const double2*>(ep + COLS / 2);
+                const double2 o0 = *reinterpret_cast<const double2*>(op), o1 = *reinterpret_cast<const double2*>(op + COLS / 2);
+                const double e[TN] = {e0.x, e0.y, e1.x, e1.y}, o[TN] = {o0.x, o0.y, o1.x, o1.y};
+#pragma unroll
+                for (int r = 0; r < kTM / 2; ++r) {
+                    const double2 a = ap[r];  // cos, sin of frequency ty * 4 + r
+#pragma unroll
+                    for (int u = 0; u < TN; ++u) {
+                        acc[2 * r][u] = fma(a.x, e[u], acc[2 * r][u]);
+                        acc[2 * r + 1][u] = fma(a.y, o[u], acc[2 * r + 1][u]);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        // epilogue: per thread, C_{s,g}(w) partials of its columns in fixed order, in structure-of-arrays
+        // order red[(q*cpb + sg)*kThreads + tid]
+        for (int q = 0; q < 4 * cpb; ++q) red[(size_t)q * kThreads + tid] = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int q = 0; q < kTM / 2; ++q) {
+            const int wl = ty * (kTM / 2) + q;
+            const int wi = w0 + wl;
+#pragma unroll
+            for (int u = 0; u < TN; ++u) {
+                const int col = thread_col<TN, COLS>(tx, u);
+                const int b = col / cpb;
+                if (b >= A.bpt || binfo[b] < 0 || wi >= A.n_w) continue;
+                double sn, cs;
+                middle_phase(A.w[wi], bt[b], bz[b], ci, t_mid, sn, cs);
+                const double yr = acc[2 * q][u], yi = acc[2 * q + 1][u];
+                double2& d = red[(size_t)(q * cpb + (col % cpb)) * kThreads + tid];
+                d.x += cs * yr - sn * yi;
+                d.y += cs * yi + sn * yr;
+            }
+        }
+        __syncthreads();
+        for (int q = tid; q < kWT * cpb; q += kThreads) {
+            const int wl = q / cpb, sg = q % cpb;
+            const int tyw = wl / (kTM / 2), qq = wl % (kTM / 2);
+            double2 sum = Cacc[q];
+            for (int t = 0; t < 16; ++t) {
+                const double2 v = red[(size_t)(qq * cpb + sg) * kThreads + tyw * 16 + t];
+                sum.x += v.x;
+                sum.y += v.y;
+            }
+            Cacc[q] = sum;
+        }
+        __syncthreads();
+    }
+    for (int q = tid; q < kWT * cpb; q += kThreads) {
+        const int wl = q / cpb, sg = q % cpb;
+        const int s = sg >> 1, g = sg & 1;
+        const int wi = w0 + wl;
+        if (wi >= A.n_w) continue;
+        const size_t at = ((((size_t)frame * A.tiles_per_frame + tile) * parts + part) * 2 + g) * A.S + s;
+        A.partial[at * A.n_w + wi] = Cacc[q];
     }
 }
 
@@ -1603,9 +1792,6 @@ static size_t gemm_smem_bytes(int S) {
     b += 64 * sizeof(int) + 2 * 64 * sizeof(double);
     return b;
 }
-
-template <class Real>
-constexpr int gemm_tn() { return sizeof(Real) == 4 ? 8 : 4; }
 
 struct FactGeom {
     int bpt, tiles_per_frame, t_pad, nblk, tile_cols;
@@ -1777,11 +1963,14 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
     const size_t per = (size_t)2 * S * n_w;
     // tensor-core path: each column tile's CTAs split the cos-theta rows so that
     // the grid fills whole waves of one CTA per SM
+    constexpr bool fold = std::is_same<Real, double>::value;
     const int row_parts =
-        !tc ? 1
-            : job.row_parts > 0 ? std::min(std::min(job.row_parts, 16), n_cos)
-                                : tc_row_parts((size_t)((n_w + 63) / 64) * kn * G.tiles_per_frame, n_cos, dev->n_sm);
-    dev->last_row_parts = row_parts;
+        fold ? fold_row_parts(n_cos)
+        : !tc ? 1
+              : job.row_parts > 0 ? std::min(std::min(job.row_parts, 16), n_cos)
+                                  : tc_row_parts((size_t)((n_w + 63) / 64) * kn * G.tiles_per_frame, n_cos, dev->n_sm);
+    // (the launch shape's row parts are the tensor-core GEMM's)
+    dev->last_row_parts = tc ? row_parts : 1;
     dev->fact_partial.ensure((size_t)kn * G.tiles_per_frame * row_parts * per * sizeof(double2));
     A.partial = (double2*)dev->fact_partial.p;
     if constexpr (tc) {
@@ -1825,18 +2014,23 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
         launches += reduce_tiles(dev, job, A.partial, G.tiles_per_frame, row_parts, per, k0, kn, out, real_tiles);
         return launches;
     } else {
-        constexpr int TN = gemm_tn<Real>();
-        const size_t smem = gemm_smem_bytes<Real, TN>(S);
-        if (smem > 227 * 1024) throw Error{"too many coefficient sets for the factored kernel's shared memory"};
-        CUDA_OK(cudaFuncSetAttribute(k_gemm<Real, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const size_t smem = fold ? fold_smem_bytes(S) : gemm_smem_bytes<float, 8>(S);
+        if (smem > 227 * 1024 || (fold && S > 4))
+            throw Error{"too many coefficient sets for the factored kernel's shared memory"};
         const size_t gy = (size_t)kn * G.tiles_per_frame;
         if (gy > 65535) throw Error{"too many column tiles in one k-hat chunk"};
-        dim3 grid((unsigned)((n_w + kWT - 1) / kWT), (unsigned)gy);
-        k_gemm<Real, TN><<<grid, kThreads, smem, dev->stream>>>(A);
+        const dim3 grid((unsigned)((n_w + kWT - 1) / kWT), (unsigned)gy, (unsigned)row_parts);
+        if constexpr (fold) {
+            CUDA_OK(cudaFuncSetAttribute(k_gemm_fold, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            k_gemm_fold<<<grid, kThreads, smem, dev->stream>>>(A, fold_work(S));
+        } else {
+            CUDA_OK(cudaFuncSetAttribute(k_gemm<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            k_gemm<float, 8><<<grid, kThreads, smem, dev->stream>>>(A);
+        }
         CUDA_OK(cudaGetLastError());
         ++launches;
         record_event(dev, ev3[2]);
-        launches += reduce_tiles(dev, job, A.partial, G.tiles_per_frame, 1, per, k0, kn, out, real_tiles);
+        launches += reduce_tiles(dev, job, A.partial, G.tiles_per_frame, row_parts, per, k0, kn, out, real_tiles);
         return launches;
     }
 }
@@ -1879,8 +2073,8 @@ size_t factored_bytes_per_frame(const SpectrumJob& job) {
                             ? (size_t)job.n_cos * G.tiles_per_frame * G.nblk * kI8BlockSet +
                                   (size_t)job.n_sel * job.n_cos * sizeof(double)
                             : (size_t)job.n_cos * G.cols_pad * G.t_pad * real;
-    // partials: up to 16 row parts per column tile on the tensor-core path
-    const size_t parts = job.kernel == BGWX_KERNEL_MIXED ? 16 : 1;
+    // partials: up to 16 row parts per column tile on the tensor-core and the FP64 path
+    const size_t parts = job.kernel == BGWX_KERNEL_MIXED_SIMT ? 1 : 16;
     return beta + (size_t)G.tiles_per_frame * parts * 2 * job.n_sets * job.n_w * sizeof(double2);
 }
 
