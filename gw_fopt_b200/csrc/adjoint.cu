@@ -83,8 +83,10 @@ struct AdjArgs {
 //   P_{a,gs}(k) = sum_w H_{a,gs}(w) M_i(w, k),   H = conj(G_gs(w)) E_{a,i}(w),
 //   Re P = sum_w (Hr Mr - Hi Mi),   Im Q = sum_w w (Hr Mi + Hi Mr):
 // two real products of depth W per (frame, row), computed by k_adj_pq.
+// (V2: double2, or float2 for the FP32 products.)
+template <class V2>
 __global__ void k_adj_mtab(const double* __restrict__ cos_t, const double* __restrict__ t_arr,
-                           const double* __restrict__ w, int n_cos, int n_w, int n_t, double2* __restrict__ mt) {
+                           const double* __restrict__ w, int n_cos, int n_w, int n_t, V2* __restrict__ mt) {
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= (size_t)n_cos * n_w * n_t) return;
     const int k = (int)(q % n_t);
@@ -92,39 +94,48 @@ __global__ void k_adj_mtab(const double* __restrict__ cos_t, const double* __res
     const int i = (int)(q / ((size_t)n_t * n_w));
     double sn, cs;
     sincos(w[wi] * (t_arr[k] * (1.0 - cos_t[i])), &sn, &cs);
-    mt[q] = make_double2(cs, sn);
+    using R = decltype(mt->x);
+    mt[q] = V2{(R)cs, (R)sn};
 }
 
 constexpr int kPqRows = 64;   // (bubble, set, g) rows per tile
 constexpr int kPqCols = 64;   // time steps per tile
 constexpr int kPqW = 16;      // frequencies per shared-memory stage
 
-// One CTA per (row tile x step tile, cos-theta row i, frame).  Thread
+// One CTA per (row tile, cos-theta row i, frame), over all step tiles.  Thread
 // (ty, tx) of 16 x 16 owns rows ty + 16 u and steps tx + 16 v (u, v < 4).
 // F32: the products run in FP32 (H and M rounded to FP32, one FP32 sum per stage of kPqW
 // frequencies), each stage's sums added to FP64 accumulators: about 16 x 2^-24 of the terms
 // per stage instead of FP64 rounding, at twice the FMA rate.
+// w_held: frequencies whose H tile stays in shared memory: all of them (H is then formed once per CTA,
+// one sincos per (frequency, bubble)) or one stage (formed again for every step tile).  The M tiles are
+// fetched one stage ahead.  What bounds it: the FMAs (2.4 ms in FP32 for 32 frames of 256 bubbles, 64
+// rows, 256 steps, 64 w), then the FP64 folds: 5.14 ms there; with a CTA per step tile and a sincos per
+// (frequency, bubble, g) it took 6.22 ms (in FP64, one frame of 48 bubbles: 333 us, before 375).
 template <int S, bool F32>
-__global__ void __launch_bounds__(kAdjThreads) k_adj_pq(AdjArgs A, const double2* __restrict__ mt, int row_tiles) {
+__global__ void __launch_bounds__(kAdjThreads, F32 ? 2 : 1) k_adj_pq(AdjArgs A, const void* __restrict__ mtab, int w_held) {
     constexpr int S2 = 2 * S;
     using V2 = typename std::conditional<F32, float2, double2>::type;
     using R = typename std::conditional<F32, float, double>::type;
-    __shared__ V2 Hs[kPqW][kPqRows];
-    __shared__ V2 Ms[kPqW][kPqCols];
-    __shared__ R ws[kPqW];
+    extern __shared__ __align__(16) unsigned char pq_smem[];
+    V2* Hs = reinterpret_cast<V2*>(pq_smem);                 // [w_held][kPqRows]
+    V2* Ms = Hs + (size_t)w_held * kPqRows;                  // [2][kPqW][kPqCols]
+    R* ws = reinterpret_cast<R*>(Ms + 2 * kPqW * kPqCols);   // [w_held]: the frequencies of Hs
+    const V2* mt = static_cast<const V2*>(mtab);
     const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
-    const int rt = blockIdx.x % row_tiles, kt = blockIdx.x / row_tiles;
     const int i = blockIdx.y, f = blockIdx.z;
     const int W = A.n_w;
     const int n_rows = A.n_sel * S2;
-    const int r0 = rt * kPqRows, k0 = kt * kPqCols;
+    const int r0 = blockIdx.x * kPqRows;
+    // the tile's bubbles (the first and the last may lie in two tiles)
+    const int slot0 = r0 / S2, n_slots = (r0 + kPqRows - 1) / S2 - slot0 + 1;
     // k_adj_rows reads P and Q only at steps after a row's bubble nucleated: a tile whose steps
     // all precede that for every bubble of its rows has nothing to compute
     __shared__ int s_kmin;
     if (tid == 0) s_kmin = A.n_t;
     __syncthreads();
-    if (tid < kPqRows / S2) {
-        const int slot = r0 / S2 + tid;
+    if (tid < n_slots) {
+        const int slot = slot0 + tid;
         if (slot < A.n_sel) {
             const double ta = A.bub[(size_t)f * A.n_tot + A.sel[slot]].t;
             int lo = 0, hi = A.n_t;  // first step with t_k - t_a > 0 (monotone in k)
@@ -136,53 +147,80 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_pq(AdjArgs A, const double2
             atomicMin(&s_kmin, lo);
         }
     }
-    __syncthreads();
-    if (k0 + kPqCols <= s_kmin) return;
+    const int n_stages = (W + kPqW - 1) / kPqW;
     const double ci = A.cos_t[i];
+    // H of frequencies [w0, w0 + n) into Hs: row r = slot * S2 + gs
+    auto form_h = [&](int w0, int n) {
+        for (int q = tid; q < n; q += kAdjThreads) ws[q] = (R)(w0 + q < W ? A.w[w0 + q] : 0.0);
+        for (int q = tid; q < n * n_slots; q += kAdjThreads) {
+            const int wl = q / n_slots, slot = slot0 + q % n_slots;
+            const int wi = w0 + wl;
+            const bool in = wi < W && slot < A.n_sel;
+            double sn = 0.0, cs = 0.0;
+            if (in) {
+                const D4 xa = A.bub[(size_t)f * A.n_tot + A.sel[slot]];
+                sincos(A.w[wi] * (xa.t * ci - xa.z), &sn, &cs);
+            }
+#pragma unroll
+            for (int gs = 0; gs < S2; ++gs) {
+                double2 h = make_double2(0.0, 0.0);
+                if (in) {
+                    const double2 g = A.gbar[((size_t)f * S2 + gs) * W + wi];
+                    // conj(g) * (cs + i sn)
+                    h = make_double2(g.x * cs + g.y * sn, g.x * sn - g.y * cs);
+                }
+                const int rl = slot * S2 + gs - r0;
+                if (rl >= 0 && rl < kPqRows) Hs[wl * kPqRows + rl] = V2{(R)h.x, (R)h.y};
+            }
+        }
+    };
+    const bool held = w_held >= W;
+    if (held) form_h(0, n_stages * kPqW);
+    __syncthreads();
+    const int kt0 = s_kmin / kPqCols, n_kt = (A.n_t + kPqCols - 1) / kPqCols;
+    // stage q of the CTA: step tile kt0 + q / n_stages, frequencies 16 (q % n_stages) ..
+    V2 pre[kPqW * kPqCols / kAdjThreads];
+    auto fetch = [&](int q) {
+        const int kt = kt0 + q / n_stages, w0 = q % n_stages * kPqW;
+#pragma unroll
+        for (int e = 0; e < kPqW * kPqCols / kAdjThreads; ++e) {
+            const int at = tid + e * kAdjThreads, wi = w0 + at / kPqCols, k = kt * kPqCols + at % kPqCols;
+            pre[e] = (kt < n_kt && wi < W && k < A.n_t) ? mt[((size_t)i * W + wi) * A.n_t + k] : V2{R(0), R(0)};
+        }
+    };
     double P[4][4], Q[4][4];
+    if (kt0 < n_kt) fetch(0);
+    for (int q = 0; q < (n_kt - kt0) * n_stages; ++q) {
+        const int kt = kt0 + q / n_stages, st = q % n_stages;
+        V2* M = Ms + (q & 1) * kPqW * kPqCols;
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+        for (int e = 0; e < kPqW * kPqCols / kAdjThreads; ++e) M[tid + e * kAdjThreads] = pre[e];
+        if (!held) {
+            __syncthreads();  // every thread is done with the last stage's H
+            form_h(st * kPqW, kPqW);
+        }
+        __syncthreads();
+        fetch(q + 1);
+        if (st == 0) {
 #pragma unroll
-        for (int v = 0; v < 4; ++v) P[u][v] = Q[u][v] = 0.0;
-    for (int w0 = 0; w0 < W; w0 += kPqW) {
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) P[u][v] = Q[u][v] = 0.0;
+        }
         R Ps[4][4], Qs[4][4];  // this stage's sums
 #pragma unroll
         for (int u = 0; u < 4; ++u)
 #pragma unroll
             for (int v = 0; v < 4; ++v) Ps[u][v] = Qs[u][v] = R(0);
-        __syncthreads();
-        // H tile: row r = slot * S2 + gs
-        for (int q = tid; q < kPqW * kPqRows; q += blockDim.x) {
-            const int wl = q / kPqRows, rl = q % kPqRows;
-            const int wi = w0 + wl, r = r0 + rl;
-            double2 h = make_double2(0.0, 0.0);
-            if (wi < W && r < n_rows) {
-                const int slot = r / S2, gs = r % S2;
-                const D4 xa = A.bub[(size_t)f * A.n_tot + A.sel[slot]];
-                double sn, cs;
-                sincos(A.w[wi] * (xa.t * ci - xa.z), &sn, &cs);
-                const double2 g = A.gbar[((size_t)f * S2 + gs) * W + wi];
-                // conj(g) * (cs + i sn)
-                h = make_double2(g.x * cs + g.y * sn, g.x * sn - g.y * cs);
-            }
-            Hs[wl][rl] = V2{(R)h.x, (R)h.y};
-        }
-        for (int q = tid; q < kPqW * kPqCols; q += blockDim.x) {
-            const int wl = q / kPqCols, kl = q % kPqCols;
-            const int wi = w0 + wl, k = k0 + kl;
-            const double2 m = (wi < W && k < A.n_t) ? mt[((size_t)i * W + wi) * A.n_t + k] : make_double2(0.0, 0.0);
-            Ms[wl][kl] = V2{(R)m.x, (R)m.y};
-        }
-        if (tid < kPqW) ws[tid] = (R)(w0 + tid < W ? A.w[w0 + tid] : 0.0);
-        __syncthreads();
+        const V2* H = Hs + (held ? (size_t)st * kPqW * kPqRows : 0);
 #pragma unroll 4
         for (int wl = 0; wl < kPqW; ++wl) {
             V2 h[4], m[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) h[u] = Hs[wl][ty + 16 * u];
+            for (int u = 0; u < 4; ++u) h[u] = H[wl * kPqRows + ty + 16 * u];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) m[v] = Ms[wl][tx + 16 * v];
-            const R om = ws[wl];
+            for (int v = 0; v < 4; ++v) m[v] = M[wl * kPqCols + tx + 16 * v];
+            const R om = ws[(held ? st * kPqW : 0) + wl];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -198,22 +236,38 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_pq(AdjArgs A, const double2
                 P[u][v] += (double)Ps[u][v];
                 Q[u][v] += (double)Qs[u][v];
             }
-    }
+        if (st < n_stages - 1) continue;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int r = r0 + ty + 16 * u;
-        if (r >= n_rows) continue;
-        const int slot = r / S2, gs = r % S2;
-        const size_t row = ((size_t)f * A.n_sel + slot) * A.n_cos + i;
+        for (int u = 0; u < 4; ++u) {
+            const int r = r0 + ty + 16 * u;
+            if (r >= n_rows) continue;
+            const int slot = r / S2, gs = r % S2;
+            const size_t row = ((size_t)f * A.n_sel + slot) * A.n_cos + i;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int k = k0 + tx + 16 * v;
-            if (k >= A.n_t) continue;
-            const size_t o = (row * A.n_t + k) * S2 + gs;
-            A.s.bbar[o] = P[u][v];
-            A.s.imq[o] = Q[u][v];
+            for (int v = 0; v < 4; ++v) {
+                const int k = kt * kPqCols + tx + 16 * v;
+                if (k >= A.n_t) continue;
+                const size_t o = (row * A.n_t + k) * S2 + gs;
+                A.s.bbar[o] = P[u][v];
+                A.s.imq[o] = Q[u][v];
+            }
         }
     }
+}
+
+// The H tile of every frequency stays in shared memory while two CTAs fit an SM.
+template <int S, bool F32>
+static void launch_pq(const AdjArgs& A, size_t kn, cudaStream_t st, const void* mt) {
+    const size_t v2 = F32 ? sizeof(float2) : sizeof(double2);
+    const int W16 = (A.n_w + kPqW - 1) / kPqW * kPqW;
+    const size_t m_tiles = 2 * kPqW * kPqCols * v2, per_w = kPqRows * v2 + v2 / 2;
+    const int w_held = W16 * per_w + m_tiles <= 110 * 1024 ? W16 : kPqW;
+    const size_t smem = w_held * per_w + m_tiles;
+    const int row_tiles = (A.n_sel * 2 * S + kPqRows - 1) / kPqRows;
+    const dim3 g((unsigned)row_tiles, (unsigned)A.n_cos, (unsigned)kn);
+    CUDA_OK(cudaFuncSetAttribute(k_adj_pq<S, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_adj_pq<S, F32><<<g, kAdjThreads, smem, st>>>(A, mt, w_held);
+    CUDA_OK(cudaGetLastError());
 }
 
 // ---------------------------------------------------------------------------
@@ -695,15 +749,10 @@ template <int S, int SMC>
 static uint64_t launch_typed(const AdjArgs& A, size_t kn, cudaStream_t st, const double2* mt, const double* tt) {
     uint64_t launches = 0;
     {
-        const int row_tiles = (A.n_sel * 2 * S + kPqRows - 1) / kPqRows;
-        const int col_tiles = (A.n_t + kPqCols - 1) / kPqCols;
-        if ((long)row_tiles * col_tiles > 0x7fffffffL) throw Error{"adjoint grid too large"};
-        dim3 g((unsigned)(row_tiles * col_tiles), (unsigned)A.n_cos, (unsigned)kn);
         if (A.f32pq)
-            k_adj_pq<S, true><<<g, kAdjThreads, 0, st>>>(A, mt, row_tiles);
+            launch_pq<S, true>(A, kn, st, mt);
         else
-            k_adj_pq<S, false><<<g, kAdjThreads, 0, st>>>(A, mt, row_tiles);
-        CUDA_OK(cudaGetLastError());
+            launch_pq<S, false>(A, kn, st, mt);
         ++launches;
     }
     {
@@ -738,6 +787,12 @@ static uint64_t dispatch_m(const AdjArgs& A, size_t kn, cudaStream_t st, const d
     return launch_typed<S, S * M>(A, kn, st, mt, tt);
 }
 
+// The backward's precision follows the forward's kernel: FP32 products of depth kPqW for the
+// mixed kernels, FP64 otherwise.
+static bool adjoint_f32(const SpectrumJob& job) {
+    return job.kernel == BGWX_KERNEL_MIXED || job.kernel == BGWX_KERNEL_MIXED_SIMT;
+}
+
 uint64_t launch_adjoint_tables(Device* dev, const SpectrumJob& job, const D4* bub, const uint32_t* sel,
                                const double* cos_t, const double* t_arr, const double* w, const double* powers,
                                double2* mt, double* tt) {
@@ -747,8 +802,12 @@ uint64_t launch_adjoint_tables(Device* dev, const SpectrumJob& job, const D4* bu
             throw Error{"damping width too small for the adjoint (exp overflow)"};
     }
     const size_t n = job.n_cos * job.n_w * job.n_t;
-    k_adj_mtab<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(cos_t, t_arr, w, (int)job.n_cos,
-                                                                       (int)job.n_w, (int)job.n_t, mt);
+    const unsigned blocks = (unsigned)((n + 255) / 256);
+    if (adjoint_f32(job))
+        k_adj_mtab<<<blocks, 256, 0, dev->stream>>>(cos_t, t_arr, w, (int)job.n_cos, (int)job.n_w, (int)job.n_t,
+                                                    reinterpret_cast<float2*>(mt));
+    else
+        k_adj_mtab<<<blocks, 256, 0, dev->stream>>>(cos_t, t_arr, w, (int)job.n_cos, (int)job.n_w, (int)job.n_t, mt);
     CUDA_OK(cudaGetLastError());
     const size_t nt = job.n_sel * job.n_t;
     k_adj_ttab<<<(unsigned)((nt + 255) / 256), 256, 0, dev->stream>>>(
@@ -790,9 +849,7 @@ uint64_t launch_adjoint_chunk(Device* dev, const SpectrumJob& job, const D4* bub
     A.rot = rot;
     A.gbar = gbar;
     A.kn = (int)kn;
-    // the backward's precision follows the forward's kernel: FP32 products of depth kPqW for the
-    // mixed kernels, FP64 otherwise
-    A.f32pq = (job.kernel == BGWX_KERNEL_MIXED || job.kernel == BGWX_KERNEL_MIXED_SIMT) ? 1 : 0;
+    A.f32pq = adjoint_f32(job) ? 1 : 0;
     A.has_damp = job.has_damping ? 1 : 0;
     A.damp = job.damping;
     A.dphi = 2.0 * M_PI / (double)job.n_phi;
