@@ -274,7 +274,8 @@ static void launch_pq(const AdjArgs& A, size_t kn, cudaStream_t st, const void* 
 // Per (bubble, step) factors of the collided scaling, frame independent:
 // with r = tau/dt, a r^p D = a (tau^p e^{tau/w}) (dt^{-p} e^{-dt/w}), so the
 // patch factor tau^p e^{tau/w} is formed once per patch and the step factor
-// once per (bubble, step).  Row layout: dt^2, dt^3, ln dt, 1/dt, then
+// once per (bubble, step).  Layout [bubble][entry][step] (a warp of k_adj_rows reads
+// consecutive steps of one entry); entries: dt^2, dt^3, ln dt, 1/dt, then
 // dt^{-p_q} e^{-dt/w} for every (set, term) q; zeros where dt <= 0.
 __global__ void k_adj_ttab(const D4* __restrict__ bub, const uint32_t* __restrict__ sel, int n_sel,
                            const double* __restrict__ t_arr, int n_t, const double* __restrict__ powers, int SM,
@@ -283,14 +284,15 @@ __global__ void k_adj_ttab(const D4* __restrict__ bub, const uint32_t* __restric
     if (q >= (size_t)n_sel * n_t) return;
     const int slot = (int)(q / n_t), k = (int)(q % n_t);
     const double dtk = t_arr[k] - bub[sel[slot]].t;
-    double* row = tt + q * (4 + SM);
+    double* row = tt + (size_t)slot * (4 + SM) * n_t + k;  // entry m at row[m n_t]
     const bool on = dtk > 0.0;
+    const size_t nt = n_t;
     row[0] = on ? dtk * dtk : 0.0;
-    row[1] = on ? dtk * dtk * dtk : 0.0;
-    row[2] = on ? log(dtk) : 0.0;
-    row[3] = on ? 1.0 / dtk : 0.0;
+    row[nt] = on ? dtk * dtk * dtk : 0.0;
+    row[2 * nt] = on ? log(dtk) : 0.0;
+    row[3 * nt] = on ? 1.0 / dtk : 0.0;
     const double e = has_damp ? exp(-dtk / damp) : 1.0;
-    for (int m = 0; m < SM; ++m) row[4 + m] = on ? exp(-powers[m] * log(dtk)) * e : 0.0;
+    for (int m = 0; m < SM; ++m) row[(4 + m) * nt] = on ? exp(-powers[m] * log(dtk)) * e : 0.0;
 }
 
 // ---------------------------------------------------------------------------
@@ -311,11 +313,16 @@ __global__ void k_adj_ttab(const D4* __restrict__ bub, const uint32_t* __restric
 //   tbar_j  = sum_g x_jg sum_q a_q y_jq (p_q/tau_j + 1/w) B(kc_j)
 //   abar_q += sum_j sum_g x_jg y_jq B(kc_j)
 //   pbar_q += a_q sum_j sum_g x_jg y_jq (ln tau_j B(kc_j) - L(kc_j))
-// One warp per (frame, bubble, row) walks the steps in chunks of 32 from the
-// last (lane = step): a warp suffix scan of each component plus the carry of
-// the later chunks, the chunk's suffix sums to shared memory, and each patch
-// whose kc_j falls in the chunk reads its entry once.  Work per row is
-// O(n_t + n_phi) where the direct form is O(n_t n_phi).
+// One warp per (frame, bubble, row) walks the steps in chunks of 64 from the
+// last (a lane has two consecutive steps): a warp suffix scan of the pair sums
+// of each component plus the carry of the later chunks, the lanes' sums and
+// the odd steps' terms to shared memory, and each patch whose kc_j falls in
+// the chunk reads its entry once.  Work per row is O(n_t + n_phi) where the
+// direct form is O(n_t n_phi).  What bounds it is the shared-memory pipe, most
+// of it the scan's shuffles (5 x 2 per component and chunk).
+// 32 frames of 256 bubbles, 64 rows, 64 patches, 256 steps, one set of two
+// terms: 4.5 ms at 78% of that pipe; with one step a lane (twice the shuffles)
+// and the step factors of one step side by side (12 lines a load) 6.2 ms.
 constexpr int kRowWarps = 4;
 
 template <int SMC>
@@ -333,7 +340,8 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_adj_rows(AdjArgs A, const do
     extern __shared__ double rows_smem[];
     const unsigned full = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* sw = rows_smem + (size_t)warp * C * 32;  // [component][step in chunk]
+    double* sI = rows_smem + (size_t)warp * C * 65;  // [component][33]: suffix sum from step 2 l; [32]: the carry
+    double* sy = sI + C * 33;                        // [component][32]: the term of step 2 l + 1
     const long row = (long)blockIdx.x * kRowWarps + warp;
     const long R = (long)A.n_sel * A.n_cos;  // rows per frame
     const int f = (int)(row / R);
@@ -393,10 +401,10 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_adj_rows(AdjArgs A, const do
         }
     }
 
-    // sw[32 c] holds the suffix sum of component c from the start of the last chunk
+    // sI[33 c] holds the suffix sum of component c from the start of the last chunk
     // done (the carry into the next one): zero before the first
 #pragma unroll
-    for (int c = 0; c < C; ++c) sw[c * 32 + lane] = 0.0;
+    for (int c = 0; c < C; ++c) sI[c * 33 + lane] = 0.0;
     __syncwarp();
     double acc_t = 0.0, acc_z = 0.0, abar[SMC], pbar[SMC];
 #pragma unroll
@@ -404,49 +412,66 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_adj_rows(AdjArgs A, const do
 
     const size_t base = ((size_t)f * A.n_sel + slot) * A.n_cos + i;
     const double* trow = tt + (size_t)slot * n_t * TW;
-    for (int c0 = ((n_t - 1) >> 5) << 5; c0 >= (k0 & ~31); c0 -= 32) {
-        const int k = c0 + lane;
+    for (int c0 = ((n_t - 1) >> 6) << 6; c0 >= (k0 & ~63); c0 -= 64) {
         double y[C];
 #pragma unroll
-        for (int c = 0; c < C; ++c) y[c] = 0.0;
-        if (k >= k0 && k < n_t) {
-            const double* tk = trow + (size_t)k * TW;
-            const double d2 = tk[0], d3 = tk[1], ld = tk[2], invd = tk[3];
-            const double uk = (k == 0 || k == n_t - 1) ? 0.5 : 1.0;
-            const double pre = rowc * uk * A.cutw[k];
-            const double pd3 = pre * d3;
-            const size_t o = (base * n_t + k) * S2;
-            double bb[S2], iq[S2];
+        for (int h = 1; h >= 0; --h) {
+            const int k = c0 + 2 * lane + h;
+            double v[C];
 #pragma unroll
-            for (int g = 0; g < S2; ++g) {
-                bb[g] = A.s.bbar[o + g];
-                iq[g] = A.s.imq[o + g];
+            for (int c = 0; c < C; ++c) v[c] = 0.0;
+            if (k >= k0 && k < n_t) {
+                const double* tk = trow + k;
+                const double d2 = tk[0], d3 = tk[n_t], ld = tk[2 * (size_t)n_t], invd = tk[3 * (size_t)n_t];
+                const double uk = (k == 0 || k == n_t - 1) ? 0.5 : 1.0;
+                const double pre = rowc * uk * A.cutw[k];
+                const double pd3 = pre * d3;
+                const double2* bp = reinterpret_cast<const double2*>(A.s.bbar + (base * n_t + k) * S2);
+                const double2* ip = reinterpret_cast<const double2*>(A.s.imq + (base * n_t + k) * S2);
+                double bb[S2], iq[S2];
+#pragma unroll
+                for (int g = 0; g < S; ++g) {
+                    const double2 b2 = bp[g], i2 = ip[g];
+                    bb[2 * g] = b2.x;
+                    bb[2 * g + 1] = b2.y;
+                    iq[2 * g] = i2.x;
+                    iq[2 * g + 1] = i2.y;
+                }
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    double sb = 0.0, si = 0.0;
+#pragma unroll
+                    for (int s = 0; s < S; ++s) {
+                        sb += bb[g * S + s];
+                        si += iq[g * S + s];
+                    }
+                    v[oV + g] = pd3 * si;
+                    v[oU + g] = 3.0 * pre * d2 * sb + ci * v[oV + g];
+#pragma unroll
+                    for (int q = 0; q < SMC; ++q) {
+                        const int s = q / M;
+                        const double be = tk[(size_t)(4 + q) * n_t];
+                        const double c1 = -p_c[q] * invd - invw;
+                        const double zq = pd3 * iq[g * S + s] * be;
+                        const double bq = pd3 * bb[g * S + s] * be;
+                        v[oZ + g * SMC + q] = zq;
+                        v[oB + g * SMC + q] = bq;
+                        v[oL + g * SMC + q] = bq * ld;
+                        v[oT + g * SMC + q] = pre * bb[g * S + s] * be * (3.0 * d2 + d3 * c1) + ci * zq;
+                    }
+                }
             }
 #pragma unroll
-            for (int g = 0; g < 2; ++g) {
-                double sb = 0.0, si = 0.0;
-#pragma unroll
-                for (int s = 0; s < S; ++s) {
-                    sb += bb[g * S + s];
-                    si += iq[g * S + s];
-                }
-                y[oV + g] = pd3 * si;
-                y[oU + g] = 3.0 * pre * d2 * sb + ci * y[oV + g];
-#pragma unroll
-                for (int q = 0; q < SMC; ++q) {
-                    const int s = q / M;
-                    const double be = tk[4 + q];
-                    const double c1 = -p_c[q] * invd - invw;
-                    const double zq = pd3 * iq[g * S + s] * be;
-                    const double bq = pd3 * bb[g * S + s] * be;
-                    y[oZ + g * SMC + q] = zq;
-                    y[oB + g * SMC + q] = bq;
-                    y[oL + g * SMC + q] = bq * ld;
-                    y[oT + g * SMC + q] = pre * bb[g * S + s] * be * (3.0 * d2 + d3 * c1) + ci * zq;
+            for (int c = 0; c < C; ++c) {
+                if (h == 1) {
+                    sy[c * 32 + lane] = v[c];
+                    y[c] = v[c];
+                } else {
+                    y[c] += v[c];
                 }
             }
         }
-        // inclusive suffix sums within the chunk, then the later chunks' total
+        // inclusive suffix sums of the pairs within the chunk, then the later chunks' total
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
 #pragma unroll
@@ -456,22 +481,31 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_adj_rows(AdjArgs A, const do
             }
         }
 #pragma unroll
-        for (int c = 0; c < C; ++c) y[c] += sw[c * 32];
+        for (int c = 0; c < C; ++c) {
+            const double carry = sI[c * 33];
+            y[c] += carry;
+            if (lane == 0) sI[c * 33 + 32] = carry;
+        }
         __syncwarp();
 #pragma unroll
-        for (int c = 0; c < C; ++c) sw[c * 32 + lane] = y[c];
+        for (int c = 0; c < C; ++c) sI[c * 33 + lane] = y[c];
         __syncwarp();
 #pragma unroll
         for (int jj = 0; jj < JPL; ++jj) {
             const int kj = kc[jj];
-            if (kj < c0 || kj >= c0 + 32 || kj >= n_t) continue;
-            const double* e = sw + (kj - c0);  // component c at e[32 c]
+            if (kj < c0 || kj >= c0 + 64 || kj >= n_t) continue;
+            const int l = (kj - c0) >> 1, odd = kj & 1;
+            // suffix sum of component c from step kj
+            auto e = [&](int c) {
+                const double from = sI[c * 33 + l + odd];
+                return odd ? sy[c * 32 + l] + from : from;
+            };
             const int j = lane + 32 * jj;
             const double wj = (j == 0 || j == A.n_phi - 1) ? 0.5 : 1.0;
             const double x0 = wj * A.cos2[j], x1 = wj * A.sin2[j];
             // the uncollided steps k < kc_j: the totals U(0) and V(0) are added after the loop
-            acc_t += x0 * e[32 * oU] + x1 * e[32 * (oU + 1)];
-            acc_z -= x0 * e[32 * oV] + x1 * e[32 * (oV + 1)];
+            acc_t += x0 * e(oU) + x1 * e(oU + 1);
+            acc_z -= x0 * e(oV) + x1 * e(oV + 1);
             const double tj = tau_j[jj];
             const double lt = log(tj);
             const double et = A.has_damp ? exp(tj * invw) : 1.0;
@@ -480,10 +514,10 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_adj_rows(AdjArgs A, const do
             for (int q = 0; q < SMC; ++q) {
                 const double yq = exp(p_c[q] * lt) * et;
                 const double c2 = p_c[q] / tj + invw;
-                const double Tx = x0 * e[32 * (oT + q)] + x1 * e[32 * (oT + SMC + q)];
-                const double Zx = x0 * e[32 * (oZ + q)] + x1 * e[32 * (oZ + SMC + q)];
-                const double Bx = x0 * e[32 * (oB + q)] + x1 * e[32 * (oB + SMC + q)];
-                const double Lx = x0 * e[32 * (oL + q)] + x1 * e[32 * (oL + SMC + q)];
+                const double Tx = x0 * e(oT + q) + x1 * e(oT + SMC + q);
+                const double Zx = x0 * e(oZ + q) + x1 * e(oZ + SMC + q);
+                const double Bx = x0 * e(oB + q) + x1 * e(oB + SMC + q);
+                const double Lx = x0 * e(oL + q) + x1 * e(oL + SMC + q);
                 const double ay = a_c[q] * yq;
                 acc_t -= ay * Tx;
                 acc_z += ay * Zx;
@@ -496,8 +530,8 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_adj_rows(AdjArgs A, const do
         __syncwarp();
     }
     // every patch's uncollided part starts from the totals U(0), V(0)
-    acc_t -= xs0 * sw[32 * oU] + xs1 * sw[32 * (oU + 1)];
-    acc_z += xs0 * sw[32 * oV] + xs1 * sw[32 * (oV + 1)];
+    acc_t -= xs0 * sI[33 * oU] + xs1 * sI[33 * (oU + 1)];
+    acc_z += xs0 * sI[33 * oV] + xs1 * sI[33 * (oV + 1)];
 #pragma unroll
     for (int jj = 0; jj < JPL; ++jj) {
         const int j = lane + 32 * jj;
@@ -740,8 +774,8 @@ __global__ void k_adj_params(AdjArgs A, long n_rows) {
 // ---------------------------------------------------------------------------
 template <int S, int SMC, int JPL>
 static void launch_rows(const AdjArgs& A, long rows, cudaStream_t st, const double* tt) {
-    const size_t smem = (size_t)kRowWarps * row_components<SMC>() * 32 * sizeof(double);
-    static_assert(kRowWarps * row_components<4>() * 32 * sizeof(double) <= 48 * 1024, "row kernel shared memory");
+    const size_t smem = (size_t)kRowWarps * row_components<SMC>() * 65 * sizeof(double);
+    CUDA_OK(cudaFuncSetAttribute(k_adj_rows<S, SMC, JPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_adj_rows<S, SMC, JPL><<<(unsigned)((rows + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, smem, st>>>(A, tt);
 }
 
