@@ -16,20 +16,20 @@
 //   f = sum_m a_m (tau_j / dt)^{p_m} exp(-(dt - tau_j) / width)   (collided),
 //   dt^3 sum_j q_j f_j = dt^3 U(k) + sum_m a_m dt^{3-p_m} e^{-dt/width} Pm(k),
 // where U(k) sums q_j over the patches not yet collided at step k and Pm(k)
-// sums q_j tau_j^{p_m} e^{tau_j/width} over those already collided.  k_events
-// sorts each row's collided patches by the first time step at which the
-// reference's test (t_k - t_a) >= tau_j holds (exact FP64 comparisons), in
-// buckets of kKC steps, and stores U at every bucket boundary as a backward
-// sum of the remaining terms (forming it as total minus collided cancels
-// catastrophically once most patches have collided); the GEMM kernel turns
-// running prefix sums into beta tile by tile.
+// sums q_j tau_j^{p_m} e^{tau_j/width} over those already collided.  k_beta adds
+// each collided patch to the first time step at which the reference's test
+// (t_k - t_a) >= tau_j holds (exact FP64 comparisons) and forms Pm as running
+// sums and U as backward sums of the remaining terms (total minus collided
+// cancels catastrophically once most patches have collided).
 //
 // Kernels:
 //   k_time_tables   per bubble and t: dt^3 and dt^{3-p} e^{-dt/width}
-//   k_events        per (frame, bubble, row): bucketed, stably sorted events
-//   k_spec_factored per (w tile, column tile): loop over rows i, GEMM over t
-//                   in chunks of kKC with beta produced in shared memory,
-//                   FP64 epilogue; Real = double (FP64) or float (mixed)
+//   k_beta          per (frame, bubble, row): beta, as FP64 or FP32 values or as
+//                   int8 digits with one scale per row (k_beta_sorted: the
+//                   digits of calls whose masks the adjoint reads again)
+//   k_gemm_fold     FP64 product over t, folded about the middle of the time grid
+//   k_gemm          FP32 product over t in chunks of kKC, FP64 epilogue
+//                   (spectrum_tc.cu: the int8 digits' tensor-core product)
 //   k_reduce_tiles  deterministic sum of the column-tile partials per frame
 
 #include <cuda_runtime.h>
@@ -58,7 +58,14 @@ constexpr int kThreads = 256;
 constexpr int kTM = 8;           // register tile rows per thread (columns: TN = 8 FP32, 4 FP64)
 
 // ---------------------------------------------------------------------------
-// Step factors of a bubble, table row q over steps at ((slot (1 + SM) + q) tf + k): row 0 the step weight
+// Place of step k in a row of the step factors and of k_beta's bins: within each block of 32 steps the first
+// two of every four steps come first, so that lanes with four steps each read them as two 16-byte words
+// without a bank conflict (or half a line) between them.
+__host__ __device__ __forceinline__ int step_at(int k) {
+    return (k & ~31) | ((k & 2) << 3) | ((k >> 1) & 14) | (k & 1);
+}
+
+// Step factors of a bubble, table row q over steps at ((slot (1 + SM) + q) tf + step_at(k)): row 0 the step weight
 // (time cutoff x trapezoid end weight) times dt^3, row 1 + q the same times a_q dt^{3-p_q} e^{-dt/width};
 // zero where dt <= 0 and past n_t (tf is n_t rounded up to whole blocks of 32 steps).
 __global__ void k_time_tables(const D4* __restrict__ bub, const uint32_t* __restrict__ sel, int n_sel,
@@ -70,7 +77,7 @@ __global__ void k_time_tables(const D4* __restrict__ bub, const uint32_t* __rest
     if (slot >= n_sel || k >= tf || sel[slot] == kNoSlot) return;
     const double ta = bub[sel[slot]].t;
     const double dt = k < n_t ? t_arr[k] - ta : 0.0;
-    double* row = D + (size_t)slot * (1 + SM) * tf + k;
+    double* row = D + (size_t)slot * (1 + SM) * tf + step_at(k);
     const bool on = dt > 0.0;
     const double wk = k < n_t ? cutw[k] * ((k == 0 || k == n_t - 1) ? 0.5 : 1.0) : 0.0;
     const double d3 = on ? dt * (dt * dt) : 0.0;
@@ -85,7 +92,7 @@ __global__ void k_time_tables(const D4* __restrict__ bub, const uint32_t* __rest
 }
 
 // Per (bubble, block of 32 steps): the least and the largest D_q(k) of each
-// table row over the block's steps (one warp, lane = step), stored as (min, max)
+// table row over the block's steps (one warp, a lane each), stored as (min, max)
 // pairs.
 __global__ void k_time_maxima(const double* __restrict__ D, int n_sel, int tf, int nblk, int Q,
                               double* __restrict__ Dmax) {
@@ -123,10 +130,14 @@ __global__ void k_time_maxima(const double* __restrict__ D, int n_sel, int tf, i
 // beta(k) = rf_i u_k cut_k [dt^3 U(k) + sum_m a_m dt^{3-p_m} e^{-dt/w} Pm(k)]
 // is written to beta[frame][i][col][k], col = slot*2S + 2s + g.
 //
-// What bounds it: issue.  Sorting the events into blocks and again into steps,
+// What bounds it: issue and shared memory.  Sorting the events into blocks and again into steps,
 // with totals and scans over every block, took two thirds of 62.8 ms for 8
 // frames of 4096 bubbles x 192 rows; the digits and stores of the quiet steps a
-// quarter.
+// quarter.  Now 39.8 ms there (the 51 GB of digits and 10 GB of delays alone:
+// 9.3 ms at the measured copy rate), and 1.42 ms in FP64 for 4 frames of 512
+// bubbles x 128 rows x 512 steps (2.19).  Issue and the shared-memory pipe are
+// each 62 % busy; with the steps of a block in order (two-way bank conflicts)
+// and the delays' two steps read one after the other it took 47 ms.
 struct BetaArgs {
     const double* tau;     // (kn, n_sel, n_cos*n_phi)
     const D4* bub;         // bubbles (frame 0; times are frame independent)
@@ -203,24 +214,35 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
     const double ta = A.bub[A.sel[slot]].t;
     const double inv_dt = 1.0 / A.dt;  // the estimate below is only a starting point
     constexpr int kNever = 0x7fffffff;
-    auto step_of = [&](double tj) -> int {
-        if (!(tj > 0.0)) return kNever;
-        // first k with (t_k - t_a) >= tau_j: arithmetic estimate, then exact
-        // comparisons (the predicate is monotone in k) settle the boundary
+    // first k with (t_k - t_a) >= tau_j: arithmetic estimate, then exact comparisons (the predicate is
+    // monotone in k) settle the boundary; the two steps they read first are loaded ahead
+    auto guess = [&](double tj) -> int {
         const double est = ceil((ta + tj - A.t_arr[0]) * inv_dt);
-        int lo = est < 0.0 ? 0 : (est > (double)A.n_t ? A.n_t : (int)est);
-        while (lo > 0 && A.t_arr[lo - 1] - ta >= tj) --lo;
-        while (lo < A.n_t && !(A.t_arr[lo] - ta >= tj)) ++lo;
+        return est < 0.0 ? 0 : (est > (double)A.n_t ? A.n_t : (int)est);
+    };
+    auto settle = [&](double tj, int lo, double below, double here) -> int {
+        if (!(tj > 0.0)) return kNever;
+        if ((lo > 0 && below - ta >= tj) || (lo < A.n_t && !(here - ta >= tj))) {
+            while (lo > 0 && A.t_arr[lo - 1] - ta >= tj) --lo;
+            while (lo < A.n_t && !(A.t_arr[lo] - ta >= tj)) ++lo;
+        }
         return lo < A.n_t ? lo : kNever;
     };
     int k_lo = kNever, k_hi = -1;
     const int n_own = max(0, min(c_pat, A.n_phi - lane * c_pat));  // this lane's patches
     const int own = lane * pitch;
-    for (int m = 0; m < n_own; ++m) {
-        const int kj = step_of(s_tau[own + m]);
+    for (int m = 0; m < n_own; m += 2) {  // two patches' loads in flight
+        const bool two = m + 1 < n_own;
+        const double tj = s_tau[own + m], tj2 = two ? s_tau[own + m + 1] : 0.0;
+        const int lo = guess(tj), lo2 = guess(tj2);
+        const double below = __ldg(A.t_arr + max(lo - 1, 0)), here = __ldg(A.t_arr + min(lo, A.n_t - 1));
+        const double below2 = __ldg(A.t_arr + max(lo2 - 1, 0)), here2 = __ldg(A.t_arr + min(lo2, A.n_t - 1));
+        const int kj = settle(tj, lo, below, here), kj2 = settle(tj2, lo2, below2, here2);
         s_kj[own + m] = kj;
-        k_lo = min(k_lo, kj);
+        if (two) s_kj[own + m + 1] = kj2;
+        k_lo = min(k_lo, min(kj, kj2));
         if (kj != kNever) k_hi = max(k_hi, kj);
+        if (kj2 != kNever) k_hi = max(k_hi, kj2);
     }
     k_lo = __reduce_min_sync(full, k_lo);
     k_hi = __reduce_max_sync(full, k_hi);
@@ -248,6 +270,14 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
         if (lane < 4 + 2 * SMC) s_const[lane] = lane == 0 ? u0 : lane == 1 ? u1 : 0.0;
         __syncwarp();
     }
+    const int at4 = step_at(4 * lane);  // the lane's four steps of a segment: at4, at4 + 1, at4 + 16, at4 + 17
+    auto four = [&](const double* p, double (&v)[4]) {
+        const double2 lo = reinterpret_cast<const double2*>(p + at4)[0], hi = reinterpret_cast<const double2*>(p + at4)[8];
+        v[0] = lo.x;
+        v[1] = lo.y;
+        v[2] = hi.x;
+        v[3] = hi.y;
+    };
     // The running sums of segment g into bins w: rows 0, 1 the uncollided sums U after each step, the
     // others the collided sums Pm up to it (lane: steps 4 lane .. 4 lane + 3).
     auto form = [&](int g, double* w) {
@@ -269,7 +299,7 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
                 const int rounds = __reduce_max_sync(full, rank);
                 for (int r = 0; r <= rounds; ++r) {
                     if (rank == r) {
-                        double* e = w + (k_run - s0);
+                        double* e = w + step_at(k_run - s0);
 #pragma unroll
                         for (int q = 0; q < NQ; ++q) e[q * kSeg] += run[q];
                     }
@@ -313,8 +343,8 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
             for (int q = 0; q < NQ; ++q) base[q] += __shfl_xor_sync(full, base[q], o);
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
-            double2* e = reinterpret_cast<double2*>(w + q * kSeg + 4 * lane);
-            const double2 lo = e[0], hi = e[1];
+            double2* e = reinterpret_cast<double2*>(w + q * kSeg + at4);
+            const double2 lo = e[0], hi = e[8];
             if (q < 2) {  // the sum of the later steps' events
                 const double v2 = hi.y, v1 = hi.x + v2, v0 = lo.y + v1;
                 double run = lo.x + v0;
@@ -327,7 +357,7 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
                 if (lane == 31) later = 0.0;
                 later += base[q];
                 e[0] = make_double2(v0 + later, v1 + later);
-                e[1] = make_double2(v2 + later, later);
+                e[8] = make_double2(v2 + later, later);
                 if (g == 0 && lane == 0) s_const[q] = run + base[q];
                 if (g == n_seg - 1 && lane == 0) s_const[2 + q] = base[q];
             } else {  // this step's and the earlier ones'
@@ -342,7 +372,7 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
                 if (lane == 0) before = 0.0;
                 before += base[q];
                 e[0] = make_double2(v0 + before, v1 + before);
-                e[1] = make_double2(v2 + before, v3 + before);
+                e[8] = make_double2(v2 + before, v3 + before);
                 if (g == n_seg - 1 && lane == 31) s_const[2 + q] = run + base[q];
             }
         }
@@ -350,8 +380,8 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
     };
     // table row q at the lane's four steps of the blocks from b on
     auto factors = [&](int q, int b, double (&v)[4]) {
-        const double2* d = reinterpret_cast<const double2*>(Dslot + (size_t)q * A.tf + (b << 5) + 4 * lane);
-        const double2 lo = __ldg(d), hi = __ldg(d + 1);
+        const double2* d = reinterpret_cast<const double2*>(Dslot + (size_t)q * A.tf + (b << 5) + at4);
+        const double2 lo = __ldg(d), hi = __ldg(d + 8);
         v[0] = lo.x;
         v[1] = lo.y;
         v[2] = hi.x;
@@ -361,22 +391,26 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
     auto seg_values = [&](int g, const double* w, int s, double (&xc)[4], double (&xs)[4]) {
         const int b = b_ev + g * kSegBlocks;
         const bool on = b + (lane >> 3) < NB;
-        double d[4] = {0.0, 0.0, 0.0, 0.0};
+        double d[4] = {0.0, 0.0, 0.0, 0.0}, c[4], e[4];
         if (on) factors(0, b, d);
+        four(w, c);
+        four(w + kSeg, e);
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-            xc[m] = d[m] * w[4 * lane + m];
-            xs[m] = d[m] * w[kSeg + 4 * lane + m];
+            xc[m] = d[m] * c[m];
+            xs[m] = d[m] * e[m];
         }
         const int t0 = s * A.M, t1 = t0 + A.M;
 #pragma unroll
         for (int t = 0; t < SMC; ++t) {
             if (SMC > 1 && (t < t0 || t >= t1)) continue;
             if (on) factors(1 + t, b, d);
+            four(w + (2 + 2 * t) * kSeg, c);
+            four(w + (3 + 2 * t) * kSeg, e);
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                xc[m] = fma(d[m], w[(2 + 2 * t) * kSeg + 4 * lane + m], xc[m]);
-                xs[m] = fma(d[m], w[(3 + 2 * t) * kSeg + 4 * lane + m], xs[m]);
+                xc[m] = fma(d[m], c[m], xc[m]);
+                xs[m] = fma(d[m], e[m], xs[m]);
             }
         }
 #pragma unroll
@@ -470,7 +504,7 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
                         {
                             const int b = bc + bi;
                             const bool aft = b >= b_aft;
-                            const double* d = Dslot + (b << 5) + lane;
+                            const double* d = Dslot + (b << 5) + lane;  // the block's steps in any order
                             const double d0 = d[0];
                             double m = 0.0;
                             for (int s2 = 0; s2 < A.S; ++s2) {
@@ -549,15 +583,15 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
             if (!kept) form(g, w);
             for (int s = 0; s < A.S; ++s) {
                 double xc[4], xs[4];
-                double2* e = reinterpret_cast<double2*>(w + (2 + 2 * s * A.M) * kSeg + 4 * lane);
+                double2* e = reinterpret_cast<double2*>(w + (2 + 2 * s * A.M) * kSeg + at4);
                 double2* f = e + kSeg / 2;
                 if (kept) {
 #pragma unroll
                     for (int m = 0; m < 2; ++m) {
-                        xc[2 * m] = e[m].x;
-                        xc[2 * m + 1] = e[m].y;
-                        xs[2 * m] = f[m].x;
-                        xs[2 * m + 1] = f[m].y;
+                        xc[2 * m] = e[8 * m].x;
+                        xc[2 * m + 1] = e[8 * m].y;
+                        xs[2 * m] = f[8 * m].x;
+                        xs[2 * m + 1] = f[8 * m].y;
                     }
                 } else {
                     seg_values(g, w, s, xc, xs);
@@ -567,8 +601,8 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
                     for (int m = 0; m < 4; ++m) vmax = fmax(vmax, fmax(fabs(xc[m]), fabs(xs[m])));
 #pragma unroll
                     for (int m = 0; m < 2; ++m) {
-                        e[m] = make_double2(xc[2 * m], xc[2 * m + 1]);
-                        f[m] = make_double2(xs[2 * m], xs[2 * m + 1]);
+                        e[8 * m] = make_double2(xc[2 * m], xc[2 * m + 1]);
+                        f[8 * m] = make_double2(xs[2 * m], xs[2 * m + 1]);
                     }
                 } else {
                     uint32_t pc[4], ps[4];
@@ -952,7 +986,7 @@ __global__ void __launch_bounds__(256, 3) k_beta_sorted(BetaArgs A, int8_t* __re
     auto value = [&](int k, int s, const double* P, double Uc, double Us, double mul, double& xc, double& xs) {
         double g[1 + SMC];
 #pragma unroll
-        for (int q = 0; q < 1 + SMC; ++q) g[q] = __ldg(Dslot + (size_t)q * A.tf + min(k, A.n_t - 1));
+        for (int q = 0; q < 1 + SMC; ++q) g[q] = __ldg(Dslot + (size_t)q * A.tf + step_at(min(k, A.n_t - 1)));
         double vc = g[0] * Uc, vs = g[0] * Us;
         const int t0 = s * A.M, t1 = t0 + A.M;  // the terms of set s
 #pragma unroll
@@ -1234,7 +1268,7 @@ __global__ void __launch_bounds__(256, 3) k_beta_sorted(BetaArgs A, int8_t* __re
 #pragma unroll
             for (int q = 0; q < 2 * SMC; ++q) P[q] = rinv * pbeg[(size_t)b * 2 * SMC + q];
             const double Uc = rinv * uend[2 * b], Us = rinv * uend[2 * b + 1];
-            const double* Db = Dslot + k0;
+            const double* Db = Dslot + step_at(k0);
             int8_t* blk = blk_row + (size_t)b * kI8BlockSet;
             for (int s2 = 0; s2 < A.S; ++s2) {
                 uint32_t pc[4], ps[4];
@@ -1247,7 +1281,7 @@ __global__ void __launch_bounds__(256, 3) k_beta_sorted(BetaArgs A, int8_t* __re
                     } else {
                         double g[1 + SMC];
 #pragma unroll
-                        for (int q = 0; q < 1 + SMC; ++q) g[q] = __ldg(Db + (size_t)q * A.tf + m);
+                        for (int q = 0; q < 1 + SMC; ++q) g[q] = __ldg(Db + (size_t)q * A.tf + (m & 1) + 8 * (m & 2));
                         xc = g[0] * Uc;
                         xs = g[0] * Us;
 #pragma unroll
@@ -1535,7 +1569,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
 // the middle phase goes into the epilogue's.  What bounds it: FP64 FMAs (half of the plain form's; 9.2 ms
 // before, of which 4.1 at the FP64 peak, for 4 frames of 512 bubbles x 128 rows x 512 steps x 128 w).  The
 // rows are split over CTAs, 8 rows each at least: a small call had 16 CTAs (1.7 ms for 8 frames of 48
-// bubbles).  The split depends on the grid alone, so that a realization's sums do not depend on its batch.
+// bubbles).  Now 5.05 ms for the former.  The split depends on the grid alone, so that a realization's sums do not depend on its batch.
 constexpr int kFoldTN = 4, kFoldCols = 16 * kFoldTN, kFoldBS = kFoldCols + 2;
 
 struct FoldSmem {  // doubles
