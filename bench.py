@@ -385,7 +385,7 @@ def run_b200(args):
             work = "2 x (2 n_w) x n_t x columns x n_cos flops per frame"
         else:
             achieved = counted
-            kname = "k_spec_direct + k_reduce"
+            kname = "k_direct_b + k_direct_a"
             work = "counted F = 6 PTE + 8 Phi + 20 Phi_t per step"
         roofline = {"bound": bound, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                     "frac": (achieved / peak) if achieved else None,

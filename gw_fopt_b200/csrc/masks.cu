@@ -44,9 +44,9 @@
 // directions the pass runs over the whole list.  What is still open (a near-lightlike first
 // collider, an unlisted first collider, one of the conditions above broken) takes steps 1-3 in a second kernel.
 // What bounds it: issue (77 % of the slots); per direction about 9 instructions per entry and 100 more,
-// per list about 400.  8 frames of 4096 bubbles x 192 x 192 directions: 11.3 ms (40.4 ms with a walk down
+// per list about 400.  8 frames of 4096 bubbles x 192 x 192 directions: 13.7 ms (40.4 ms with a walk down
 // the rows, each direction's candidate verified in FP64 against every entry with a smaller key); 32 frames
-// of 256 bubbles x 64 x 64: 0.64 ms (2.26).
+// of 256 bubbles x 64 x 64: 0.73 ms (2.26).
 //
 // Whenever a bound reaches past the list (or the list has no candidate and is
 // not complete) the direction falls back to the exhaustive scan over all
@@ -221,7 +221,7 @@ __device__ __forceinline__ void collider_bounds(const D4& d, double& key, double
 // shared memory (up to n_cache of them; the others are formed again) for the three passes of the radix
 // select, and the rho bounds and outliers are taken on the way.  Reading them in every pass, and one thread
 // walking the 2048 bins, took 1.9 ms for 4096 bubbles among 28672 (L2 bandwidth) and 168 us for 256 among
-// 1792 (the walk).
+// 1792 (the walk); now 1.25 ms there.
 template <int NT>
 __global__ void __launch_bounds__(NT)
     k_neighbors(const D4* __restrict__ bub, size_t n_int, size_t n_tot, const uint32_t* __restrict__ sel,

@@ -2,7 +2,7 @@
 //
 // Stages, per chunk of k-hat frames:
 //   k_rotate       bubbles (t, x, y, z) rotated by R(k)            [optional]
-//   k_neighbors, k_masks_list (masks.cu)
+//   k_neighbors, k_masks_list, k_masks_rest (masks.cu)
 //                  exact first-collider search per (k, bubble, patch)
 //   spectrum_direct.cu    plain FP64 spectrum, tensor and integrand
 //   spectrum_factored.cu  FP64 and mixed factored spectrum (spectrum_tc.cu: its tensor-core GEMM)

@@ -22,8 +22,8 @@
 // What bounds it: FP64 issue in k_direct_a (about 14 operations and 4 per column for each phase);
 // k_direct_b is a few per cent.  The single kernel this replaces (one block per bubble, pow() for
 // every patch and step, a barrier per step) took 53.6 ms for 5 bubbles x 50 x 100 patches x 800 steps
-// x 120 w and 38.2 ms for 4 frames of 64 bubbles x 64 x 64 x 256 x 64 w with 3 sets; see the
-// measured lines at the launches below.
+// x 120 w and 38.2 ms for 4 frames of 64 bubbles x 64 x 64 x 256 x 64 w with 3 sets; these two take
+// 0.1 ms and 1.04 ms (k_direct_b 0.27, k_direct_a 0.76: FP64 pipe half busy, 0.34 ms of FP64 work).
 
 #include <cuda_runtime.h>
 
