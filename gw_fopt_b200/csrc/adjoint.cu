@@ -27,11 +27,11 @@
 //   k_adj_pq      per (frame, row): Re P and Im Q as two real products of depth W
 //   k_adj_rows    one warp per (frame, bubble, row): the patch sums above in event form (suffix
 //                 sums over the steps read at each patch's collision step), dL/dtau per patch
-//   k_adj_bubble  per (frame, bubble): the row partials of t_a and z_a
+//   k_adj_bubble  per (frame, bubble): the row partials of t_a, z_a and the parameters
 //   k_adj_geom    per (frame, bubble, patch): dL/dtau -> both bubbles of the collision, and the
 //                 bubble parts above, summed as fixed-point integers (deterministic; two passes:
 //                 exponent bound, then sums) and added to the gradients by k_adj_fixout
-//   k_adj_params  per parameter: fixed-order sum of the row partials
+//   k_adj_params  per parameter: fixed-order sum over the bubbles
 
 #include <cuda_runtime.h>
 
@@ -670,21 +670,29 @@ __device__ __forceinline__ void warp_runs_add(long long* gfix, long key, const l
 __global__ void k_adj_gexp_init(int* gexp) { *gexp = -2000; }
 
 // PASS 0: the exponent bound of the chunk's contributions; PASS 1: their fixed-point sums.
+// A warp takes 32 kGeomItems consecutive items, mostly one bubble's: its own sums stay in the lanes until the
+// bubble changes.  What bounds it: the atomics of the colliders' parts in pass 1, the loads' latency in pass 0.
+// 32 frames of 256 bubbles x 64 x 64: 0.32 and 1.36 ms (0.80 and 1.43 with an item a thread).
+constexpr int kGeomItems = 8;
+
 template <int PASS>
-__global__ void k_adj_geom(AdjArgs A) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_adj_geom(AdjArgs A) {
     const int f = blockIdx.y;
+    const size_t q0 = ((size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * kGeomItems + (threadIdx.x & 31);
     long ka, kb;
     double g[4];
-    geom_item(A, f, q, ka, kb, g);
     if constexpr (PASS == 0) {
         int e = -2000;
+#pragma unroll 4
+        for (int it = 0; it < kGeomItems; ++it) {
+            geom_item(A, f, q0 + 32 * it, ka, kb, g);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            int ex;
-            if (g[c] != 0.0 && isfinite(g[c])) {
-                frexp(g[c], &ex);  // |g| < 2^ex
-                e = max(e, ex);
+            for (int c = 0; c < 4; ++c) {
+                int ex;
+                if (g[c] != 0.0 && isfinite(g[c])) {
+                    frexp(g[c], &ex);  // |g| < 2^ex
+                    e = max(e, ex);
+                }
             }
         }
 #pragma unroll
@@ -692,34 +700,45 @@ __global__ void k_adj_geom(AdjArgs A) {
         if ((threadIdx.x & 31) == 0 && e > -2000) atomicMax(A.s.gexp, e);
     } else {
         const int sh = 61 - *A.s.gexp;
-        long long h[4], l[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            long long X = 0;
-            if (isfinite(g[c])) {
-                X = __double2ll_rn(ldexp(g[c], sh));
-            } else if (kb >= 0 || ka >= 0) {
-                // a non-finite gradient is passed on as it is
-                if (kb >= 0) atomicAdd(A.g_bub + 4 * kb + c, g[c]);
-                if (ka >= 0 && kb >= 0) atomicAdd(A.g_bub + 4 * ka + c, -g[c]);
-                else if (ka >= 0) atomicAdd(A.g_bub + 4 * ka + c, g[c]);
-            }
-            h[c] = X >> 31;
-            l[c] = X & 0x7fffffffLL;
-        }
-        // a patch adds +g to its collider and -g to its radiating bubble; a bubble part adds +g
-        const bool patch = kb >= 0;
-        warp_runs_add(A.s.gfix, kb, h, l);
-        if (patch) {
-            // -X = (-H - 1) 2^31 + (2^31 - L) for L > 0, and -H 2^31 for L = 0
+        long own = -1;  // the bubble whose part the lane holds
+        long long oh[4] = {0, 0, 0, 0}, ol[4] = {0, 0, 0, 0};
+        for (int it = 0; it < kGeomItems; ++it) {
+            geom_item(A, f, q0 + 32 * it, ka, kb, g);
+            // a patch adds +g to its collider and -g to its radiating bubble; a bubble part adds +g
+            const bool patch = kb >= 0;
+            long long h[4], l[4], X[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const long long X = h[c] * (1LL << 31) + l[c];
-                h[c] = (-X) >> 31;
-                l[c] = (-X) & 0x7fffffffLL;
+                X[c] = 0;
+                if (isfinite(g[c])) {
+                    X[c] = __double2ll_rn(ldexp(g[c], sh));
+                } else if (kb >= 0 || ka >= 0) {
+                    // a non-finite gradient is passed on as it is
+                    if (kb >= 0) atomicAdd(A.g_bub + 4 * kb + c, g[c]);
+                    if (ka >= 0 && kb >= 0) atomicAdd(A.g_bub + 4 * ka + c, -g[c]);
+                    else if (ka >= 0) atomicAdd(A.g_bub + 4 * ka + c, g[c]);
+                }
+                h[c] = X[c] >> 31;
+                l[c] = X[c] & 0x7fffffffLL;
+            }
+            if (__any_sync(0xffffffffu, kb >= 0)) warp_runs_add(A.s.gfix, kb, h, l);
+            if (__any_sync(0xffffffffu, ka >= 0 && own >= 0 && ka != own)) {
+                warp_runs_add(A.s.gfix, own, oh, ol);
+                own = -1;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) oh[c] = ol[c] = 0;
+            }
+            if (ka >= 0) {
+                own = ka;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const long long Y = patch ? -X[c] : X[c];
+                    oh[c] += Y >> 31;
+                    ol[c] += Y & 0x7fffffffLL;
+                }
             }
         }
-        warp_runs_add(A.s.gfix, ka, h, l);
+        warp_runs_add(A.s.gfix, own, oh, ol);
     }
 }
 
@@ -735,17 +754,30 @@ __global__ void k_adj_fixout(AdjArgs A) {
     p[1] = 0;
 }
 
+// The row partials of one (frame, bubble) added up by a warp: the bubble's own gradient, and the parameters' sums into its
+// first row, where k_adj_params reads them (32 frames x 256 bubbles x 64 rows: 0.32 ms with every row read there,
+// by one block per parameter).
 template <int SMC>
 __global__ void k_adj_bubble(AdjArgs A) {
-    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const int slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int f = blockIdx.y;
     if (slot >= A.n_sel) return;
-    double st = 0.0, sz = 0.0;
-    for (int i = 0; i < A.n_cos; ++i) {
-        const double* rp = A.s.rowpart + (((size_t)f * A.n_sel + slot) * A.n_cos + i) * (2 + 2 * SMC);
-        st += rp[0];
-        sz += rp[1];
+    double sum[2 + 2 * SMC];
+    double* rows = A.s.rowpart + ((size_t)f * A.n_sel + slot) * A.n_cos * (2 + 2 * SMC);
+#pragma unroll
+    for (int q = 0; q < 2 + 2 * SMC; ++q) sum[q] = 0.0;
+    for (int i = lane; i < A.n_cos; i += 32) {
+#pragma unroll
+        for (int q = 0; q < 2 + 2 * SMC; ++q) sum[q] += rows[(size_t)i * (2 + 2 * SMC) + q];
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < 2 + 2 * SMC; ++q) sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], o);
+    if (lane != 0) return;
+#pragma unroll
+    for (int q = 2; q < 2 + 2 * SMC; ++q) rows[q] = sum[q];
+    const double st = sum[0], sz = sum[1];
     // z' = R[2,:] . x  =>  dL/dx += dL/dz' R[2,:]
     double gx = 0.0, gy = 0.0, gz = sz;
     rotate_back(A.rot ? A.rot + 9 * f : nullptr, gx, gy, gz);
@@ -757,11 +789,12 @@ __global__ void k_adj_bubble(AdjArgs A) {
 }
 
 template <int SMC>
-__global__ void k_adj_params(AdjArgs A, long n_rows) {
+__global__ void k_adj_params(AdjArgs A, long n_bubbles) {
     __shared__ double red[kAdjThreads];
     const int q = blockIdx.x;  // 0 .. 2*SMC-1
     double s = 0.0;
-    for (long r = threadIdx.x; r < n_rows; r += blockDim.x) s += A.s.rowpart[r * (2 + 2 * SMC) + 2 + q];
+    for (long r = threadIdx.x; r < n_bubbles; r += blockDim.x)
+        s += A.s.rowpart[r * A.n_cos * (2 + 2 * SMC) + 2 + q];
     red[threadIdx.x] = s;
     __syncthreads();
     for (int off = blockDim.x / 2; off > 0; off >>= 1) {
@@ -797,19 +830,19 @@ static uint64_t launch_typed(const AdjArgs& A, size_t kn, cudaStream_t st, const
         else launch_rows<S, SMC, 8>(A, rows, st, tt);
         CUDA_OK(cudaGetLastError());
         ++launches;
-        dim3 gb((unsigned)((A.n_sel + 127) / 128), (unsigned)kn);
+        dim3 gb((unsigned)((A.n_sel + 3) / 4), (unsigned)kn);
         k_adj_bubble<SMC><<<gb, 128, 0, st>>>(A);
         CUDA_OK(cudaGetLastError());
         // every bubble gradient of the chunk: fixed-point sums (deterministic)
         const size_t per = (size_t)A.n_sel * A.n_cos * A.n_phi + A.n_sel;
-        dim3 gg((unsigned)((per + 255) / 256), (unsigned)kn);
+        dim3 gg((unsigned)((per + 256 * kGeomItems - 1) / (256 * kGeomItems)), (unsigned)kn);
         k_adj_gexp_init<<<1, 1, 0, st>>>(A.s.gexp);
         k_adj_geom<0><<<gg, 256, 0, st>>>(A);
         k_adj_geom<1><<<gg, 256, 0, st>>>(A);
         k_adj_fixout<<<(unsigned)((4 * A.n_tot + 255) / 256), 256, 0, st>>>(A);
         CUDA_OK(cudaGetLastError());
         launches += 5;
-        k_adj_params<SMC><<<2 * SMC, kAdjThreads, 0, st>>>(A, rows);
+        k_adj_params<SMC><<<2 * SMC, kAdjThreads, 0, st>>>(A, rows / A.n_cos);
         CUDA_OK(cudaGetLastError());
         ++launches;
     }
