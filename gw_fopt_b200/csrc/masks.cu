@@ -705,7 +705,7 @@ __device__ __forceinline__ bool mask_block_fill(const MaskArgs& A, MaskBlock& S,
         for (int e = 0; e < no; ++e) aside |= c == S.oidx[e];
         if (aside) {
             f.w = -CUDART_INF_F;
-        } else if (nrm > 0.0) {  // any other collider keeps a form that is largest and never certified
+        } else if (nrm > 0.0) {  // any other collider keeps a form that is largest, which leaves the direction open
             const double inv = 1.0 / nrm, l1 = fabs(dc.t) + fabs(dc.x) + fabs(dc.y) + fabs(dc.z);
             const double w = 32.0 * 5.9604644775390625e-08 * l1 * inv, slope = theta_slope(S, dc, nrm);
             f = make_float4((float)(dc.x * inv), (float)(dc.y * inv), (float)(dc.z * inv), (float)(w - dc.t * inv));
@@ -950,7 +950,10 @@ __global__ void __launch_bounds__(kMaskListThreads, kMaskBlocks) k_masks_list(Ma
                 // tau with the reference's operations (compute_delta_tab, GBF:457-466)
                 const double tq = __ddiv_rn(S.nrm[q], dmul(2.0, dd));
                 const float top = t_cut >= 0.0f ? fminf(t_cut, S.fval[q].w) : S.fval[q].w;
-                if (sure && dd > 1e-10 && __double2float_ru(tq) <= top && (S.no == 0 || passes_outliers(S, q, x))) tau = tq;
+                // (tq > 0: a null or timelike collider passes every check with a delay that is not positive)
+                if (sure && dd > 1e-10 && tq > 0.0 && __double2float_ru(tq) <= top &&
+                    (S.no == 0 || passes_outliers(S, q, x)))
+                    tau = tq;
             }
         }
         if (rw <= r_last && col < A.n_cols) {
