@@ -709,10 +709,13 @@ __device__ __forceinline__ bool mask_block_fill(const MaskArgs& A, MaskBlock& S,
             const double inv = 1.0 / nrm, l1 = fabs(dc.t) + fabs(dc.x) + fabs(dc.y) + fabs(dc.z);
             const double w = 32.0 * 5.9604644775390625e-08 * l1 * inv, slope = theta_slope(S, dc, nrm);
             f = make_float4((float)(dc.x * inv), (float)(dc.y * inv), (float)(dc.z * inv), (float)(w - dc.t * inv));
-            // max(A, Q) / d = 2 tau max(A, Q) / n <= 4e5, and theta < kmax (1e-6: these bounds' rounding)
+            // max(A, Q) / d = 2 tau max(A, Q) / n <= 4e5, and theta < kmax (1e-6: these bounds' rounding).
+            // A patch list ends at keys above T (1 + 1e-5), so theta = tau (1 + 1e-12 + slope) must not reach
+            // further: only near-lightlike colliders have a slope of 1e-5 (most are below 1e-8), and the
+            // directions that they decide take steps 1-3
             const double top = fmin(2e5 * nrm / fmax(A1, Q), S.kmax / (1.0 + 1e-12 + slope));
             v = make_float4((float)(dx * inv), __double2float_ru(2.0 * w), __double2float_ru(1e-9 * (A1 + Q) * inv),
-                            slope < 0.01 ? __double2float_rd((1.0 - 1e-6) * top) : 0.0f);
+                            slope < 9e-6 ? __double2float_rd((1.0 - 1e-6) * top) : 0.0f);
         }
         S.form[q] = f;
         S.fval[q] = v;
@@ -922,8 +925,8 @@ __global__ void __launch_bounds__(kMaskListThreads, kMaskBlocks) k_masks_list(Ma
                 for (int e = 0; e < n_patch; ++e) visit(pform[e], e);
                 q = n_patch ? ppos[best] : -1;
             } else {
-                // the whole list, until the keys exceed every lane's delay and its bound theta (2 w < 0.01 g and
-                // slope < 0.01 below, so both are under 0.52 / g)
+                // the whole list, until the keys exceed every lane's delay and its bound theta (2 w < 0.01 g below
+                // and slope < 1e-5, so both are under 0.52 / g)
                 for (int e0 = 0; e0 < S.n; e0 += 16) {
                     const unsigned t = g1 > 0.0f ? __float_as_uint(__fdividef(0.52f, g1)) : 0x7f800000u;
                     if (e0 && S.key[e0] > (double)__uint_as_float(__reduce_max_sync(0xffffffffu, t))) break;

@@ -77,3 +77,24 @@ def test_pairs_that_never_collide(gpu_available, n_cos, n_phi, pair, others, sea
     assert np.array_equal(codes, rc)
     assert np.array_equal(tau, rt)
     assert np.all((codes >= 0) == (tau > 0.0))
+
+
+# Colliders that nucleate just ahead of the wall, D / A = (|dx| - dt) / (|dx| + |dt|) from 1e-6 (where a
+# collider is set aside) to 1e-3, all within a relative 1e-5 of one delay: the bound up to which a check can
+# fail reaches past the candidate's own delay there.
+@pytest.mark.parametrize("n_cos,n_phi", [(33, 40), (64, 65)])
+@pytest.mark.parametrize("lo,hi", [(1.5e-6, 3e-6), (3e-6, 3e-5), (3e-5, 1e-3)])
+@pytest.mark.parametrize("search", [by_handle, by_table])
+def test_near_lightlike_colliders(gpu_available, n_cos, n_phi, lo, hi, search):
+    rng = np.random.default_rng(12)
+    n = 60
+    u = rng.normal(size=(n, 3))
+    u[30:] = u[:30] + 1e-4 * rng.normal(size=(30, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    d = np.exp(rng.uniform(np.log(lo), np.log(hi), n))
+    r = 0.5 * (1.0 + 1e-5 * rng.uniform(-1.0, 1.0, n))
+    b = np.concatenate([[[0.0, 0.0, 0.0, 0.0]], np.column_stack([r * (1.0 - 2.0 * d), r[:, None] * u])])
+    codes, tau = search(b, n_cos, n_phi)
+    rc, rt = O.first_colliding(b, NONE, n_cos, n_phi, with_delta_tab=True)
+    assert np.array_equal(codes, rc)
+    assert np.array_equal(tau, rt)
