@@ -167,7 +167,7 @@ struct Readback {
 size_t spectrum_max_frames_per_launch(const Device* dev, const SpectrumJob& job) {
     const size_t nd = job.n_cos * job.n_phi;
     const size_t per_k = job.n_sel * nd * sizeof(double) +
-                         (job.kernel == BGWX_KERNEL_FP64_DIRECT ? direct_bytes_per_frame(dev, job)
+                         (job.kernel == BGWX_KERNEL_FP64_DIRECT ? direct_bytes_per_frame(job)
                                                                 : factored_bytes_per_frame(job));
     const size_t kc = std::max<size_t>(1, mask_budget_bytes(per_k * job.n_k) / std::max<size_t>(per_k, 1));
     return std::min<size_t>(kc, 65535);

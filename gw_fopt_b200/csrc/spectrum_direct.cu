@@ -379,10 +379,10 @@ __device__ __forceinline__ void phase_of(const double2* tab, double x, double& s
 
 struct RowSumArgs {
     DirArgs d;
-    int per_warp;     // blocks of 32 steps (spectrum) or bubbles (integrand) taken in turn by one warp
-    int n_parts;      // partial sums per (pair, column, w) over the whole job
-    int part0;        // first part of this launch's steps
-    double2* partial; // spectrum: (pairs of the job, n_parts, G, S, W); integrand: (bubble parts, G, S, W, n_t)
+    int per_warp;     // spectrum: blocks of 32 steps taken in turn by one warp; integrand: bubbles of a part
+    int n_parts;      // spectrum: blocks of 32 steps of the job
+    int part0;        // spectrum: the first of this launch
+    double2* partial; // spectrum: (pairs of the launch, n_parts, G, S, W); integrand: (bubble parts, G, S, W, n_t)
 };
 
 __device__ __forceinline__ void copy16_async(void* smem, const void* gmem) {
@@ -445,8 +445,9 @@ constexpr int kRowStages = 3;
 // pairs (i, n_cos - 1 - i) of the NC columns and 32 steps arrive in shared memory by asynchronous
 // copies, three stages deep (from L1 and L2 directly the loads' latency was 70 % of the time: 2.09 ms
 // against 0.34 ms of FP64 work for 4 frames of 64 bubbles, 64 rows, 256 steps, 64 w, 6 columns).
+// Two blocks per SM for the spectrum (the integrand's accumulators take what registers they need).
 template <int NC, int NW, bool BIG, bool PER_T>
-__global__ void __launch_bounds__(32 * kDirWarps) k_direct_a(RowSumArgs R, int G, int w_tiles) {
+__global__ void __launch_bounds__(32 * kDirWarps, PER_T ? 0 : 2) k_direct_a(RowSumArgs R, int G, int w_tiles) {
     constexpr int RP = stage_pairs<NC>();
     constexpr int kStageDoubles = RP * 2 * NC * 32;
     extern __shared__ __align__(16) double s_dyn[];
@@ -466,15 +467,25 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_direct_a(RowSumArgs R, int G
     double wv[NW];
 #pragma unroll
     for (int u = 0; u < NW; ++u) wv[u] = A.in.w[min(w0 + u, A.n_w - 1)];
-    // the integrand sums over bubbles per lane; the spectrum adds each unit up over the warp's lanes
-    // (steps) at once and keeps one value per lane, the register budget of two blocks per SM
+    // The integrand sums over a part's bubbles per lane; the spectrum adds each unit up over the warp's lanes
+    // (steps) at once and stores it, one value per lane (the register budget of two blocks per SM).  What is
+    // added to what depends on neither the launch's pairs and steps nor the units of a warp, so a frame's
+    // spectrum has the same bits alone and among others, whatever the scratch memory.
     constexpr int NV = 2 * NW * NC;
     double c_sum[PER_T ? NV : 1];
 #pragma unroll
     for (int v = 0; v < (PER_T ? NV : 1); ++v) c_sum[v] = 0.0;
+    const size_t W = A.n_w;
+    auto place = [&](int e) {  // (G, S, W) index of value e / 2
+        const int u = e / (2 * NC), col = c0 + (e / 2) % NC;
+        return ((size_t)(col % G) * A.S + col / G) * W + w0 + u;
+    };
     // units taken in turn.  Spectrum: step blocks [lo, hi) of one pair; integrand: pairs [lo, hi) at one step block
     const int n_grp = (nkc + R.per_warp - 1) / R.per_warp;
     size_t lo, hi, fixed;
+    double2* o_part = R.partial;  // integrand: the part's array
+    double* o_unit = nullptr;     // spectrum: where this lane's value of unit lo goes (null: it holds none)
+    const size_t o_step = 2 * (size_t)cols * W;
     auto bubble = [&](size_t f) {
         const size_t fs = A.fs0 + f;
         return A.in.bub[(fs / A.n_sel) * A.n_tot + A.in.sel[fs % A.n_sel]];
@@ -483,15 +494,35 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_direct_a(RowSumArgs R, int G
     double t = 0.0, dta = 0.0;
     if constexpr (PER_T) {
         fixed = unit_block % nkc;
-        lo = (size_t)(unit_block / nkc) * R.per_warp;
-        hi = min(lo + R.per_warp, A.n_fs);
+        // this launch's bubbles of the part
+        const size_t part = A.fs0 / R.per_warp + unit_block / nkc;
+        lo = max(part * R.per_warp, A.fs0) - A.fs0;
+        hi = min((part + 1) * R.per_warp, A.fs0 + A.n_fs) - A.fs0;
+        o_part += part * cols * W * A.n_t + A.k0 + 32 * fixed + lane;
+        if (lo + A.fs0 > part * R.per_warp && A.k0 + 32 * (int)fixed + lane < A.k1) {
+            // the part was begun by an earlier launch
+#pragma unroll
+            for (int e = 0; e < NV; e += 2)
+                if (w0 + e / (2 * NC) < A.n_w) {
+                    const double2 v = o_part[place(e) * A.n_t];
+                    c_sum[e] = v.x;
+                    c_sum[e + 1] = v.y;
+                }
+        }
     } else {
         fixed = unit_block / n_grp;
         lo = (size_t)(unit_block % n_grp) * R.per_warp;
         hi = min(lo + R.per_warp, (size_t)nkc);
+        const int e = lane_value<NV>(lane);
+        if (e >= 0 && w0 + e / (2 * NC) < A.n_w)
+            o_unit = reinterpret_cast<double*>(R.partial) + (fixed * R.n_parts + R.part0 + lo) * o_step + 2 * place(e) + (e & 1);
         // step blocks before the bubble nucleates hold nothing
         xa = bubble(fixed);
-        while (lo < hi && !(A.in.t_arr[min(A.k0 + 32 * (int)lo + 31, A.k1 - 1)] - xa.t > 0.0)) ++lo;
+        for (; lo < hi && !(A.in.t_arr[min(A.k0 + 32 * (int)lo + 31, A.k1 - 1)] - xa.t > 0.0); ++lo)
+            if (o_unit) {
+                *o_unit = 0.0;
+                o_unit += o_step;
+            }
     }
     const size_t rstep = (size_t)cols * A.tp;
     const int n_pairs = (A.n_cos + 1) >> 1;
@@ -582,42 +613,52 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_direct_a(RowSumArgs R, int G
 #pragma unroll
             for (int e = 0; e < NV; ++e) c_sum[e] += v[e];
         } else {
-            c_sum[0] += lane_sums<NV>(v);
+            const double total = lane_sums<NV>(v);
+            if (o_unit) {
+                *o_unit = total;
+                o_unit += o_step;
+            }
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    const size_t W = A.n_w;
-    auto place = [&](int e) {  // (G, S, W) index of value e / 2
-        const int u = e / (2 * NC), col = c0 + (e / 2) % NC;
-        return ((size_t)(col % G) * A.S + col / G) * W + w0 + u;
-    };
     if constexpr (PER_T) {
-        const int k = A.k0 + 32 * (int)fixed + lane;
-        if (k >= A.k1) return;
-        double2* o = R.partial + (size_t)(unit_block / nkc) * cols * W * A.n_t;
+        if (A.k0 + 32 * (int)fixed + lane >= A.k1) return;
 #pragma unroll
         for (int e = 0; e < NV; e += 2)
-            if (w0 + e / (2 * NC) < A.n_w) o[place(e) * A.n_t + k] = make_double2(c_sum[e], c_sum[e + 1]);
-    } else {
-        double* o = reinterpret_cast<double*>(
-            R.partial + ((A.fs0 + fixed) * R.n_parts + R.part0 + unit_block % n_grp) * cols * W);
-        const int e = lane_value<NV>(lane);
-        if (e >= 0 && w0 + e / (2 * NC) < A.n_w) o[2 * place(e) + (e & 1)] = c_sum[0];
+            if (w0 + e / (2 * NC) < A.n_w) o_part[place(e) * A.n_t] = make_double2(c_sum[e], c_sum[e + 1]);
     }
 }
 
-// out[k][q] = sum over the n parts of partial[k][part][q] (+ out[k][q] with ADD), in an order that
-// depends on n only: 8 strided lanes of the block's rows, then the lanes in order.
-template <bool ADD>
-__global__ void k_direct_reduce(const double2* __restrict__ partial, size_t n, size_t per, double2* __restrict__ out) {
+// out[p][q] = the sum of pair p's n_parts values at partial[p][part][q], in order.
+__device__ __forceinline__ double2 part_sum(const double2* __restrict__ p, int n_parts, size_t per) {
+    double2 v = make_double2(0.0, 0.0);
+#pragma unroll 8
+    for (int a = 0; a < n_parts; ++a, p += per) {
+        v.x += p->x;
+        v.y += p->y;
+    }
+    return v;
+}
+
+__global__ void k_direct_pairs(const double2* __restrict__ partial, int n_parts, size_t per, size_t n_pairs,
+                               double2* __restrict__ out) {
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t per_pair = n_parts * per;
+    if (q < n_pairs * per) out[q] = part_sum(partial + q / per * per_pair + q % per, n_parts, per);
+}
+
+// out[k][q] = the sum over frame k's n pairs of their parts' sums: 8 strided lanes of the block's rows, then the
+// lanes in order (an order that depends on n and n_parts only).
+__global__ void k_direct_reduce(const double2* __restrict__ partial, size_t n, int n_parts, size_t per,
+                                double2* __restrict__ out) {
     __shared__ double2 red[8][32];
     const size_t q = (size_t)blockIdx.x * 32 + threadIdx.x;
-    const double2* p = partial + (size_t)blockIdx.y * n * per;
+    const size_t per_pair = n_parts * per;
+    const double2* p = partial + blockIdx.y * n * per_pair + q;
     double2 acc = make_double2(0.0, 0.0);
     if (q < per) {
-#pragma unroll 4
         for (size_t a = threadIdx.y; a < n; a += 8) {
-            const double2 v = p[a * per + q];
+            const double2 v = part_sum(p + a * per_pair, n_parts, per);
             acc.x += v.x;
             acc.y += v.y;
         }
@@ -625,13 +666,12 @@ __global__ void k_direct_reduce(const double2* __restrict__ partial, size_t n, s
     red[threadIdx.y][threadIdx.x] = acc;
     __syncthreads();
     if (threadIdx.y || q >= per) return;
-    double2& o = out[(size_t)blockIdx.y * per + q];
-    double2 sum = ADD ? o : make_double2(0.0, 0.0);
+    double2 sum = make_double2(0.0, 0.0);
     for (int y = 0; y < 8; ++y) {
         sum.x += red[y][threadIdx.x].x;
         sum.y += red[y][threadIdx.x].y;
     }
-    o = sum;
+    out[(size_t)blockIdx.y * per + q] = sum;
 }
 
 // Separated factors need (tau / dt_last)^p, (dt_last / dt)^p and the damping exponentials inside the
@@ -671,7 +711,6 @@ struct DirectPlan {
     int nw, nc;          // frequencies per warp, columns per pass
     int nkc;             // blocks of 32 steps
     int per_warp;        // step blocks per warp
-    int n_parts;
 };
 
 // Columns per pass: all six of the tensor form, or up to four sets' two; frequencies per warp: as
@@ -687,7 +726,6 @@ DirectPlan direct_plan(const Device* dev, const SpectrumJob& job, size_t pairs) 
     const size_t warps = pairs * ((job.n_w + p.nw - 1) / p.nw) * (S * p.G / p.nc) * p.nkc;
     const size_t want = (size_t)dev->n_sm * 4 * 16;
     p.per_warp = (int)std::max<size_t>(1, std::min<size_t>(p.nkc, warps / want));
-    p.n_parts = (p.nkc + p.per_warp - 1) / p.per_warp;
     return p;
 }
 
@@ -756,13 +794,31 @@ void dispatch_a(const RowSumArgs& R, const DirectPlan& P, size_t gx, bool big, c
     }
 }
 
-constexpr size_t kDirectBufferBytes = (size_t)1 << 30;  // B of one launch
+constexpr size_t kDirectBufferBytes = (size_t)1 << 30;   // B of one launch
+constexpr size_t kDirectPartialBytes = (size_t)1 << 28;  // partial sums of one launch (spectrum), of the job (integrand)
+// Warps that the integrand's parts are cut for: 8 per scheduler of a B200.  A constant, so that the order of its sums
+// depends on the job alone.
+constexpr size_t kIntegrandWarps = 148 * 4 * 8;
+
+// Steps and pairs of a launch whose B, `step_bytes` a step and pair, fits `limit`: whole step blocks of
+// k_direct_b, one at least; all of a pair's steps before a second pair.
+struct DirectRange {
+    size_t steps, pairs;
+};
+DirectRange direct_range(size_t n_t, size_t pairs, size_t step_bytes, size_t limit) {
+    DirectRange r;
+    const size_t all = (n_t + kStepBlock - 1) / kStepBlock * kStepBlock;
+    r.steps = std::min(all, std::max<size_t>(1, limit / (step_bytes * kStepBlock)) * kStepBlock);
+    r.pairs = std::min(pairs, std::max<size_t>(1, limit / (step_bytes * r.steps)));
+    if (r.steps < all) r.pairs = 1;
+    return r;
+}
 
 }  // namespace
 
-size_t direct_bytes_per_frame(const Device* dev, const SpectrumJob& job) {
-    const DirectPlan P = direct_plan(dev, job, job.n_sel);
-    return job.n_sel * P.n_parts * P.G * job.n_sets * job.n_w * sizeof(double2);
+// (the pairs' sums; the other work arrays are cut to size)
+size_t direct_bytes_per_frame(const SpectrumJob& job) {
+    return job.n_sel * (job.tensor ? 6 : 2) * job.n_sets * job.n_w * sizeof(double2);
 }
 
 uint64_t launch_direct(Device* dev, const SpectrumJob& job, const DirectInputs& in, size_t kn, double2* out) {
@@ -770,39 +826,46 @@ uint64_t launch_direct(Device* dev, const SpectrumJob& job, const DirectInputs& 
     const DirectPlan P = direct_plan(dev, job, pairs);
     const size_t cols = (size_t)P.G * job.n_sets, per = cols * job.n_w;
     const bool exact = direct_exact(job), big = direct_big(job);
-    dev->partial.ensure(pairs * P.n_parts * per * sizeof(double2));
-    // B holds a range of pairs over a range of steps (whole groups of per_warp step blocks)
-    const size_t group = (size_t)P.per_warp * 32;
-    const size_t col_bytes = job.n_cos * cols * sizeof(double);
-    const size_t range = 4 * group;  // whole step blocks of k_direct_b too
-    const size_t steps = std::max<size_t>(1, std::min<size_t>((job.n_t + range - 1) / range,
-                                                              kDirectBufferBytes / (col_bytes * range))) * range;
-    const size_t n_fs = std::min(pairs, std::max<size_t>(1, kDirectBufferBytes / (col_bytes * std::min(steps, (size_t)P.nkc * 32))));
     DirArgs A = direct_args(job, in);
     launch_steps(dev, A);
     uint64_t launches = 1;
-    for (size_t k0 = 0; k0 < job.n_t; k0 += steps) {
-        A.k0 = (int)k0;
-        A.k1 = (int)std::min(job.n_t, k0 + steps);
-        A.tp = (A.k1 - A.k0 + 31) & ~31;
-        dev->beta.ensure(n_fs * job.n_cos * cols * A.tp * sizeof(double));
-        A.B = (double*)dev->beta.p;
-        for (size_t f0 = 0; f0 < pairs; f0 += n_fs) {
-            A.fs0 = f0;
-            A.n_fs = std::min(n_fs, pairs - f0);
+    const size_t step_bytes = job.n_cos * cols * sizeof(double), part_bytes = P.nkc * per * sizeof(double2);
+    DirectRange r = direct_range(job.n_t, pairs, step_bytes, kDirectBufferBytes);
+    r.pairs = std::min(r.pairs, std::max<size_t>(1, kDirectPartialBytes / part_bytes));
+    dev->partial.ensure(r.pairs * part_bytes);
+    dev->beta.ensure(r.pairs * step_bytes * r.steps);
+    A.B = (double*)dev->beta.p;
+    // in several launches each pair's parts are added up before the next ones overwrite them
+    const bool once = r.pairs == pairs;
+    if (!once) dev->fact_partial.ensure(pairs * per * sizeof(double2));
+    for (size_t f0 = 0; f0 < pairs; f0 += r.pairs) {
+        A.fs0 = f0;
+        A.n_fs = std::min(r.pairs, pairs - f0);
+        for (size_t k0 = 0; k0 < job.n_t; k0 += r.steps) {
+            A.k0 = (int)k0;
+            A.k1 = (int)std::min(job.n_t, k0 + r.steps);
+            A.tp = (A.k1 - A.k0 + 31) & ~31;
             if (job.tensor)
                 launch_b<6>(A, exact, dev->stream);
             else
                 launch_b<2>(A, exact, dev->stream);
-            const RowSumArgs R{A, P.per_warp, P.n_parts, (int)(k0 / group), (double2*)dev->partial.p};
+            const RowSumArgs R{A, P.per_warp, P.nkc, (int)(k0 / 32), (double2*)dev->partial.p};
             const size_t groups = ((A.k1 - A.k0 + 31) / 32 + P.per_warp - 1) / P.per_warp;
             dispatch_a<false>(R, P, A.n_fs * groups, big, dev->stream);
             launches += 2;
         }
+        if (!once) {
+            const size_t n = A.n_fs * per;
+            if ((n + 255) / 256 > 0x7fffffffULL) throw Error{"direct kernel: too many partial sums for one launch"};
+            k_direct_pairs<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(
+                (const double2*)dev->partial.p, P.nkc, per, A.n_fs, (double2*)dev->fact_partial.p + f0 * per);
+            CUDA_OK(cudaGetLastError());
+            ++launches;
+        }
     }
     const dim3 gr((unsigned)((per + 31) / 32), (unsigned)kn);
-    k_direct_reduce<false><<<gr, dim3(32, 8), 0, dev->stream>>>((const double2*)dev->partial.p, job.n_sel * P.n_parts,
-                                                                per, out);
+    k_direct_reduce<<<gr, dim3(32, 8), 0, dev->stream>>>((const double2*)(once ? dev->partial : dev->fact_partial).p,
+                                                         job.n_sel, once ? P.nkc : 1, per, out);
     CUDA_OK(cudaGetLastError());
     return launches + 1;
 }
@@ -812,50 +875,43 @@ uint64_t launch_direct_integrand(Device* dev, const SpectrumJob& job, const Dire
     DirectPlan P = direct_plan(dev, job, pairs);
     const size_t cols = (size_t)P.G * job.n_sets, per = cols * job.n_w * job.n_t;
     const bool exact = direct_exact(job), big = direct_big(job);
-    // B holds a range of bubbles over all steps, or one bubble over a range of steps
-    const size_t step_bytes = job.n_cos * cols * 32 * sizeof(double);
-    // (a multiple of four 32-step blocks: whole step blocks of k_direct_b)
-    const size_t nkc = std::min<size_t>((P.nkc + 3) & ~3, std::max<size_t>(1, kDirectBufferBytes / (4 * step_bytes)) * 4);
-    const size_t n_fs = std::min(pairs, std::max<size_t>(1, kDirectBufferBytes / (step_bytes * nkc)));
-    // bubbles per warp: few enough for the chip to be full, as many as keep the partial outputs small
+    // bubbles of a part: few enough for the chip to be full, as many as keep the parts' outputs small
     const size_t warps = ((job.n_w + P.nw - 1) / P.nw) * (cols / P.nc) * P.nkc;
-    const size_t want = (size_t)dev->n_sm * 4 * 8;
-    size_t groups = std::min(n_fs, std::max<size_t>(1, (want + warps - 1) / warps));
-    groups = std::min(groups, std::max<size_t>(1, kDirectBufferBytes / (per * sizeof(double2))));
-    P.per_warp = (int)((n_fs + groups - 1) / groups);
-    dev->partial.ensure(((n_fs + P.per_warp - 1) / P.per_warp) * per * sizeof(double2));
-    dev->beta.ensure(n_fs * nkc * step_bytes);
+    size_t parts = std::min(pairs, std::max<size_t>(1, (kIntegrandWarps + warps - 1) / warps));
+    parts = std::min(parts, std::max<size_t>(1, kDirectPartialBytes / (per * sizeof(double2))));
+    P.per_warp = (int)((pairs + parts - 1) / parts);
+    parts = (pairs + P.per_warp - 1) / P.per_warp;
     const size_t gx = (per + 31) / 32;
     if (gx > 0x7fffffffULL) throw Error{"direct kernel: integrand too large for one launch"};
     DirArgs A = direct_args(job, in);
-    A.B = (double*)dev->beta.p;
     launch_steps(dev, A);
     uint64_t launches = 1;
-    for (size_t f0 = 0; f0 < pairs; f0 += n_fs) {
+    const size_t step_bytes = job.n_cos * cols * sizeof(double);
+    const DirectRange r = direct_range(job.n_t, pairs, step_bytes, kDirectBufferBytes);
+    dev->partial.ensure(parts * per * sizeof(double2));
+    dev->beta.ensure(r.pairs * step_bytes * r.steps);
+    A.B = (double*)dev->beta.p;
+    for (size_t f0 = 0; f0 < pairs; f0 += r.pairs) {
         A.fs0 = f0;
-        A.n_fs = std::min(n_fs, pairs - f0);
-        const size_t parts = (A.n_fs + P.per_warp - 1) / P.per_warp;
-        for (size_t k0 = 0; k0 < job.n_t; k0 += 32 * nkc) {
+        A.n_fs = std::min(r.pairs, pairs - f0);
+        const size_t touched = (f0 + A.n_fs - 1) / P.per_warp - f0 / P.per_warp + 1;
+        for (size_t k0 = 0; k0 < job.n_t; k0 += r.steps) {
             A.k0 = (int)k0;
-            A.k1 = (int)std::min(job.n_t, k0 + 32 * nkc);
+            A.k1 = (int)std::min(job.n_t, k0 + r.steps);
             A.tp = (A.k1 - A.k0 + 31) & ~31;
             if (job.tensor)
                 launch_b<6>(A, exact, dev->stream);
             else
                 launch_b<2>(A, exact, dev->stream);
             const RowSumArgs R{A, P.per_warp, 0, 0, (double2*)dev->partial.p};
-            dispatch_a<true>(R, P, parts * (size_t)(A.tp / 32), big, dev->stream);
+            dispatch_a<true>(R, P, touched * (size_t)(A.tp / 32), big, dev->stream);
             launches += 2;
         }
-        const dim3 gr((unsigned)gx, 1), block(32, 8);
-        if (f0 == 0)
-            k_direct_reduce<false><<<gr, block, 0, dev->stream>>>((const double2*)dev->partial.p, parts, per, out);
-        else
-            k_direct_reduce<true><<<gr, block, 0, dev->stream>>>((const double2*)dev->partial.p, parts, per, out);
-        CUDA_OK(cudaGetLastError());
-        ++launches;
     }
-    return launches;
+    k_direct_reduce<<<dim3((unsigned)gx, 1), dim3(32, 8), 0, dev->stream>>>((const double2*)dev->partial.p, parts, 1,
+                                                                          per, out);
+    CUDA_OK(cudaGetLastError());
+    return launches + 1;
 }
 
 }  // namespace bgw

@@ -30,6 +30,6 @@ uint64_t launch_direct(Device* dev, const SpectrumJob& job, const DirectInputs& 
 uint64_t launch_direct_integrand(Device* dev, const SpectrumJob& job, const DirectInputs& in, double2* out);
 
 // Device bytes per k-hat frame of the work arrays that grow with the frames.
-size_t direct_bytes_per_frame(const Device* dev, const SpectrumJob& job);
+size_t direct_bytes_per_frame(const SpectrumJob& job);
 
 }  // namespace bgw
