@@ -54,15 +54,26 @@ struct DevBuf {
     bool shadow_valid = false;
     unsigned long long gen = 0;  // (re)allocations of this buffer
     void ensure(size_t bytes) {
-        if (bytes <= cap) return;
+        if (!try_ensure(bytes)) throw Error{"CUDA error: out of memory (" + std::to_string(bytes) + " bytes)"};
+    }
+    // False when the device has no room for `bytes`.
+    bool try_ensure(size_t bytes) {
+        if (bytes <= cap) return true;
         if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
         size_t want = bytes < 256 ? 256 : bytes;
-        CUDA_OK(cudaMalloc(&p, want));
+        const cudaError_t e = cudaMalloc(&p, want);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();  // or the next launch's check would report it
+            p = nullptr;
+            return false;
+        }
+        CUDA_OK(e);
         cap = want;
         shadow_valid = false;
         ++gen;
+        return true;
     }
     ~DevBuf() {
         if (p) cudaFree(p);

@@ -794,7 +794,8 @@ void dispatch_a(const RowSumArgs& R, const DirectPlan& P, size_t gx, bool big, c
     }
 }
 
-constexpr size_t kDirectBufferBytes = (size_t)1 << 30;   // B of one launch
+constexpr size_t kDirectBufferBytes = (size_t)1 << 30;   // B of one launch, at most
+constexpr size_t kDirectSmallBytes = (size_t)1 << 28;    // ... taken without a look at the free memory
 constexpr size_t kDirectPartialBytes = (size_t)1 << 28;  // partial sums of one launch (spectrum), of the job (integrand)
 // Warps that the integrand's parts are cut for: 8 per scheduler of a B200.  A constant, so that the order of its sums
 // depends on the job alone.
@@ -814,6 +815,26 @@ DirectRange direct_range(size_t n_t, size_t pairs, size_t step_bytes, size_t lim
     return r;
 }
 
+// The largest range whose work arrays the device has room for: `reserve` allocates those of a range under a limit
+// for B and says whether it could.  256 MiB serve a job that needs no more; a larger one, and one that they were
+// refused, gets a third of the free memory up to 1 GiB (the query takes 67 us).
+template <class F>
+DirectRange reserve_range(const Device* dev, const SpectrumJob& job, size_t pairs, size_t step_bytes, F&& reserve) {
+    auto third = [&]() -> size_t {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return kDirectSmallBytes;
+        return std::min((free_b + dev->beta.cap) / 3, kDirectBufferBytes);
+    };
+    size_t limit = kDirectSmallBytes;
+    if (pairs * step_bytes * job.n_t > limit) limit = third();
+    for (;;) {
+        DirectRange r = direct_range(job.n_t, pairs, step_bytes, limit);
+        if (reserve(r, limit)) return r;
+        if (limit == 0) throw Error{"CUDA error: out of memory (work arrays of the direct kernel)"};
+        limit = std::min(limit / 2, third());
+    }
+}
+
 }  // namespace
 
 // (the pairs' sums; the other work arrays are cut to size)
@@ -830,14 +851,14 @@ uint64_t launch_direct(Device* dev, const SpectrumJob& job, const DirectInputs& 
     launch_steps(dev, A);
     uint64_t launches = 1;
     const size_t step_bytes = job.n_cos * cols * sizeof(double), part_bytes = P.nkc * per * sizeof(double2);
-    DirectRange r = direct_range(job.n_t, pairs, step_bytes, kDirectBufferBytes);
-    r.pairs = std::min(r.pairs, std::max<size_t>(1, kDirectPartialBytes / part_bytes));
-    dev->partial.ensure(r.pairs * part_bytes);
-    dev->beta.ensure(r.pairs * step_bytes * r.steps);
+    const DirectRange r = reserve_range(dev, job, pairs, step_bytes, [&](DirectRange& q, size_t limit) {
+        q.pairs = std::min(q.pairs, std::max<size_t>(1, std::min(limit, kDirectPartialBytes) / part_bytes));
+        return (q.pairs == pairs || dev->fact_partial.try_ensure(pairs * per * sizeof(double2))) &&
+               dev->partial.try_ensure(q.pairs * part_bytes) && dev->beta.try_ensure(q.pairs * step_bytes * q.steps);
+    });
     A.B = (double*)dev->beta.p;
     // in several launches each pair's parts are added up before the next ones overwrite them
     const bool once = r.pairs == pairs;
-    if (!once) dev->fact_partial.ensure(pairs * per * sizeof(double2));
     for (size_t f0 = 0; f0 < pairs; f0 += r.pairs) {
         A.fs0 = f0;
         A.n_fs = std::min(r.pairs, pairs - f0);
@@ -887,9 +908,10 @@ uint64_t launch_direct_integrand(Device* dev, const SpectrumJob& job, const Dire
     launch_steps(dev, A);
     uint64_t launches = 1;
     const size_t step_bytes = job.n_cos * cols * sizeof(double);
-    const DirectRange r = direct_range(job.n_t, pairs, step_bytes, kDirectBufferBytes);
     dev->partial.ensure(parts * per * sizeof(double2));
-    dev->beta.ensure(r.pairs * step_bytes * r.steps);
+    const DirectRange r = reserve_range(dev, job, pairs, step_bytes, [&](const DirectRange& q, size_t) {
+        return dev->beta.try_ensure(q.pairs * step_bytes * q.steps);
+    });
     A.B = (double*)dev->beta.p;
     for (size_t f0 = 0; f0 < pairs; f0 += r.pairs) {
         A.fs0 = f0;
