@@ -629,17 +629,24 @@ __global__ void __launch_bounds__(32 * kDirWarps, PER_T ? 0 : 2) k_direct_a(RowS
     }
 }
 
-// out[p][q] = the sum of pair p's n_parts values at partial[p][part][q], in order.
+// The sum of a pair's n_parts values at p[part per], in order; eight loads in flight (past the end zeros, which
+// change no sum: a loop of single loads for the remainder took 2 to 4 us of a 90 us call).
 __device__ __forceinline__ double2 part_sum(const double2* __restrict__ p, int n_parts, size_t per) {
     double2 v = make_double2(0.0, 0.0);
-#pragma unroll 8
-    for (int a = 0; a < n_parts; ++a, p += per) {
-        v.x += p->x;
-        v.y += p->y;
+    for (int a = 0; a < n_parts; a += 8) {
+        double2 x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = a + u < n_parts ? p[(a + u) * per] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            v.x += x[u].x;
+            v.y += x[u].y;
+        }
     }
     return v;
 }
 
+// out[p][q] = the sum of pair p's parts at partial[p][part][q].
 __global__ void k_direct_pairs(const double2* __restrict__ partial, int n_parts, size_t per, size_t n_pairs,
                                double2* __restrict__ out) {
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -647,17 +654,19 @@ __global__ void k_direct_pairs(const double2* __restrict__ partial, int n_parts,
     if (q < n_pairs * per) out[q] = part_sum(partial + q / per * per_pair + q % per, n_parts, per);
 }
 
-// out[k][q] = the sum over frame k's n pairs of their parts' sums: 8 strided lanes of the block's rows, then the
-// lanes in order (an order that depends on n and n_parts only).
-__global__ void k_direct_reduce(const double2* __restrict__ partial, size_t n, int n_parts, size_t per,
+constexpr int kReduceRows = 32;
+
+// out[k][q] = the sum over frame k's n pairs of their parts' sums: kReduceRows strided rows of threads, then the
+// rows in order (an order that depends on n and n_parts only).
+__global__ void __launch_bounds__(32 * kReduceRows) k_direct_reduce(const double2* __restrict__ partial, size_t n, int n_parts, size_t per,
                                 double2* __restrict__ out) {
-    __shared__ double2 red[8][32];
+    __shared__ double2 red[kReduceRows][32];
     const size_t q = (size_t)blockIdx.x * 32 + threadIdx.x;
     const size_t per_pair = n_parts * per;
     const double2* p = partial + blockIdx.y * n * per_pair + q;
     double2 acc = make_double2(0.0, 0.0);
     if (q < per) {
-        for (size_t a = threadIdx.y; a < n; a += 8) {
+        for (size_t a = threadIdx.y; a < n; a += kReduceRows) {
             const double2 v = part_sum(p + a * per_pair, n_parts, per);
             acc.x += v.x;
             acc.y += v.y;
@@ -667,7 +676,7 @@ __global__ void k_direct_reduce(const double2* __restrict__ partial, size_t n, i
     __syncthreads();
     if (threadIdx.y || q >= per) return;
     double2 sum = make_double2(0.0, 0.0);
-    for (int y = 0; y < 8; ++y) {
+    for (int y = 0; y < (int)min(n, (size_t)kReduceRows); ++y) {
         sum.x += red[y][threadIdx.x].x;
         sum.y += red[y][threadIdx.x].y;
     }
@@ -885,7 +894,7 @@ uint64_t launch_direct(Device* dev, const SpectrumJob& job, const DirectInputs& 
         }
     }
     const dim3 gr((unsigned)((per + 31) / 32), (unsigned)kn);
-    k_direct_reduce<<<gr, dim3(32, 8), 0, dev->stream>>>((const double2*)(once ? dev->partial : dev->fact_partial).p,
+    k_direct_reduce<<<gr, dim3(32, kReduceRows), 0, dev->stream>>>((const double2*)(once ? dev->partial : dev->fact_partial).p,
                                                          job.n_sel, once ? P.nkc : 1, per, out);
     CUDA_OK(cudaGetLastError());
     return launches + 1;
@@ -930,7 +939,7 @@ uint64_t launch_direct_integrand(Device* dev, const SpectrumJob& job, const Dire
             launches += 2;
         }
     }
-    k_direct_reduce<<<dim3((unsigned)gx, 1), dim3(32, 8), 0, dev->stream>>>((const double2*)dev->partial.p, parts, 1,
+    k_direct_reduce<<<dim3((unsigned)gx, 1), dim3(32, kReduceRows), 0, dev->stream>>>((const double2*)dev->partial.p, parts, 1,
                                                                           per, out);
     CUDA_OK(cudaGetLastError());
     return launches + 1;
