@@ -241,8 +241,8 @@ void compute_common(bgw_generalized_bulk_flow* h, const double* w_arr, size_t n_
     if (out_device && out_len != expected)
         throw Error{"out_len=" + std::to_string(out_len) + " does not match expected length " +
                     std::to_string(expected)};
-    // the result goes straight into the caller's array (a wrong length is reported after the computation,
-    // as it always was)
+    // the result goes straight into the caller's array once it is known to be valid (a wrong length is reported
+    // after the computation, as it always was)
     static_assert(sizeof(BgwComplex64) == 2 * sizeof(double), "interleaved complex");
     const bool direct = out && out_len == expected;
     std::vector<double> result(out_device || direct ? 0 : 2 * expected, 0.0);

@@ -21,6 +21,7 @@
 #include "bgw_internal.h"
 #include "device_common.cuh"
 #include "masks.cuh"
+#include "readback.h"
 #include "spectrum_direct.cuh"
 #include "spectrum_factored.cuh"
 #include "adjoint.cuh"
@@ -131,36 +132,20 @@ size_t mask_budget_bytes(size_t need) {
     return std::max<size_t>(least, std::min(free_b / 3, cap));
 }
 
-// Device -> host copies of a call's small results: queued into pinned memory, handed over after the one
-// synchronisation (copies to pageable memory wait for the device one by one).  A larger copy goes directly.
-struct Readback {
-    static constexpr size_t kBytes = 1 << 18;
-    Device* dev;
-    size_t used = 0;
-    struct Part {
-        void* dst;
-        size_t at, bytes;
-    };
-    std::vector<Part> parts;
-    explicit Readback(Device* d) : dev(d) {
-        if (!dev->pinned) CUDA_OK(cudaMallocHost(&dev->pinned, kBytes));
+// The copies of Readback on a device's stream.
+struct StreamCopies {
+    cudaStream_t stream;
+    void copy(void* dst, const void* src, size_t bytes) {
+        CUDA_OK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream));
     }
-    void add(void* dst, const void* src, size_t bytes) {
-        if (used + bytes <= kBytes) {
-            CUDA_OK(cudaMemcpyAsync(static_cast<char*>(dev->pinned) + used, src, bytes, cudaMemcpyDeviceToHost, dev->stream));
-            parts.push_back({dst, used, bytes});
-            used = (used + bytes + 15) & ~(size_t)15;
-        } else {
-            CUDA_OK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, dev->stream));
-        }
-    }
-    void wait() {
-        CUDA_OK(cudaStreamSynchronize(dev->stream));
-        for (const Part& p : parts) std::memcpy(p.dst, static_cast<char*>(dev->pinned) + p.at, p.bytes);
-        parts.clear();
-        used = 0;
-    }
+    void wait() { CUDA_OK(cudaStreamSynchronize(stream)); }
 };
+using Results = Readback<StreamCopies>;
+
+void* staging_block(Device* dev) {
+    if (!dev->pinned) CUDA_OK(cudaMallocHost(&dev->pinned, Results::kBytes));
+    return dev->pinned;
+}
 
 }  // namespace
 
@@ -200,7 +185,7 @@ void run_masks(Device* dev, const MaskJob& job, int32_t* out_codes, double* out_
                          (int32_t*)dev->codes.p, (unsigned long long*)dev->counters.p, true, &nl);
     CUDA_OK(cudaEventRecord(dev->ev[1], dev->stream));
     unsigned long long fb = 0;
-    Readback back(dev);
+    Results back({dev->stream}, staging_block(dev));
     back.add(out_codes, dev->codes.p, job.n_sel * nd * sizeof(int32_t));
     if (out_tau) back.add(out_tau, dev->tau.p, job.n_sel * nd * sizeof(double));
     back.add(&fb, dev->counters.p, sizeof fb);
@@ -265,11 +250,12 @@ static void add_stage_times(Device* dev, BgwxTimings* tm) {
 static void check_counters(Device* dev, unsigned long long* fallbacks, void* out = nullptr, const void* src = nullptr,
                            size_t bytes = 0) {
     unsigned long long cnt[2] = {0, 0};
-    Readback back(dev);
-    back.add(cnt, dev->counters.p, sizeof cnt);
+    Results back({dev->stream}, staging_block(dev));
+    back.status(cnt, dev->counters.p, sizeof cnt);
     if (bytes) back.add(out, src, bytes);
-    back.wait();
-    if (cnt[1] != 0) throw Error{"tensor-core GEMM: a pipeline wait gave up; the result is invalid"};
+    back.wait([&] {
+        if (cnt[1] != 0) throw Error{"tensor-core GEMM: a pipeline wait gave up; the result is invalid"};
+    });
     if (fallbacks) *fallbacks = cnt[0];
 }
 
@@ -657,7 +643,7 @@ void run_adjoint(Device* dev, const SpectrumJob& job, const double* gbar, double
                                          d_gpar);
     }
     CUDA_OK(cudaEventRecord(dev->ev[5], dev->stream));
-    Readback back(dev);
+    Results back({dev->stream}, staging_block(dev));
     back.add(g_bub, d_gbub, 4 * job.n_tot * sizeof(double));
     back.add(g_par, d_gpar, 2 * SM * sizeof(double));
     back.wait();
@@ -702,7 +688,7 @@ void run_integrand(Device* dev, const SpectrumJob& job, double* out, BgwxTimings
                           coeffs, powers, t_arr,                     cutw,   w};
     launches += launch_direct_integrand(dev, job, in, (double2*)dev->out.p);
     CUDA_OK(cudaEventRecord(dev->ev[5], dev->stream));
-    Readback back(dev);
+    Results back({dev->stream}, staging_block(dev));
     back.add(out, dev->out.p, per * sizeof(double2));
     back.wait();
     float total = 0;

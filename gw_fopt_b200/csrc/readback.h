@@ -1,0 +1,80 @@
+// Device -> host copies of a call's results (host code; no CUDA header, the runtime is a parameter).
+#pragma once
+
+#include <cstddef>
+#include <cstring>
+#include <vector>
+
+namespace bgw {
+
+// Small results are queued into a staging block of pinned memory and handed over after the one synchronisation (a copy
+// to pageable memory waits for the device by itself); larger ones are copied directly.  With a status (error counters
+// of the call, queued first) nothing reaches a result's place before the status was looked at: a call that fails
+// leaves the caller's arrays alone.
+//
+// Rt: void copy(void* dst, const void* src, size_t bytes), which queues a device -> host copy, and void wait(), which
+// waits for everything queued; both throw on failure.
+template <class Rt>
+class Readback {
+public:
+    static constexpr size_t kBytes = 1 << 18;  // of the staging block
+
+    Readback(Rt rt, void* block) : rt_(rt), block_(static_cast<char*>(block)) {}
+    Readback(const Readback&) = delete;
+    Readback& operator=(const Readback&) = delete;
+
+    // At most once, before any result.
+    void status(void* dst, const void* src, size_t bytes) {
+        stage(dst, src, bytes);
+        has_status_ = true;
+    }
+    void add(void* dst, const void* src, size_t bytes) {
+        if (used_ + bytes <= kBytes)
+            stage(dst, src, bytes);
+        else if (has_status_)
+            large_.push_back({dst, src, bytes});
+        else
+            rt_.copy(dst, src, bytes);
+    }
+    // Waits; `check` looks at the status and throws when the results are invalid.
+    template <class Check>
+    void wait(Check&& check) {
+        rt_.wait();
+        size_t q = 0;
+        if (has_status_) {
+            deliver(staged_[q++]);
+            check();
+        }
+        for (; q < staged_.size(); ++q) deliver(staged_[q]);
+        for (const Part& p : large_) rt_.copy(p.dst, p.src, p.bytes);
+        if (!large_.empty()) rt_.wait();
+        staged_.clear();
+        large_.clear();
+        used_ = 0;
+        has_status_ = false;
+    }
+    void wait() {
+        wait([] {});
+    }
+
+private:
+    struct Part {
+        void* dst;
+        const void* src;  // in the staging block or, of a large part, on the device
+        size_t bytes;
+    };
+    void stage(void* dst, const void* src, size_t bytes) {
+        rt_.copy(block_ + used_, src, bytes);
+        staged_.push_back({dst, block_ + used_, bytes});
+        used_ = (used_ + bytes + 15) & ~(size_t)15;
+    }
+    static void deliver(const Part& p) { std::memcpy(p.dst, p.src, p.bytes); }
+
+    Rt rt_;
+    char* block_;
+    size_t used_ = 0;
+    bool has_status_ = false;
+    std::vector<Part> staged_, large_;
+};
+
+}  // namespace bgw
