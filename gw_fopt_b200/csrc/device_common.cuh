@@ -86,7 +86,6 @@ struct Device {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;  // own_stream or a caller-provided stream
     cudaEvent_t ev[8] = {};
-    void* pinned = nullptr;         // staging of small device -> host copies (pipeline.cu, Readback)
     std::vector<cudaEvent_t> chunk_ev;  // 3 per k-hat chunk
     std::vector<cudaEvent_t> fact_ev;   // 3 per k-hat chunk: before beta, before GEMM, after GEMM
     DevBuf bub, bubrot, dirs, cos_t, sin2, cos2, coeffs, powers, t_arr, cutw, w, sel, rot, cosphi, sinphi;

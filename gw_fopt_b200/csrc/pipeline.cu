@@ -72,7 +72,6 @@ Device::~Device() {
     if (stream) cudaStreamSynchronize(stream);
     if (ens_graph) cudaGraphExecDestroy(ens_graph);
     if (own_stream) cudaStreamDestroy(own_stream);
-    if (pinned) cudaFreeHost(pinned);
     for (auto& e : ev)
         if (e) cudaEventDestroy(e);
     for (auto& e : chunk_ev)
@@ -132,9 +131,20 @@ size_t mask_budget_bytes(size_t need) {
     return std::max<size_t>(least, std::min(free_b / 3, cap));
 }
 
+// Pinned staging blocks of all handles, on every device (256 KB each, four kept at most).  A block of its own cost each
+// new handle's first call about 0.1 ms.  Never destroyed: the process may end after the CUDA runtime has.
+BlockPool& staging_blocks() {
+    static BlockPool* pool = new BlockPool();
+    return *pool;
+}
+
 // The copies of Readback on a device's stream.
 struct StreamCopies {
     cudaStream_t stream;
+    void* take();
+    void give(void* block) {
+        staging_blocks().give(block, [](void* p) { cudaFreeHost(p); });
+    }
     void copy(void* dst, const void* src, size_t bytes) {
         CUDA_OK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream));
     }
@@ -142,9 +152,12 @@ struct StreamCopies {
 };
 using Results = Readback<StreamCopies>;
 
-void* staging_block(Device* dev) {
-    if (!dev->pinned) CUDA_OK(cudaMallocHost(&dev->pinned, Results::kBytes));
-    return dev->pinned;
+void* StreamCopies::take() {
+    return staging_blocks().take([] {
+        void* p = nullptr;
+        CUDA_OK(cudaHostAlloc(&p, Results::kBytes, cudaHostAllocPortable));
+        return p;
+    });
 }
 
 }  // namespace
@@ -185,7 +198,7 @@ void run_masks(Device* dev, const MaskJob& job, int32_t* out_codes, double* out_
                          (int32_t*)dev->codes.p, (unsigned long long*)dev->counters.p, true, &nl);
     CUDA_OK(cudaEventRecord(dev->ev[1], dev->stream));
     unsigned long long fb = 0;
-    Results back({dev->stream}, staging_block(dev));
+    Results back(StreamCopies{dev->stream});
     back.add(out_codes, dev->codes.p, job.n_sel * nd * sizeof(int32_t));
     if (out_tau) back.add(out_tau, dev->tau.p, job.n_sel * nd * sizeof(double));
     back.add(&fb, dev->counters.p, sizeof fb);
@@ -250,7 +263,7 @@ static void add_stage_times(Device* dev, BgwxTimings* tm) {
 static void check_counters(Device* dev, unsigned long long* fallbacks, void* out = nullptr, const void* src = nullptr,
                            size_t bytes = 0) {
     unsigned long long cnt[2] = {0, 0};
-    Results back({dev->stream}, staging_block(dev));
+    Results back(StreamCopies{dev->stream});
     back.status(cnt, dev->counters.p, sizeof cnt);
     if (bytes) back.add(out, src, bytes);
     back.wait([&] {
@@ -643,7 +656,7 @@ void run_adjoint(Device* dev, const SpectrumJob& job, const double* gbar, double
                                          d_gpar);
     }
     CUDA_OK(cudaEventRecord(dev->ev[5], dev->stream));
-    Results back({dev->stream}, staging_block(dev));
+    Results back(StreamCopies{dev->stream});
     back.add(g_bub, d_gbub, 4 * job.n_tot * sizeof(double));
     back.add(g_par, d_gpar, 2 * SM * sizeof(double));
     back.wait();
@@ -688,7 +701,7 @@ void run_integrand(Device* dev, const SpectrumJob& job, double* out, BgwxTimings
                           coeffs, powers, t_arr,                     cutw,   w};
     launches += launch_direct_integrand(dev, job, in, (double2*)dev->out.p);
     CUDA_OK(cudaEventRecord(dev->ev[5], dev->stream));
-    Results back({dev->stream}, staging_block(dev));
+    Results back(StreamCopies{dev->stream});
     back.add(out, dev->out.p, per * sizeof(double2));
     back.wait();
     float total = 0;

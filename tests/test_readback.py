@@ -22,6 +22,9 @@ struct Queue {
 };
 struct Rt {
     Queue* q;
+    void* block;
+    void* take() { return block; }
+    void give(void*) {}
     void copy(void* dst, const void* src, size_t bytes) { q->queued.push_back({dst, src, bytes}); }
     void wait() {
         ++q->waits;
@@ -59,7 +62,7 @@ int main() {
         q.fail = lost;
         unsigned status = 0;
         const unsigned bad = 7;
-        R r({&q}, block.data());
+        R r(Rt{&q, block.data()});
         r.status(&status, &bad, sizeof bad);
         r.add(small.data(), dev.data(), small.size());
         r.add(large.data(), dev.data(), large.size());
@@ -84,7 +87,7 @@ int main() {
     std::vector<char> block(R::kBytes), dev(kLarge);
     for (size_t i = 0; i < dev.size(); ++i) dev[i] = (char)(i * 37 + 1);
     Queue q;
-    R r({&q}, block.data());
+    R r(Rt{&q, block.data()});
     for (int status = 0; status < 2; ++status)
         for (int with_large = 0; with_large < 2; ++with_large) {
             std::vector<char> large(kLarge), whole(R::kBytes - 32), odd(13), rest(64);
@@ -108,5 +111,78 @@ int main() {
     r.add(a.data(), dev.data(), a.size());
     r.wait();
     EXPECT(q.waits == 1 && !std::memcmp(a.data(), dev.data(), a.size()));
+}
+""")
+
+
+# Staging blocks are shared by all handles: a block is in one call at a time, at most four wait, the rest are freed,
+# and a call that ends by an error gives its block back only after its copies ended, or not at all.
+def test_blocks_are_given_back(tmp_path):
+    run(tmp_path, r"""
+#include <atomic>
+#include <set>
+#include <thread>
+bgw::BlockPool pool;
+std::atomic<int> made{0}, freed{0};
+struct Pooled : Rt {
+    void* take() { return pool.take([] { ++made; return std::malloc(R::kBytes); }); }
+    void give(void* b) { pool.give(b, [](void* p) { ++freed; std::free(p); }); }
+};
+using P = bgw::Readback<Pooled>;
+int main() {
+    std::vector<char> dev(4096, 'd');
+    {   // one call after the other: one block
+        for (int k = 0; k < 50; ++k) {
+            Queue q;
+            P r(Pooled{{&q, nullptr}});
+            std::vector<char> a(100);
+            r.add(a.data(), dev.data(), a.size());
+            r.wait();
+            EXPECT(a[99] == 'd');
+        }
+        EXPECT(made == 1 && freed == 0);
+    }
+    {   // six at once: six blocks, two of them freed afterwards
+        std::set<void*> seen;
+        std::vector<void*> held;
+        for (int k = 0; k < 6; ++k) held.push_back(Pooled().take());
+        seen.insert(held.begin(), held.end());
+        EXPECT(seen.size() == 6 && made == 6);
+        for (void* b : held) Pooled().give(b);
+        EXPECT(freed == 2);
+    }
+    {   // not waited for: the copy has ended before the block goes back, or the block does not go back
+        for (int lost = 0; lost < 2; ++lost) {
+            Queue q;
+            char a[8] = {0};
+            {
+                P r(Pooled{{&q, nullptr}});
+                r.add(a, dev.data(), sizeof a);
+                q.fail = lost;
+            }
+            EXPECT(q.waits == 1 && a[0] == 0);
+            EXPECT(q.queued.empty() == !lost);
+        }
+        std::vector<void*> held;
+        const int before = made;
+        for (int k = 0; k < 4; ++k) held.push_back(Pooled().take());
+        EXPECT(made == before + 1);  // three were left
+        for (void* b : held) Pooled().give(b);
+    }
+    std::vector<std::thread> threads;
+    for (int t = 0; t < 8; ++t)
+        threads.emplace_back([t] {
+            std::vector<char> mine(512, (char)('a' + t));
+            for (int k = 0; k < 2000; ++k) {
+                Queue q;
+                P r(Pooled{{&q, nullptr}});
+                std::vector<char> a(512);
+                r.add(a.data(), mine.data(), a.size());
+                std::this_thread::yield();
+                r.wait();
+                EXPECT(a == mine);
+            }
+        });
+    for (auto& t : threads) t.join();
 }
 """)
