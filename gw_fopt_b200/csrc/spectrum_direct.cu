@@ -629,16 +629,23 @@ __global__ void __launch_bounds__(32 * kDirWarps, PER_T ? 0 : 2) k_direct_a(RowS
     }
 }
 
-// The sum of a pair's n_parts values at p[part per], in order; eight loads in flight (past the end zeros, which
-// change no sum: a loop of single loads for the remainder took 2 to 4 us of a 90 us call).
-__device__ __forceinline__ double2 part_sum(const double2* __restrict__ p, int n_parts, size_t per) {
+// A pair's parts are added up as kSubSums sums over the parts s, s + kSubSums, ..., then in the order of s.  Single
+// threads walking all parts took 2 to 4 us more of calls of 45 to 100 us: the loads of one batch wait for the last.
+constexpr int kSubSums = 4;
+
+// Sum s of a pair's n_parts values at p[part per], eight loads in flight (past the end zeros, which change no sum).
+__device__ __forceinline__ double2 sub_sum(const double2* __restrict__ p, int s, int n_parts, size_t per) {
+    constexpr int kBatch = 8;
     double2 v = make_double2(0.0, 0.0);
-    for (int a = 0; a < n_parts; a += 8) {
-        double2 x[8];
+    for (int a = s; a < n_parts; a += kBatch * kSubSums) {
+        double2 x[kBatch];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) x[u] = a + u < n_parts ? p[(a + u) * per] : make_double2(0.0, 0.0);
+        for (int u = 0; u < kBatch; ++u) {
+            const int part = a + u * kSubSums;
+            x[u] = part < n_parts ? p[part * per] : make_double2(0.0, 0.0);
+        }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < kBatch; ++u) {
             v.x += x[u].x;
             v.y += x[u].y;
         }
@@ -649,38 +656,71 @@ __device__ __forceinline__ double2 part_sum(const double2* __restrict__ p, int n
 // out[p][q] = the sum of pair p's parts at partial[p][part][q].
 __global__ void k_direct_pairs(const double2* __restrict__ partial, int n_parts, size_t per, size_t n_pairs,
                                double2* __restrict__ out) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t per_pair = n_parts * per;
-    if (q < n_pairs * per) out[q] = part_sum(partial + q / per * per_pair + q % per, n_parts, per);
+    const size_t at = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (at >= n_pairs * per) return;
+    const double2* p = partial + at / per * (n_parts * per) + at % per;
+    double2 sum = sub_sum(p, 0, n_parts, per);
+#pragma unroll
+    for (int s = 1; s < kSubSums; ++s) {
+        const double2 v = sub_sum(p, s, n_parts, per);
+        sum.x += v.x;
+        sum.y += v.y;
+    }
+    out[at] = sum;
 }
 
 constexpr int kReduceRows = 32;
+// Rows of threads that share a frame's n pairs: one a pair, as a power of two, up to 32.
+int reduce_rows(size_t n) {
+    int r = 1;
+    while (r < kReduceRows && (size_t)r < n) r *= 2;
+    return r;
+}
 
-// out[k][q] = the sum over frame k's n pairs of their parts' sums: kReduceRows strided rows of threads, then the
-// rows in order (an order that depends on n and n_parts only).
-__global__ void __launch_bounds__(32 * kReduceRows) k_direct_reduce(const double2* __restrict__ partial, size_t n, int n_parts, size_t per,
-                                double2* __restrict__ out) {
-    __shared__ double2 red[kReduceRows][32];
-    const size_t q = (size_t)blockIdx.x * 32 + threadIdx.x;
+// out[k][q] = the sum over frame k's n pairs of their parts' sums: blockDim.y strided rows of threads, then the rows
+// in order (an order that depends on n and n_parts only).  ONE: there is one part a pair; otherwise a warp's lanes
+// are kSubSums sums of 32 / kSubSums values.
+template <bool ONE>
+__global__ void __launch_bounds__(32 * kReduceRows)
+    k_direct_reduce(const double2* __restrict__ partial, size_t n, int n_parts, size_t per, double2* __restrict__ out) {
+    constexpr int NS = ONE ? 1 : kSubSums, NQ = 32 / NS;
+    __shared__ double2 red[kReduceRows][NQ];
+    const int ql = threadIdx.x % NQ, s = threadIdx.x / NQ;
+    const size_t q = (size_t)blockIdx.x * NQ + ql;
     const size_t per_pair = n_parts * per;
     const double2* p = partial + blockIdx.y * n * per_pair + q;
     double2 acc = make_double2(0.0, 0.0);
-    if (q < per) {
-        for (size_t a = threadIdx.y; a < n; a += kReduceRows) {
-            const double2 v = part_sum(p + a * per_pair, n_parts, per);
-            acc.x += v.x;
-            acc.y += v.y;
+    for (size_t a = threadIdx.y; a < n; a += blockDim.y) {
+        double2 v = make_double2(0.0, 0.0);
+        if (q < per) v = ONE ? p[a * per_pair] : sub_sum(p + a * per_pair, s, n_parts, per);
+        double2 sum = v;
+#pragma unroll
+        for (int o = 1; o < NS; ++o) {
+            sum.x += __shfl_sync(0xffffffffu, v.x, ql + o * NQ);
+            sum.y += __shfl_sync(0xffffffffu, v.y, ql + o * NQ);
         }
+        acc.x += sum.x;
+        acc.y += sum.y;
     }
-    red[threadIdx.y][threadIdx.x] = acc;
+    if (s == 0) red[threadIdx.y][ql] = acc;  // (the other lanes' sums are not in this order)
     __syncthreads();
-    if (threadIdx.y || q >= per) return;
+    if (threadIdx.y || s || q >= per) return;
     double2 sum = make_double2(0.0, 0.0);
-    for (int y = 0; y < (int)min(n, (size_t)kReduceRows); ++y) {
-        sum.x += red[y][threadIdx.x].x;
-        sum.y += red[y][threadIdx.x].y;
+    for (int y = 0; y < (int)blockDim.y; ++y) {
+        sum.x += red[y][ql].x;
+        sum.y += red[y][ql].y;
     }
     out[(size_t)blockIdx.y * per + q] = sum;
+}
+
+template <bool ONE>
+void launch_reduce(const double2* partial, size_t n, int n_parts, size_t per, size_t frames, double2* out, cudaStream_t st) {
+    constexpr size_t NQ = ONE ? 32 : 32 / kSubSums;
+    const size_t gx = (per + NQ - 1) / NQ;
+    if (gx > 0x7fffffffULL) throw Error{"direct kernel: too many outputs for one launch"};
+    k_direct_reduce<ONE><<<dim3((unsigned)gx, (unsigned)frames), dim3(32, reduce_rows(n)), 0, st>>>(partial, n, n_parts, per,
+                                                                                               out);
+    CUDA_OK(cudaGetLastError());
 }
 
 // Separated factors need (tau / dt_last)^p, (dt_last / dt)^p and the damping exponentials inside the
@@ -893,10 +933,10 @@ uint64_t launch_direct(Device* dev, const SpectrumJob& job, const DirectInputs& 
             ++launches;
         }
     }
-    const dim3 gr((unsigned)((per + 31) / 32), (unsigned)kn);
-    k_direct_reduce<<<gr, dim3(32, kReduceRows), 0, dev->stream>>>((const double2*)(once ? dev->partial : dev->fact_partial).p,
-                                                         job.n_sel, once ? P.nkc : 1, per, out);
-    CUDA_OK(cudaGetLastError());
+    if (once)
+        launch_reduce<false>((const double2*)dev->partial.p, job.n_sel, P.nkc, per, kn, out, dev->stream);
+    else
+        launch_reduce<true>((const double2*)dev->fact_partial.p, job.n_sel, 1, per, kn, out, dev->stream);
     return launches + 1;
 }
 
@@ -911,8 +951,7 @@ uint64_t launch_direct_integrand(Device* dev, const SpectrumJob& job, const Dire
     parts = std::min(parts, std::max<size_t>(1, kDirectPartialBytes / (per * sizeof(double2))));
     P.per_warp = (int)((pairs + parts - 1) / parts);
     parts = (pairs + P.per_warp - 1) / P.per_warp;
-    const size_t gx = (per + 31) / 32;
-    if (gx > 0x7fffffffULL) throw Error{"direct kernel: integrand too large for one launch"};
+    if ((per + 31) / 32 > 0x7fffffffULL) throw Error{"direct kernel: integrand too large for one launch"};
     DirArgs A = direct_args(job, in);
     launch_steps(dev, A);
     uint64_t launches = 1;
@@ -939,9 +978,7 @@ uint64_t launch_direct_integrand(Device* dev, const SpectrumJob& job, const Dire
             launches += 2;
         }
     }
-    k_direct_reduce<<<dim3((unsigned)gx, 1), dim3(32, kReduceRows), 0, dev->stream>>>((const double2*)dev->partial.p, parts, 1,
-                                                                          per, out);
-    CUDA_OK(cudaGetLastError());
+    launch_reduce<true>((const double2*)dev->partial.p, parts, 1, per, 1, out, dev->stream);
     return launches + 1;
 }
 
