@@ -261,11 +261,12 @@ static void launch_pq(const AdjArgs& A, size_t kn, cudaStream_t st, const void* 
     const size_t v2 = F32 ? sizeof(float2) : sizeof(double2);
     const int W16 = (A.n_w + kPqW - 1) / kPqW * kPqW;
     const size_t m_tiles = 2 * kPqW * kPqCols * v2, per_w = kPqRows * v2 + v2 / 2;
-    const int w_held = W16 * per_w + m_tiles <= 110 * 1024 ? W16 : kPqW;
+    constexpr size_t most = 110 * 1024;
+    const int w_held = W16 * per_w + m_tiles <= most ? W16 : kPqW;
     const size_t smem = w_held * per_w + m_tiles;
     const int row_tiles = (A.n_sel * 2 * S + kPqRows - 1) / kPqRows;
     const dim3 g((unsigned)row_tiles, (unsigned)A.n_cos, (unsigned)kn);
-    CUDA_OK(cudaFuncSetAttribute(k_adj_pq<S, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(k_adj_pq<S, F32>, most);
     k_adj_pq<S, F32><<<g, kAdjThreads, smem, st>>>(A, mt, w_held);
     CUDA_OK(cudaGetLastError());
 }
@@ -807,8 +808,8 @@ __global__ void k_adj_params(AdjArgs A, long n_bubbles) {
 // ---------------------------------------------------------------------------
 template <int S, int SMC, int JPL>
 static void launch_rows(const AdjArgs& A, long rows, cudaStream_t st, const double* tt) {
-    const size_t smem = (size_t)kRowWarps * row_components<SMC>() * 65 * sizeof(double);
-    CUDA_OK(cudaFuncSetAttribute(k_adj_rows<S, SMC, JPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t smem = (size_t)kRowWarps * row_components<SMC>() * 65 * sizeof(double);
+    allow_shared(k_adj_rows<S, SMC, JPL>, smem);
     k_adj_rows<S, SMC, JPL><<<(unsigned)((rows + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, smem, st>>>(A, tt);
 }
 

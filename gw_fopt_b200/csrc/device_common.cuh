@@ -20,6 +20,17 @@ namespace bgw {
             throw ::bgw::Error{std::string("CUDA error: ") + cudaGetErrorString(e_) + " (" #x ")"}; \
     } while (0)
 
+// Shared memory a block may have, static and dynamic (227 KB, sm_100a).
+constexpr size_t kMaxBlockShared = 232448;
+
+// Allows a kernel's launches `most` bytes of dynamic shared memory.  The attribute belongs to the kernel on the device:
+// every handle and host thread shares it.  So `most` is a constant, the largest size that any call can need, and never
+// this call's own: a smaller one set between another thread's call and its launch would have that launch refused.
+template <class Kernel>
+void allow_shared(Kernel* kernel, size_t most) {
+    CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+}
+
 // Spacetime event / interval (t, x, y, z); 32-byte aligned rows in HBM.
 struct __align__(16) D4 {
     double t, x, y, z;

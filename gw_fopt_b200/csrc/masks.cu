@@ -413,11 +413,12 @@ static void launch_neighbors(const D4* bub, size_t n_int, size_t n_tot, const ui
                              size_t n_sel, NbList* lists, cudaStream_t st) {
     if (n_sel > 0x7fffffffULL) throw Error{"too many radiating bubbles"};
     if (n_tot > 0x7fffffffULL) throw Error{"too many bubbles"};
-    const unsigned n_cache = (unsigned)std::min<size_t>(n_tot, ranges ? 8192 : 32768);
+    constexpr unsigned few = 8192, most = 32768;
+    const unsigned n_cache = (unsigned)std::min<size_t>(n_tot, ranges ? few : most);
     const size_t smem = n_cache * sizeof(unsigned);
-    auto* kernel = n_cache > 8192 ? k_neighbors<1024> : k_neighbors<256>;
-    CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<(unsigned)n_sel, n_cache > 8192 ? 1024 : 256, smem, st>>>(bub, n_int, n_tot, sel, ranges, n_cache, lists);
+    auto* kernel = n_cache > few ? k_neighbors<1024> : k_neighbors<256>;
+    allow_shared(kernel, (n_cache > few ? most : few) * sizeof(unsigned));
+    kernel<<<(unsigned)n_sel, n_cache > few ? 1024 : 256, smem, st>>>(bub, n_int, n_tot, sel, ranges, n_cache, lists);
     CUDA_OK(cudaGetLastError());
 }
 
@@ -1045,8 +1046,8 @@ static void launch_search(const MaskArgs& A, size_t kn, cudaStream_t stream) {
     if (gx > 0x7fffffffULL || kn > 65535) throw Error{"too many (bubble, patch) pairs for one launch"};
     const dim3 grid((unsigned)gx, (unsigned)kn);
     // more shared memory than the 48 KB a kernel may use without asking
-    CUDA_OK(cudaFuncSetAttribute(k_masks_list<GRID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MaskBlock)));
-    CUDA_OK(cudaFuncSetAttribute(k_masks_rest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MaskBlock)));
+    allow_shared(k_masks_list<GRID>, sizeof(MaskBlock));
+    allow_shared(k_masks_rest, sizeof(MaskBlock));
     k_masks_list<GRID><<<grid, kMaskListThreads, sizeof(MaskBlock), stream>>>(A);
     CUDA_OK(cudaGetLastError());
     k_masks_rest<<<grid, kMaskListThreads, sizeof(MaskBlock), stream>>>(A);

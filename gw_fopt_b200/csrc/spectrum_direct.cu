@@ -818,7 +818,9 @@ void launch_a(const RowSumArgs& R, int G, size_t gx, bool big, cudaStream_t st) 
     const dim3 grid((unsigned)(gx * w_tiles), (unsigned)(R.d.S * G / NC));
     const size_t smem = ((size_t)kRowStages * stage_pairs<NC>() * 2 * NC * 32 + R.d.n_cos) * sizeof(double);
     auto* kernel = big ? k_direct_a<NC, NW, true, PER_T> : k_direct_a<NC, NW, false, PER_T>;
-    CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t most = kMaxBlockShared - kPhaseTable * sizeof(double2);
+    if (smem > most) throw Error{"n_cos_thetax too large for the shared-memory layout"};
+    allow_shared(kernel, most);
     kernel<<<grid, 32 * warps, smem, st>>>(R, G, w_tiles);
     CUDA_OK(cudaGetLastError());
 }

@@ -169,6 +169,7 @@ struct BetaArgs {
     const double* Dmax;    // int8 digit layout: (n_sel, nblk, 1+S*M, 2) least and largest D over each block's steps
 };
 
+constexpr size_t kBetaShared = 220 * 1024;  // shared memory of k_beta's blocks on an SM, at most
 constexpr int kSegBlocks = 4;              // blocks of 32 steps in an event segment
 constexpr int kSeg = 32 * kSegBlocks;
 
@@ -712,7 +713,7 @@ __global__ void __launch_bounds__(32 * beta_warps(SMC), beta_blocks(SMC)) k_beta
 
 template <class Real, int SMC>
 static void launch_beta_smc(const BetaArgs& B, Real* out, size_t smem, int n_sm, int warps, cudaStream_t st) {
-    CUDA_OK(cudaFuncSetAttribute(k_beta<Real, SMC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(k_beta<Real, SMC>, kBetaShared);
     // three blocks per SM need the largest shared-memory carveout; without the preference the
     // driver may pick a smaller one (two blocks per SM) depending on the kernels run before
     CUDA_OK(cudaFuncSetAttribute(k_beta<Real, SMC>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1322,10 +1323,11 @@ static void launch_sorted_smc(BetaArgs& B, int8_t* out, cudaStream_t st) {
                 (size_t)n_phi * sizeof(uint16_t);
     pw = (pw + 15) & ~(size_t)15;
     B.per_warp_bytes = (int)pw;
-    const int warps = (int)std::min<size_t>(8, (200 * 1024) / pw);
+    constexpr size_t most = 200 * 1024;
+    const int warps = (int)std::min<size_t>(8, most / pw);
     if (warps < 1) throw Error{"n_phi too large for the beta kernel"};
     const size_t smem = (size_t)warps * pw;
-    CUDA_OK(cudaFuncSetAttribute(k_beta_sorted<SMC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(k_beta_sorted<SMC>, most);
     CUDA_OK(cudaFuncSetAttribute(k_beta_sorted<SMC>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  (int)cudaSharedmemCarveoutMaxShared));
     k_beta_sorted<SMC><<<(unsigned)((B.n_rows + warps - 1) / warps), warps * 32, smem, st>>>(B, out);
@@ -1959,7 +1961,7 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
         const size_t bins = (size_t)(2 + 2 * SM) * kSeg;
         const size_t others = 4 + 2 * (size_t)SM + beta_rows_held(SM) * 32 * pitch + 16 * pitch;
         const size_t blocks_sm = beta_blocks(SM), most = beta_warps(SM);
-        B.keep = tc && blocks_sm * (64 * pitch + most * (2 * bins + others)) * sizeof(double) <= 220 * 1024 ? 2 : 1;
+        B.keep = tc && blocks_sm * (64 * pitch + most * (2 * bins + others)) * sizeof(double) <= kBetaShared ? 2 : 1;
         const size_t per_warp = (B.keep * bins + others + 1) & ~(size_t)1;
         B.per_warp = (int)per_warp;
         B.tiles = G.tiles_per_frame;
@@ -1970,7 +1972,7 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
         if (sorted) {
             if constexpr (tc) launch_sorted(SM, B, (int8_t*)dev->beta.p, dev->stream);
         } else {
-            const size_t room = 220 * 1024 / sizeof(double);
+            const size_t room = kBetaShared / sizeof(double);
             if (64 * pitch + per_warp > room) throw Error{"n_phi too large for the beta kernel"};
             const int warps = (int)std::min<size_t>(most, (room - 64 * pitch) / per_warp);
             const size_t smem = (64 * pitch + warps * per_warp) * sizeof(double);
@@ -2055,16 +2057,16 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
         return launches;
     } else {
         const size_t smem = fold ? fold_smem_bytes(S) : gemm_smem_bytes<float, 8>(S);
-        if (smem > 227 * 1024 || (fold && S > 4))
+        if (smem > kMaxBlockShared || (fold && S > 4))
             throw Error{"too many coefficient sets for the factored kernel's shared memory"};
         const size_t gy = (size_t)kn * G.tiles_per_frame;
         if (gy > 65535) throw Error{"too many column tiles in one k-hat chunk"};
         const dim3 grid((unsigned)((n_w + kWT - 1) / kWT), (unsigned)gy, (unsigned)row_parts);
         if constexpr (fold) {
-            CUDA_OK(cudaFuncSetAttribute(k_gemm_fold, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            allow_shared(k_gemm_fold, kMaxBlockShared);
             k_gemm_fold<<<grid, kThreads, smem, dev->stream>>>(A, fold_work(S));
         } else {
-            CUDA_OK(cudaFuncSetAttribute(k_gemm<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            allow_shared(k_gemm<float, 8>, kMaxBlockShared);
             k_gemm<float, 8><<<grid, kThreads, smem, dev->stream>>>(A);
         }
         CUDA_OK(cudaGetLastError());

@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_gemm_i8(TcArgs A) {
 template <int S, int ST>
 void launch_st(const TcArgs& A, dim3 grid, cudaStream_t st) {
     const size_t smem = SmemLayout<ST>::total + 1024;
-    CUDA_OK(cudaFuncSetAttribute(k_gemm_i8<S, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(k_gemm_i8<S, ST>, smem);
     k_gemm_i8<S, ST><<<grid, kTcThreads, smem, st>>>(A);
 }
 
