@@ -15,7 +15,7 @@
 namespace bgw {
 
 constexpr int kPhaseTable = 256;            // N
-constexpr double kPhaseMax = 1.0e9;         // largest |x| the reduction is used for
+constexpr double kPhaseMax = 1.0e9;         // largest |x| the reduction is meant for
 
 // Fills the table (N entries of shared memory) with the threads of a block.
 __device__ __forceinline__ void phase_table_fill(double2* tab) {

@@ -17,7 +17,9 @@
 //               sum with one phase per (row, step, frequency).  The phase argument w (-dt c_i) is
 //               rounded as the reference rounds it.  Rows i and n_cos - 1 - i have c of opposite sign
 //               up to rounding, so one table sincos serves both: the second argument is -x + e with e
-//               formed exactly, and a first-order correction in e (|e| < 1e-10, e^2 below 2^-66).
+//               formed exactly, and a first-order correction in e.  |e| is below 8 x 2^-53 |x| (the
+//               roundings of c, -dt c and w (-dt c) on both sides), so the e^2 / 2 left out is below
+//               2^-56 for the |x| < 4e6 that this form is used for; beyond, the library's sincos.
 //
 // What bounds it: FP64 issue in k_direct_a (about 14 operations and 4 per column for each phase);
 // k_direct_b is a few per cent.  The single kernel this replaces (one block per bubble, pow() for
@@ -368,7 +370,10 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_direct_b(DirArgs A) {
     }
 }
 
-// Phase of one argument; BIG: arguments past the table reduction's range (or not finite).
+constexpr double kTwinMax = 4.0e6;  // largest |x| of the paired rows
+static_assert(kTwinMax <= kPhaseMax, "the table's own range");
+
+// Phase of one argument; BIG: arguments past kTwinMax (or not finite).
 template <bool BIG>
 __device__ __forceinline__ void phase_of(const double2* tab, double x, double& s, double& c) {
     if constexpr (BIG)
@@ -737,7 +742,7 @@ bool direct_exact(const SpectrumJob& job) {
     return false;
 }
 
-// Arguments the table reduction covers: |w| times the largest time or position difference.
+// Arguments past kTwinMax: |w| times the largest time or position difference.
 bool direct_big(const SpectrumJob& job) {
     double wmax = 0.0, xmax = 0.0;
     for (size_t q = 0; q < job.n_w; ++q) {
@@ -752,7 +757,7 @@ bool direct_big(const SpectrumJob& job) {
         if (!std::isfinite(b[0]) || !std::isfinite(r)) return true;
         xmax = std::max(xmax, std::max(std::fabs(b[0]), r));
     }
-    return !(wmax * (tmax + xmax) < kPhaseMax);
+    return !(wmax * (tmax + xmax) < kTwinMax);
 }
 
 struct DirectPlan {
