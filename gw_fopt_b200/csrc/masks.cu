@@ -1063,7 +1063,8 @@ struct MaskShape {
     int rows_per_item, lane_cols;
     unsigned n_split;
 };
-static MaskShape mask_shape(size_t nd, size_t row_len, size_t n_pairs, int chunking) {
+static MaskShape mask_shape(size_t nd, size_t row_len, size_t n_pairs, int n_sm, int chunking) {
+    const size_t fill = 8 * (size_t)n_sm;  // eight blocks per SM
     const size_t n_rows = nd / row_len;
     MaskShape m;
     m.lane_cols = n_rows >= 4 ? 8 : 32;
@@ -1073,13 +1074,13 @@ static MaskShape mask_shape(size_t nd, size_t row_len, size_t n_pairs, int chunk
     const size_t strips = (row_len + m.lane_cols - 1) / m.lane_cols;
     // few bubbles: smaller items, so that every SM has a few
     size_t groups = (n_rows + m.rows_per_item - 1) / m.rows_per_item;
-    while (m.rows_per_item > 32 / m.lane_cols && n_pairs * strips * groups < 148 * 8) {
+    while (m.rows_per_item > 32 / m.lane_cols && n_pairs * strips * groups < fill) {
         m.rows_per_item /= 2;
         groups = (n_rows + m.rows_per_item - 1) / m.rows_per_item;
     }
     const size_t total = strips * groups;  // of one bubble and frame
     if (total * m.lane_cols > 0x7fffffffULL) throw Error{"too many directions for the mask search"};
-    const size_t items = std::min<size_t>(std::max<size_t>(8, n_pairs * total / (148 * 8)),
+    const size_t items = std::min<size_t>(std::max<size_t>(8, n_pairs * total / fill),
                                           std::max<size_t>(8, 16384 / (m.lane_cols * m.rows_per_item)));
     // the launch shape may ask for 2 or 4 times the automatic number of blocks
     m.n_split = (unsigned)std::min(total, (total + items - 1) / items * (size_t)std::max(1, std::min(chunking, 4)));
@@ -1089,7 +1090,7 @@ static MaskShape mask_shape(size_t nd, size_t row_len, size_t n_pairs, int chunk
 // ------------------------------------------------------------------ host
 void launch_masks_with_lists(cudaStream_t stream, const D4* bub, size_t n_int, size_t n_tot, const uint32_t* sel,
                              size_t n_sel, const D4* dirs, size_t nd, NbList* lists, double* tau, int32_t* codes,
-                             unsigned long long* counters) {
+                             unsigned long long* counters, int n_sm) {
     if (n_tot < 2) {
         CUDA_OK(cudaMemsetAsync(tau, 0, n_sel * nd * sizeof(double), stream));
         if (codes) CUDA_OK(cudaMemsetAsync(codes, 0xff, n_sel * nd * sizeof(int32_t), stream));
@@ -1098,7 +1099,7 @@ void launch_masks_with_lists(cudaStream_t stream, const D4* bub, size_t n_int, s
     launch_neighbors(bub, n_int, n_tot, sel, nullptr, n_sel, lists, stream);
     // the directions' row structure is not known here: one row of nd directions
     if (nd > 0x7fffffffULL) throw Error{"too many directions for the mask search"};
-    const MaskShape shape = mask_shape(nd, nd, n_sel, 1);
+    const MaskShape shape = mask_shape(nd, nd, n_sel, n_sm, 1);
     const MaskArgs A{bub,  n_int,   n_tot,          sel,           nullptr,         n_sel, lists, dirs,    nullptr, nullptr,
                      1,    (int)nd, shape.n_split, shape.rows_per_item, shape.lane_cols, tau,   codes, nullptr, counters};
     launch_search<false>(A, 1, stream);
@@ -1119,7 +1120,7 @@ void launch_mask_pipeline(Device* dev, const D4* bub_unrot, const D4* bub_frames
         launch_neighbors(bub_unrot, n_int, n_tot, sel, ranges, n_sel, (NbList*)dev->nblists.p, dev->stream);
         if (launches) ++*launches;
     }
-    const MaskShape shape = mask_shape(nd, row_len, n_sel * kn, chunking);
+    const MaskShape shape = mask_shape(nd, row_len, n_sel * kn, dev->n_sm, chunking);
     dev->mask_open.ensure(n_sel * kn * shape.n_split * sizeof(unsigned));
     const MaskArgs A{bub_frames,
                      n_int,

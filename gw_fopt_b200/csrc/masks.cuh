@@ -24,10 +24,11 @@ struct NbList {
 };
 
 // Builds candidate lists into `lists` (n_sel entries) and runs the exact
-// search for one frame on `stream`; tau/codes: (n_sel, nd).  Allocates nothing.
+// search for one frame on `stream` of a device with n_sm multiprocessors; tau/codes:
+// (n_sel, nd).  Allocates nothing.
 void launch_masks_with_lists(cudaStream_t stream, const D4* bub, size_t n_int, size_t n_tot, const uint32_t* sel,
                              size_t n_sel, const D4* dirs, size_t nd, NbList* lists, double* tau, int32_t* codes,
-                             unsigned long long* counters);
+                             unsigned long long* counters, int n_sm);
 
 // Builds the lists (when build_lists) from the unrotated bubbles and runs the
 // list-based exact search for kn frames.  tau/codes: (kn, n_sel, nd); the

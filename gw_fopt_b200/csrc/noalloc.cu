@@ -71,8 +71,9 @@ extern "C" BgwStatus bgwx_first_colliding_noalloc(const double* d_bubbles, size_
                         std::to_string(kNoAllocMaxBubbles) + " radiating bubbles per call"};
         if (n_interior == 0 || n_interior > n_total) throw Error{"need 0 < n_interior <= n_total"};
         if (n_total > 0x7fffffffULL || n_dirs > 0x7fffffffULL) throw Error{"n_total or n_dirs too large"};
-        int dev = 0;
+        int dev = 0, n_sm = 0;
         CUDA_OK(cudaGetDevice(&dev));
+        CUDA_OK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
         unsigned char* base = static_cast<unsigned char*>(scratch_address(dev));
         NbList* lists = reinterpret_cast<NbList*>(base);
         unsigned long long* counter =
@@ -81,7 +82,7 @@ extern "C" BgwStatus bgwx_first_colliding_noalloc(const double* d_bubbles, size_
         CUDA_OK(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
         launch_masks_with_lists(st, reinterpret_cast<const D4*>(d_bubbles), n_interior, n_total, d_selected,
                                 n_selected, reinterpret_cast<const D4*>(d_dirs), n_dirs, lists, d_delta_tab, d_codes,
-                                counter);
+                                counter, n_sm);
         clear_last_error();
         return BGW_STATUS_OK;
     } catch (const Error& e) {
