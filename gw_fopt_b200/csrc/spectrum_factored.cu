@@ -978,10 +978,8 @@ __global__ void __launch_bounds__(256, 3) k_beta_sorted(BetaArgs A, int8_t* __re
     // offsets are compared four at a time as bytes), then warp scans give the
     // collided sums up to and the uncollided sums after every step.  Blocks
     // without events have constant sums: each lane forms 4 consecutive steps,
-    // 8 lanes a block, 4 such blocks at a time (int8 digits: 16 steps, 2 lanes
-    // a block, 16 blocks at a time).  The int8 digit layout needs the row's
-    // scale, max |beta| over its steps and columns, before any digit: a first
-    // sweep forms every value and keeps only the maximum.
+    // 8 lanes a block, 4 such blocks at a time.  The digits need the row's
+    // scale, max |beta| over its steps and columns, first.
     const double ci = A.cos_t[i];
     const double vi = (i == 0 || i == A.n_cos - 1) ? 0.5 : 1.0;
     const double rf = (0.5 * (1.0 - ci * ci) * A.dphi) * (A.dcos * vi) * A.dt * (1.0 / (6.0 * CUDART_PI));
@@ -1377,15 +1375,15 @@ __device__ __forceinline__ int thread_col(int tx, int u) {
     return u < TN / 2 ? tx * (TN / 2) + u : COLS / 2 + tx * (TN / 2) + (u - TN / 2);
 }
 
-template <class Real, int TN>
+constexpr int kGemmTN = 8, kGemmCols = 16 * kGemmTN, kGemmBS = kGemmCols + 4;  // (padded row of the beta tile)
+
 __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int COLS = 16 * TN;                                  // 128 (FP32) or 64 (FP64)
-    constexpr int BS = COLS + 16 / (int)sizeof(Real);              // padded row of the beta tile
-    constexpr int VEC = 16 / (int)sizeof(Real);                    // elements per 16-byte load
+    constexpr int TN = kGemmTN, COLS = kGemmCols, BS = kGemmBS;
+    constexpr int VEC = 4;                                         // elements per 16-byte load
     constexpr int NPRE = COLS * kKC / VEC / kThreads;              // 16-byte loads per thread per tile
-    Real* Msm = reinterpret_cast<Real*>(smem);                     // [kKC][kRows]
-    Real* Bsm = Msm + kKC * kRows;                                 // [kKC][BS]
+    float* Msm = reinterpret_cast<float*>(smem);                   // [kKC][kRows]
+    float* Bsm = Msm + kKC * kRows;                                // [kKC][BS]
     double* Pn_re = reinterpret_cast<double*>(Bsm + kKC * BS);      // [kKC][kWT]
     double* Pn_im = Pn_re + kKC * kWT;
     double* anc = Pn_im + kKC * kWT;                               // [2][kWT]
@@ -1402,7 +1400,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
     const int tile = blockIdx.y % A.tiles_per_frame;
     const int cpb = 2 * A.S;  // columns per bubble
     const D4* B = A.bub + (size_t)frame * A.n_tot;
-    const Real* beta = static_cast<const Real*>(A.beta);
+    const float* beta = static_cast<const float*>(A.beta);
 
     if (tid < 64) {
         const int slot = tile * A.bpt + tid;
@@ -1430,22 +1428,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
             const int n = q / kWT, wl = q % kWT;
             const int wi = w0 + wl;
             double sn = 0.0, cs = 1.0;
-            if (wi < A.n_w) phase<Real>(A.w[wi] * one_m_c * (n * A.dt), sn, cs);
+            if (wi < A.n_w) phase<float>(A.w[wi] * one_m_c * (n * A.dt), sn, cs);
             Pn_re[q] = cs;
             Pn_im[q] = sn;
         }
-        const Real* bi = beta + (((size_t)frame * A.n_cos + i) * A.cols_pad + col0) * A.t_pad;
+        const float* bi = beta + (((size_t)frame * A.n_cos + i) * A.cols_pad + col0) * A.t_pad;
         // 16-byte loads of the beta tile: column q / (kKC/VEC), steps VEC*(q % (kKC/VEC)) ...
-        using Vec = typename std::conditional<sizeof(Real) == 4, float4, double2>::type;
-        Vec pre[NPRE];
+        float4 pre[NPRE];
         auto fetch = [&](int k0) {
 #pragma unroll
             for (int v = 0; v < NPRE; ++v) {
                 const int q = tid + v * kThreads;
                 const int col = q / (kKC / VEC), n = (q % (kKC / VEC)) * VEC;
                 const int k = k0 + n;  // t_pad is a multiple of VEC: a load is all in or all out
-                if (k < A.t_pad) pre[v] = __ldg(reinterpret_cast<const Vec*>(bi + (size_t)col * A.t_pad + k));
-                else pre[v] = Vec{};
+                if (k < A.t_pad) pre[v] = __ldg(reinterpret_cast<const float4*>(bi + (size_t)col * A.t_pad + k));
+                else pre[v] = float4{};
             }
         };
         double acc[kTM][TN];
@@ -1461,7 +1458,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
             if (tid < kWT) {
                 const int wi = w0 + tid;
                 double sn = 0.0, cs = 0.0;
-                if (wi < A.n_w) phase<Real>(A.w[wi] * one_m_c * A.t_arr[k0], sn, cs);
+                if (wi < A.n_w) phase<float>(A.w[wi] * one_m_c * A.t_arr[k0], sn, cs);
                 anc[tid] = cs;
                 anc[kWT + tid] = sn;
             }
@@ -1469,7 +1466,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
             for (int v = 0; v < NPRE; ++v) {
                 const int q = tid + v * kThreads;
                 const int col = q / (kKC / VEC), n = (q % (kKC / VEC)) * VEC;
-                const Real* pv = reinterpret_cast<const Real*>(&pre[v]);
+                const float* pv = reinterpret_cast<const float*>(&pre[v]);
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) Bsm[(n + e) * BS + col] = pv[e];
             }
@@ -1479,8 +1476,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
                 const double ar = anc[wl], ai = anc[kWT + wl];
                 const double pr = Pn_re[q], pi = Pn_im[q];
                 const bool valid = k0 + n < A.n_t;
-                Msm[n * kRows + 2 * wl] = valid ? (Real)(ar * pr - ai * pi) : (Real)0;
-                Msm[n * kRows + 2 * wl + 1] = valid ? (Real)(ar * pi + ai * pr) : (Real)0;
+                Msm[n * kRows + 2 * wl] = valid ? (float)(ar * pr - ai * pi) : 0.0f;
+                Msm[n * kRows + 2 * wl + 1] = valid ? (float)(ar * pi + ai * pr) : 0.0f;
             }
             __syncthreads();
             if (ch + 1 < n_chunks) fetch(k0 + kKC);  // in flight during the GEMM below
@@ -1538,7 +1535,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(FactArgs A) {
                 const int b = col / cpb;
                 if (b >= A.bpt || binfo[b] < 0 || wi >= A.n_w) continue;
                 double sn, cs;
-                phase<Real>(A.w[wi] * (bt[b] * ci - bz[b]), sn, cs);
+                phase<float>(A.w[wi] * (bt[b] * ci - bz[b]), sn, cs);
                 const double yr = acc[2 * q][u], yi = acc[2 * q + 1][u];
                 double2& d = red[(size_t)(q * cpb + (col % cpb)) * kThreads + tid];
                 d.x += cs * yr - sn * yi;
@@ -1821,11 +1818,8 @@ __global__ void k_reduce_real(const double2* __restrict__ partial, const uint32_
 }
 
 // ---------------------------------------------------------------------------
-template <class Real, int TN>
 static size_t gemm_smem_bytes(int S) {
-    constexpr int COLS = 16 * TN;
-    constexpr int BS = COLS + 16 / (int)sizeof(Real);
-    size_t b = (size_t)kKC * kRows * sizeof(Real) + (size_t)kKC * BS * sizeof(Real);
+    size_t b = (size_t)kKC * kRows * sizeof(float) + (size_t)kKC * kGemmBS * sizeof(float);
     b = (b + 15) & ~(size_t)15;
     b += 2 * (size_t)kKC * kWT * sizeof(double);   // step table
     b += 2 * (size_t)kWT * sizeof(double);         // anchors
@@ -2056,7 +2050,8 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
         launches += reduce_tiles(dev, job, A.partial, G.tiles_per_frame, row_parts, per, k0, kn, out, real_tiles);
         return launches;
     } else {
-        const size_t smem = fold ? fold_smem_bytes(S) : gemm_smem_bytes<float, 8>(S);
+        const size_t smem = fold ? fold_smem_bytes(S) : gemm_smem_bytes(S);
+        // (the folded product's layout has room for 6 sets; more than 4 were always refused in FP64)
         if (smem > kMaxBlockShared || (fold && S > 4))
             throw Error{"too many coefficient sets for the factored kernel's shared memory"};
         const size_t gy = (size_t)kn * G.tiles_per_frame;
@@ -2066,8 +2061,8 @@ static uint64_t launch_typed(Device* dev, const SpectrumJob& job, const D4* bub_
             allow_shared(k_gemm_fold, kMaxBlockShared);
             k_gemm_fold<<<grid, kThreads, smem, dev->stream>>>(A, fold_work(S));
         } else {
-            allow_shared(k_gemm<float, 8>, kMaxBlockShared);
-            k_gemm<float, 8><<<grid, kThreads, smem, dev->stream>>>(A);
+            allow_shared(k_gemm, kMaxBlockShared);
+            k_gemm<<<grid, kThreads, smem, dev->stream>>>(A);
         }
         CUDA_OK(cudaGetLastError());
         ++launches;
