@@ -17,15 +17,16 @@
 //               sum with one phase per (row, step, frequency).  The phase argument w (-dt c_i) is
 //               rounded as the reference rounds it.  Rows i and n_cos - 1 - i have c of opposite sign
 //               up to rounding, so one table sincos serves both: the second argument is -x + e with e
-//               formed exactly, and a first-order correction in e.  |e| is below 8 x 2^-53 |x| (the
-//               roundings of c, -dt c and w (-dt c) on both sides), so the e^2 / 2 left out is below
-//               2^-56 for the |x| < 4e6 that this form is used for; beyond, the library's sincos.
+//               formed exactly, and a first-order correction in e.  |e| is below 10 x 2^-53 |w| dt (5 for
+//               the roundings of the two c, 2 each for -dt c and its product with w), so the e^2 / 2 left
+//               out is below 2^-56 for the |w| dt < 4e6 that this form is used for; beyond, the library's
+//               sincos for both.
 //
 // What bounds it: FP64 issue in k_direct_a (about 14 operations and 4 per column for each phase);
 // k_direct_b is a few per cent.  The single kernel this replaces (one block per bubble, pow() for
 // every patch and step, a barrier per step) took 53.6 ms for 5 bubbles x 50 x 100 patches x 800 steps
 // x 120 w and 38.2 ms for 4 frames of 64 bubbles x 64 x 64 x 256 x 64 w with 3 sets; these two take
-// 0.1 ms and 1.04 ms (k_direct_b 0.27, k_direct_a 0.76: FP64 pipe half busy, 0.34 ms of FP64 work).
+// 0.08 ms and 1.01 ms (k_direct_b 0.27, k_direct_a 0.75: FP64 pipe half busy, 0.34 ms of FP64 work).
 
 #include <cuda_runtime.h>
 
@@ -370,7 +371,7 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_direct_b(DirArgs A) {
     }
 }
 
-constexpr double kTwinMax = 4.0e6;  // largest |x| of the paired rows
+constexpr double kTwinMax = 4.0e6;  // largest argument of the paired rows
 static_assert(kTwinMax <= kPhaseMax, "the table's own range");
 
 // Phase of one argument; BIG: arguments past kTwinMax (or not finite).
